@@ -371,13 +371,12 @@ struct DeviceState {
   // wait that gives up writes its code here; it is read (and cleared) at the
   // context's next synchronization point, never by the evaluation itself
   DevBuf tc_err;
-  // tile-sparse FP64 contraction: screening spheres and AO ranges of the
-  // shells (basis order), coefficient_t with an even row length when the MO
-  // count is odd
+  // FP64 tile kernels: shell records (basis order), coefficient_t with an
+  // even row length when the MO count is odd, compact AO tiles
   uint64_t f64_sph_basis = ~0ull, f64_sph_nucl = ~0ull;
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
-  DevBuf f64_sph, coef_f;
+  DevBuf f64_sph, coef_f, f64_tiles;
 };
 
 namespace {
@@ -878,77 +877,112 @@ void nucleus_box(const Context* ctx, double* lo, double* hi) {
     }
 }
 
-// FP64 MO contraction out[p][c][mo] = sum_k ao[p][c][k] coefficient_t[k][mo]
-// of P points (coordinates coord with stride cstride), tile-sparse: points
-// in spatial tiles, and for each tile only the AOs of the shells that reach
-// one of its points (the others are exact zeros there), summed in the basis
-// order.
-qmckl_exit_code contract_f64(qmckl_context context, DeviceState* ds, int64_t P, int comps, const double* coord,
-                             int64_t cstride, const double* ao, double* out) {
+// The per-shell records of the FP64 tile kernels (basis order).
+qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
   const char* fname = "qmckl_b200_mo_fp64";
   Context* ctx = ctx_of(context);
   const AoBasisRec& B = ctx->ao_basis;
-  const int64_t A = B.ao_num, M = ctx->mo_basis.mo_num, S = B.shell_num, N = ctx->nucleus.num;
-  if (P <= 0) return QMCKL_SUCCESS;
-  qmckl_exit_code rc;
+  const AoDerived& d = B.d;
+  const int64_t A = B.ao_num, S = B.shell_num, N = ctx->nucleus.num;
   const double cutoff = cutoff_of(ctx);
-  // shell screening spheres in the basis order
-  if (!ds->f64_sph.p || ds->f64_sph_basis != B.basis_version || ds->f64_sph_nucl != ctx->nucleus.coord_version ||
-      ds->f64_sph_cutoff != cutoff) {
-    std::vector<double4> sph((size_t)S);
-    std::vector<int2> sao((size_t)S);
-    for (int64_t m = 0; m < N; ++m)
-      for (int64_t sh = B.nucleus_index[m]; sh < B.nucleus_index[m] + B.nucleus_shell_num[m]; ++sh) {
-        const int l = B.shell_ang_mom[sh];
-        const int64_t a0 = B.d.ao_index[sh];
-        const int64_t na = std::max<int64_t>(0, std::min<int64_t>((int64_t)(l + 1) * (l + 2) / 2, A - a0));
-        sph[(size_t)sh] = make_double4(ctx->nucleus.coord[m], ctx->nucleus.coord[m + N], ctx->nucleus.coord[m + 2 * N],
-                                       shell_r2max(ctx, (int)sh, (int)m, cutoff));
-        sao[(size_t)sh] = make_int2((int)a0, (int)na);
-      }
-    const size_t sb = (sizeof(double4) * (size_t)S + 255) / 256 * 256;
-    rc = ensure(context, ds->f64_sph, sb + sizeof(int2) * (size_t)S, fname);
-    if (rc != QMCKL_SUCCESS) return rc;
-    QB_CUDA(cudaMemcpy(ds->f64_sph.p, sph.data(), sizeof(double4) * (size_t)S, cudaMemcpyHostToDevice), fname);
-    QB_CUDA(cudaMemcpy((uint8_t*)ds->f64_sph.p + sb, sao.data(), sizeof(int2) * (size_t)S, cudaMemcpyHostToDevice),
-            fname);
-    ds->f64_sph_basis = B.basis_version;
-    ds->f64_sph_nucl = ctx->nucleus.coord_version;
-    ds->f64_sph_cutoff = cutoff;
-  }
-  const size_t sb = (sizeof(double4) * (size_t)S + 255) / 256 * 256;
-  // coefficient_t with 16-byte aligned rows (a padded copy for an odd MO count)
-  const double* Bt = (const double*)ds->coef_t.p;
-  int64_t ldb = M;
-  if (M & 1) {
-    ldb = M + 1;
-    if (ds->coef_f_version != ctx->mo_basis.coef_version || !ds->coef_f.p) {
-      std::vector<double> cf((size_t)(A * ldb), 0.0);
-      const std::vector<double>& c = ctx->mo_basis.coefficient;
-      for (int64_t k = 0; k < A; ++k)
-        for (int64_t i = 0; i < M; ++i) cf[(size_t)(k * ldb + i)] = c[(size_t)(i * A + k)];
-      rc = ensure(context, ds->coef_f, sizeof(double) * cf.size(), fname);
-      if (rc != QMCKL_SUCCESS) return rc;
-      QB_CUDA(cudaMemcpy(ds->coef_f.p, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice), fname);
-      ds->coef_f_version = ctx->mo_basis.coef_version;
+  if (ds->f64_sph.p && ds->f64_sph_basis == B.basis_version && ds->f64_sph_nucl == ctx->nucleus.coord_version &&
+      ds->f64_sph_cutoff == cutoff)
+    return QMCKL_SUCCESS;
+  std::vector<F64Shell> sh((size_t)S);
+  for (int64_t m = 0; m < N; ++m)
+    for (int64_t s = B.nucleus_index[m]; s < B.nucleus_index[m] + B.nucleus_shell_num[m]; ++s) {
+      F64Shell& e = sh[(size_t)s];
+      const int l = B.shell_ang_mom[s];
+      const int64_t a0 = d.ao_index[s];
+      e.x = ctx->nucleus.coord[m];
+      e.y = ctx->nucleus.coord[m + N];
+      e.z = ctx->nucleus.coord[m + 2 * N];
+      e.r2max = shell_r2max(ctx, (int)s, (int)m, cutoff);
+      e.crange = cutoff * d.nucleus_range[m];
+      e.a0 = (int32_t)a0;
+      e.na = (int32_t)std::max<int64_t>(0, std::min<int64_t>((int64_t)(l + 1) * (l + 2) / 2, A - a0));
+      e.cb = d.shell_coef_start[s];
+      e.ce = d.shell_coef_start[s + 1];
+      e.l = l;
+      e.nucl = (int32_t)m;
     }
-    Bt = (const double*)ds->coef_f.p;
+  qmckl_exit_code rc = ensure(context, ds->f64_sph, sizeof(F64Shell) * (size_t)S, fname);
+  if (rc != QMCKL_SUCCESS) return rc;
+  QB_CUDA(cudaMemcpy(ds->f64_sph.p, sh.data(), sizeof(F64Shell) * (size_t)S, cudaMemcpyHostToDevice), fname);
+  ds->f64_sph_basis = B.basis_version;
+  ds->f64_sph_nucl = ctx->nucleus.coord_version;
+  ds->f64_sph_cutoff = cutoff;
+  return QMCKL_SUCCESS;
+}
+
+// coefficient_t with an even row length (a padded copy for an odd MO count).
+qmckl_exit_code coef_even(qmckl_context context, DeviceState* ds, const double** Bt, int64_t* ldb) {
+  const char* fname = "qmckl_b200_mo_fp64";
+  Context* ctx = ctx_of(context);
+  const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
+  *ldb = M + (M & 1);
+  if (!(M & 1)) {
+    qmckl_exit_code rc = sync_coef(context, ds);
+    *Bt = (const double*)ds->coef_t.p;
+    return rc;
   }
-  // scratch: keys[P], perm[P], cell counts, then the tiles' AO lists (256-byte aligned)
-  const size_t sort_bytes = (sizeof(int) * 2 * (size_t)P + sizeof(unsigned int) * (kSortCells + 1) + 255) / 256 * 256;
-  rc = ensure(context, ds->order, sort_bytes + f64_plan_bytes(P, comps, A), fname);
+  if (ds->coef_f_version != ctx->mo_basis.coef_version || !ds->coef_f.p) {
+    std::vector<double> cf((size_t)(A * *ldb), 0.0);
+    const std::vector<double>& c = ctx->mo_basis.coefficient;
+    for (int64_t k = 0; k < A; ++k)
+      for (int64_t i = 0; i < M; ++i) cf[(size_t)(k * *ldb + i)] = c[(size_t)(i * A + k)];
+    qmckl_exit_code rc = ensure(context, ds->coef_f, sizeof(double) * cf.size(), fname);
+    if (rc != QMCKL_SUCCESS) return rc;
+    QB_CUDA(cudaMemcpy(ds->coef_f.p, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice), fname);
+    ds->coef_f_version = ctx->mo_basis.coef_version;
+  }
+  *Bt = (const double*)ds->coef_f.p;
+  return QMCKL_SUCCESS;
+}
+
+// FP64 MO VGL / value out[p][c][mo] of P points (coord [3][P]): points in
+// spatial tiles, per tile only the AOs of the shells that reach one of its
+// points, produced compactly and summed in the basis order (f64_tiles.cu).
+// The AO array is not formed.  cr: cusp radii or null.  Tiles go in chunks
+// that bound the scratch to about 4 GiB (one tile at least).
+qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, int comps, const double* coord,
+                           const double* cr, double* out) {
+  const char* fname = "qmckl_b200_mo_fp64";
+  Context* ctx = ctx_of(context);
+  const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
+  if (P <= 0) return QMCKL_SUCCESS;
+  const double* Bt = nullptr;
+  int64_t ldb = 0;
+  qmckl_exit_code rc = sync_f64_shells(context, ds);
+  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Bt, &ldb);
+  if (rc != QMCKL_SUCCESS) return rc;
+  const int pts = f64_tile_points(comps, P);
+  const int64_t tiles = (P + pts - 1) / pts;
+  const int64_t budget = (int64_t)4 << 30;
+  const int64_t most = std::max<int64_t>(1, budget / (int64_t)f64_tile_bytes(comps, pts, A));
+  const int64_t chunks = (tiles + most - 1) / most;
+  const int64_t chunk = (tiles + chunks - 1) / chunks;
+  const size_t sort_bytes = sizeof(int) * 2 * (size_t)P + sizeof(unsigned int) * (kSortCells + 1);
+  rc = ensure(context, ds->order, sort_bytes, fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, f64_tile_bytes(comps, pts, A) * (size_t)chunk, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   int* keys = (int*)ds->order.p;
   int* perm = keys + P;
   unsigned int* counts = (unsigned int*)(perm + P);
-  void* plan = (uint8_t*)ds->order.p + sort_bytes;
   double lo[3], hi[3];
   nucleus_box(ctx, lo, hi);
-  QB_CUDA(point_order(coord, P, lo, hi, keys, counts, perm, ds->stream, cstride), fname);
-  QB_CUDA(launch_f64_plan(P, comps, coord, cstride, perm, (int)S, ds->f64_sph.p, (uint8_t*)ds->f64_sph.p + sb, A, plan,
-                          ds->stream),
-          fname);
-  QB_CUDA(launch_gemm_f64_sparse(P, comps, M, ao, A, perm, plan, A, Bt, ldb, out, M, ds->stream), fname);
+  if (tiles > 1)
+    QB_CUDA(point_order(coord, P, lo, hi, keys, counts, perm, ds->stream, P), fname);
+  else
+    perm = nullptr;   // one tile: any order
+  const F64Tiles t = f64_tiles_at(ds->f64_tiles.p, chunk, comps, pts, A);
+  for (int64_t t0 = 0; t0 < tiles; t0 += chunk) {
+    const int64_t n = std::min(chunk, tiles - t0);
+    QB_CUDA(launch_ao_tiles(ds->T, P, comps, coord, P, perm, t0, n, (const F64Shell*)ds->f64_sph.p, cutoff_of(ctx),
+                            ctx->precision > 23, cr, t, ds->stream),
+            fname);
+    QB_CUDA(launch_tile_gemm(P, comps, t0, n, M, A, t, perm, Bt, ldb, out, ds->stream), fname);
+  }
   return QMCKL_SUCCESS;
 }
 
@@ -1035,20 +1069,14 @@ qmckl_exit_code run_mo_mixed(qmckl_context context, DeviceState* ds, int64_t P, 
   return QMCKL_SUCCESS;
 }
 
-qmckl_exit_code run_mo(qmckl_context context, DeviceState* ds, int64_t P, const double* coord,
-                       double* ao_scratch, double* out, int comps) {
+// FP64-form MO VGL / value with the cusp adjustment where the context has one.
+qmckl_exit_code run_mo_fp64_form(qmckl_context context, DeviceState* ds, int64_t P, const double* coord, double* out,
+                                 int comps) {
   Context* ctx = ctx_of(context);
   const int64_t M = ctx->mo_basis.mo_num;
-  if (use_mixed(ctx)) return run_mo_mixed(context, ds, P, coord, out, comps);
-  qmckl_exit_code rc = sync_coef(context, ds);
-  if (rc != QMCKL_SUCCESS) return rc;
   const double *cr = nullptr, *cprm = nullptr;
-  rc = sync_cusp(context, ds, &cr, &cprm);
-  if (rc != QMCKL_SUCCESS) return rc;
-  rc = comps == 5 ? run_ao_vgl(context, ds, P, coord, ao_scratch, cr)
-                  : run_ao_value(context, ds, P, coord, ao_scratch, cr);
-  if (rc != QMCKL_SUCCESS) return rc;
-  rc = contract_f64(context, ds, P, comps, coord, P, ao_scratch, out);
+  qmckl_exit_code rc = sync_cusp(context, ds, &cr, &cprm);
+  if (rc == QMCKL_SUCCESS) rc = run_mo_f64(context, ds, P, comps, coord, cr, out);
   if (rc != QMCKL_SUCCESS) return rc;
   if (cr != nullptr)
     QB_CUDA(launch_cusp_mo(P, comps, coord, P, (int)ctx->nucleus.num, (const double*)ds->nucl.p, cr, cprm, (int)M, out,
@@ -1101,7 +1129,7 @@ void dev_detach(Context* ctx) {
                     &ds->ao_hessian, &ds->coef_rows, &ds->adj_coord, &ds->adj_buf, &ds->adj_part, &ds->adj_nucl,
                     &ds->tc3_coef, &ds->env, &ds->nuc_ao, &ds->forces, &ds->adj_wp, &ds->adj_ct,
                     &ds->cusp, &ds->ao_masked, &ds->en_dist, &ds->mo_hessian, &ds->kskip, &ds->kstat,
-                    &ds->tc_err, &ds->f64_sph, &ds->coef_f})
+                    &ds->tc_err, &ds->f64_sph, &ds->coef_f, &ds->f64_tiles})
     release(*b);
   if (ds->copy_stream) {
     cudaStreamSynchronize(ds->copy_stream);
@@ -1324,7 +1352,7 @@ qmckl_exit_code dev_provide_mo_vgl(qmckl_context context, double* host_out) {
     return qmckl_failwith(context, QMCKL_FAILURE, "qmckl_provide_mo_basis_mo_vgl", "only Gaussian basis sets are implemented");
   if (!ctx->ao_basis.provided)
     return qmckl_failwith(context, QMCKL_NOT_PROVIDED, "qmckl_ao_basis", NULL);
-  const int64_t P = ctx->point.num, A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
+  const int64_t P = ctx->point.num, M = ctx->mo_basis.mo_num;
   const size_t bytes = sizeof(double) * 5 * M * P;
   bool copied = false;   // set when the evaluation already copied the slices to host_out
   if (ctx->point.date > ctx->mo_basis.mo_vgl_date || ds->mo_vgl.cap < bytes) {
@@ -1334,26 +1362,8 @@ qmckl_exit_code dev_provide_mo_vgl(qmckl_context context, double* host_out) {
     if (rc != QMCKL_SUCCESS) return rc;
     if (use_mixed(ctx)) {
       rc = run_mo_mixed(context, ds, P, (const double*)ds->coord.p, (double*)ds->mo_vgl.p, 5, host_out, &copied);
-    } else if (!ctx->mo_basis.r_cusp.empty()) {
-      // FP64 form with the cusp adjustment: the AOs that it leaves out are
-      // zeroed in a separate AO array (the cached ao_vgl stays the plain one)
-      rc = ensure(context, ds->ao_masked, sizeof(double) * 5 * A * P, "qmckl_provide_mo_basis_mo_vgl");
-      if (rc != QMCKL_SUCCESS) return rc;
-      rc = run_mo(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_masked.p, (double*)ds->mo_vgl.p, 5);
     } else {
-      // FP64 form: the AO array is materialised (and cached) as in the reference
-      rc = sync_coef(context, ds);
-      if (rc != QMCKL_SUCCESS) return rc;
-      const size_t abytes = sizeof(double) * 5 * A * P;
-      if (ctx->point.date > ctx->ao_basis.ao_vgl_date || ds->ao_vgl.cap < abytes) {
-        rc = ensure(context, ds->ao_vgl, abytes, "qmckl_provide_ao_basis_ao_vgl");
-        if (rc != QMCKL_SUCCESS) return rc;
-        rc = run_ao_vgl(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_vgl.p);
-        if (rc != QMCKL_SUCCESS) return rc;
-        ctx->ao_basis.ao_vgl_date = ctx->date;
-      }
-      rc = contract_f64(context, ds, P, 5, (const double*)ds->coord.p, P, (const double*)ds->ao_vgl.p,
-                        (double*)ds->mo_vgl.p);
+      rc = run_mo_fp64_form(context, ds, P, (const double*)ds->coord.p, (double*)ds->mo_vgl.p, 5);
     }
     if (rc != QMCKL_SUCCESS) return rc;
     ctx->mo_basis.mo_vgl_date = ctx->date;
@@ -1368,7 +1378,7 @@ qmckl_exit_code dev_provide_mo_value(qmckl_context context, double* host_out) {
   DeviceState* ds = state(context);
   if (ctx->ao_basis.type != 'G')
     return qmckl_failwith(context, QMCKL_FAILURE, "qmckl_provide_mo_basis_mo_value", "only Gaussian basis sets are implemented");
-  const int64_t P = ctx->point.num, A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
+  const int64_t P = ctx->point.num, M = ctx->mo_basis.mo_num;
   const size_t bytes = sizeof(double) * M * P;
   if (ctx->point.date > ctx->mo_basis.mo_value_date || ds->mo_value.cap < bytes) {
     rc = ensure(context, ds->mo_value, bytes, "qmckl_provide_mo_basis_mo_value");
@@ -1384,23 +1394,8 @@ qmckl_exit_code dev_provide_mo_value(qmckl_context context, double* host_out) {
       if (rc != QMCKL_SUCCESS) return rc;
       if (use_mixed(ctx)) {
         rc = run_mo_mixed(context, ds, P, (const double*)ds->coord.p, (double*)ds->mo_value.p, 1);
-      } else if (!ctx->mo_basis.r_cusp.empty()) {
-        rc = ensure(context, ds->ao_masked, sizeof(double) * A * P, "qmckl_provide_mo_basis_mo_value");
-        if (rc != QMCKL_SUCCESS) return rc;
-        rc = run_mo(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_masked.p, (double*)ds->mo_value.p, 1);
       } else {
-        rc = sync_coef(context, ds);
-        if (rc != QMCKL_SUCCESS) return rc;
-        const size_t abytes = sizeof(double) * A * P;
-        if (ctx->point.date > ctx->ao_basis.ao_value_date || ds->ao_value.cap < abytes) {
-          rc = ensure(context, ds->ao_value, abytes, "qmckl_provide_ao_basis_ao_value");
-          if (rc != QMCKL_SUCCESS) return rc;
-          rc = run_ao_value(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_value.p);
-          if (rc != QMCKL_SUCCESS) return rc;
-          ctx->ao_basis.ao_value_date = ctx->date;
-        }
-        rc = contract_f64(context, ds, P, 1, (const double*)ds->coord.p, P, (const double*)ds->ao_value.p,
-                          (double*)ds->mo_value.p);
+        rc = run_mo_fp64_form(context, ds, P, (const double*)ds->coord.p, (double*)ds->mo_value.p, 1);
       }
       if (rc != QMCKL_SUCCESS) return rc;
     }
@@ -1633,13 +1628,7 @@ static qmckl_exit_code mo_device(qmckl_context context, const char* fname, int64
   Context* ctx = ctx_of(context);
   DeviceState* ds = state(context);
   if (use_mixed(ctx)) return run_mo_mixed(context, ds, point_num, d_coord, d_out, comps);
-  const size_t abytes = sizeof(double) * comps * ctx->ao_basis.ao_num * point_num;
-  DevBuf& scratch = comps == 5 ? ds->ao_vgl : ds->ao_value;
-  rc = ensure(context, scratch, abytes, fname);
-  if (rc != QMCKL_SUCCESS) return rc;
-  // the AO scratch no longer holds the context's cached points
-  if (comps == 5) ctx->ao_basis.ao_vgl_date = 0; else ctx->ao_basis.ao_value_date = 0;
-  return run_mo(context, ds, point_num, d_coord, (double*)scratch.p, d_out, comps);
+  return run_mo_fp64_form(context, ds, point_num, d_coord, d_out, comps);
 }
 
 qmckl_exit_code qmckl_b200_mo_vgl_device(qmckl_context context, const int64_t point_num, const double* d_coord,

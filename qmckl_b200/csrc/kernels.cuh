@@ -118,20 +118,37 @@ cudaError_t launch_ao_vgl_split(const DevTables& T, int64_t point_num, const dou
 cudaError_t launch_gemm_f64(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda,
                             const double* B, int64_t ldb, double* C, int64_t ldc, cudaStream_t s);
 
-// Tile-sparse FP64 MO contraction (gemm_f64.cu).  launch_f64_plan writes,
-// for tiles of 128 / comps points in the order perm, the list of AOs whose
-// shell reaches some point of the tile (basis order; sph[s] = double4 of the
-// shell's nucleus and squared screening radius, shell_ao[s] = int2 first AO
-// and AO count) into plan (f64_plan_bytes); launch_gemm_f64_sparse then
-// computes out[p][c][n] = sum over the tile's list of ao[p][c][k] * Bt[k][n]
-// (Bt: coefficient_t with ldb even and 16-byte aligned rows).
-size_t f64_plan_bytes(int64_t point_num, int comps, int64_t ao_num);
-cudaError_t launch_f64_plan(int64_t point_num, int comps, const double* coord, int64_t cstride, const int* perm,
-                            int shell_num, const void* sph, const void* shell_ao, int64_t ao_num, void* plan,
-                            cudaStream_t s);
-cudaError_t launch_gemm_f64_sparse(int64_t point_num, int comps, int64_t N, const double* ao, int64_t lda,
-                                   const int* perm, const void* plan, int64_t ao_num, const double* Bt, int64_t ldb,
-                                   double* C, int64_t ldc, cudaStream_t s);
+// Tile-sparse FP64 MO evaluation (f64_tiles.cu).  One record per shell: its
+// nucleus and the squared radius beyond which its AOs are exact zeros
+// (r2max, negative: no primitives), the nucleus screening bound
+// cutoff * range, its AOs [a0, a0 + na), its (exponent, coefficient) entries
+// [cb, ce) of DevTables::coef_ac, its angular momentum and nucleus.
+struct F64Shell {
+  double x, y, z, r2max, crange;
+  int32_t a0, na, cb, ce, l, nucl;
+};
+// Compact tiles of pts = f64_tile_points points each, f64_tile_bytes per
+// tile: ac[tile][ao_num][comps * pts + 4] (the first kcount[tile] rows hold
+// the tile's live AOs klist[tile][.]).
+struct F64Tiles {
+  int pts;
+  double* ac;
+  int* klist;
+  int* kcount;
+};
+int f64_tile_points(int comps, int64_t P);
+size_t f64_tile_bytes(int comps, int pts, int64_t ao_num);
+F64Tiles f64_tiles_at(void* scratch, int64_t ntiles, int comps, int pts, int64_t ao_num);
+// The AO tiles [tile0, tile0 + ntiles) of the points in the order perm
+// (null: as they are), coord [3][cstride]; cusp_r as in launch_ao_vgl_f64.
+cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const double* coord, int64_t cstride,
+                            const int* perm, int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff,
+                            bool dp_exp, const double* cusp_r, const F64Tiles& t, cudaStream_t s);
+// C[point][comps][N] of those tiles' points = AO tile * Bt (coefficient_t
+// with ldb even and 16-byte aligned rows).
+cudaError_t launch_tile_gemm(int64_t P, int comps, int64_t tile0, int64_t ntiles, int64_t N, int64_t ao_num,
+                             const F64Tiles& t, const int* perm, const double* Bt, int64_t ldb, double* C,
+                             cudaStream_t s);
 
 // Split-K FP64 GEMM with A transposed: part[z][m][n] = sum over the z-th K
 // range of A[k][m] * B[k][n] (A element (m, k) at A[k * lda + m]), for

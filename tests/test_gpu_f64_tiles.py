@@ -1,0 +1,87 @@
+"""FP64 MO evaluation over compact spatial tiles (f64_tiles.cu) at the edges
+of its tiles and of its dispatch, against the oracle (GPU).
+
+VGL tiles hold 32 points and value tiles 32 or, from 75,776 points on, 128;
+the contraction takes 80-column tiles once there are four CTAs per SM of them
+and narrower ones below; a tile's AO list is staged 1024 entries at a time;
+more than 1024 shells are numbered by another pass.  The bar is the parity
+bar of the FP64 form (1e-12, tests/conftest.py).
+"""
+import numpy as np
+import pytest
+import torch
+
+from conftest import parity_error
+from oracle import pyoracle as O
+from qmckl_b200 import gen
+from qmckl_b200 import qmckl as pq
+from qmckl_b200.system import make_context
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def _molecule(cid, m, seed):
+    d = gen.high_l_config(1) if cid == "hl" else gen.config(cid, walk_num=1)
+    rng = np.random.default_rng(seed)
+    q, _ = np.linalg.qr(rng.standard_normal((d["ao_num"], m)))
+    d["mo_coef"] = np.ascontiguousarray(q.T)
+    d["mo_num"] = m
+    return d
+
+
+def _points(d, P, seed):
+    rng = np.random.default_rng(seed)
+    xyz = np.asarray(d["nucl_coord"]).reshape(3, -1).T
+    return xyz[rng.integers(0, xyz.shape[0], P)] + rng.standard_normal((P, 3))
+
+
+def _device(ctx, pts, m, comps):
+    c = torch.tensor(np.ascontiguousarray(pts.T), dtype=torch.float64, device="cuda")
+    out = torch.full((pts.shape[0], comps, m), float("nan"), dtype=torch.float64, device="cuda")
+    f = pq.b200_mo_vgl_device if comps == 5 else pq.b200_mo_value_device
+    torch.cuda.synchronize()
+    f(ctx, pts.shape[0], c.data_ptr(), out.data_ptr())
+    pq.b200_synchronize(ctx)
+    return out.cpu().numpy()
+
+
+@pytest.mark.parametrize("cid,P,m,comps", [
+    (0, 1, 1, 5), (0, 31, 33, 5), (0, 32, 64, 5), (0, 33, 81, 5), (0, 1300, 90, 5), (0, 9473, 90, 5),
+    (0, 1, 1, 1), (0, 33, 31, 1), (0, 4736, 65, 1), (0, 75775, 17, 1), (0, 75777, 81, 1),
+    ("hl", 70, 120, 5), ("hl", 70, 101, 1), (1, 32, 160, 5), (4, 32, 350, 5), (4, 40, 33, 1)])
+def test_tiles(cid, P, m, comps):
+    d = _molecule(cid, m, 100 + P)
+    pts = _points(d, P, 200 + P)
+    ctx = make_context(d, points=False, form=pq.FORM_FP64)
+    try:
+        got = _device(ctx, pts, m, comps)
+    finally:
+        pq.context_destroy(ctx)
+    if comps == 5:
+        ref = O.mo_vgl(d["mo_coef"], O.ao_vgl(O.Basis(d), pts, d["nucl_coord"]))
+    else:
+        ref = O.mo_value(d["mo_coef"], O.ao_value(O.Basis(d), pts, d["nucl_coord"])).reshape(P, 1, m)
+    assert parity_error(got, ref) < TOL
+
+
+def test_nan_point_stays_alone():
+    d = _molecule(0, 90, 5)
+    pts = _points(d, 100, 6)
+    ctx = make_context(d, points=False, form=pq.FORM_FP64)
+    try:
+        bad = pts.copy()
+        bad[17, 1] = np.nan
+        got = _device(ctx, bad, 90, 5)
+        far = pts.copy()
+        far[17] = [np.inf, 0.0, 0.0]
+        got_far = _device(ctx, far, 90, 5)
+    finally:
+        pq.context_destroy(ctx)
+    ref = O.mo_vgl(d["mo_coef"], O.ao_vgl(O.Basis(d), pts, d["nucl_coord"]))
+    keep = np.arange(100) != 17
+    assert np.isnan(got[17]).any()
+    assert parity_error(got[keep], ref[keep]) < TOL
+    assert (got_far[17] == 0.0).all()
+    assert parity_error(got_far[keep], ref[keep]) < TOL
