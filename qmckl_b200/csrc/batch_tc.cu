@@ -425,7 +425,7 @@ struct Batch {
   std::vector<BatchSys> sys;
   int64_t coord_total = 0, out_total = 0, perm_total = 0;
   int n_tile_max = 0, rec_max = 0, kb_max = 0;
-  DBuf coef, krec, kskip, desc, tmaps, items, ctl, perm, keys, counts, loop_err, nucl, env;
+  DBuf coef, krec, kskip, desc, tmaps, items, ctl, perm, sort, loop_err, nucl, env;
   int n_items = 0;
   // tuning
   int prod_warps = 16;
@@ -781,7 +781,7 @@ qmckl_exit_code qmckl_b200_batch_destroy(qmckl_b200_batch batch) {
   cudaSetDevice(B->device);
   if (B->stream) cudaStreamSynchronize(B->stream);
   drop_graph(B);
-  for (DBuf* b : {&B->coef, &B->krec, &B->kskip, &B->desc, &B->tmaps, &B->items, &B->ctl, &B->perm, &B->keys, &B->counts,
+  for (DBuf* b : {&B->coef, &B->krec, &B->kskip, &B->desc, &B->tmaps, &B->items, &B->ctl, &B->perm, &B->sort,
                   &B->loop_err, &B->nucl, &B->env})
     if (b->p) cudaFree(b->p);
   if (B->h_err) cudaFreeHost(B->h_err);
@@ -885,8 +885,7 @@ qmckl_exit_code qmckl_b200_batch_mo_vgl_loop_device(qmckl_b200_batch batch, cons
   cudaSetDevice(B->device);
   int64_t pmax = 0;
   for (auto& S : B->sys) pmax = std::max(pmax, S.P);
-  if (dalloc(B->keys, sizeof(int) * std::max<int64_t>(pmax, 1)) != cudaSuccess ||
-      dalloc(B->counts, sizeof(unsigned) * (kSortCells + 1)) != cudaSuccess ||
+  if (dalloc(B->sort, std::max<size_t>(point_order_bytes(pmax), 1)) != cudaSuccess ||
       dalloc(B->loop_err, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     return QMCKL_ALLOCATION_FAILED;
@@ -897,7 +896,7 @@ qmckl_exit_code qmckl_b200_batch_mo_vgl_loop_device(qmckl_b200_batch batch, cons
     if (S.P == 0) continue;
     const double* c = d_coord + S.coord_off;
     int* pm = (int*)B->perm.p + S.perm_off;
-    e = point_order(c, S.P, S.lo, S.hi, (int*)B->keys.p, (unsigned*)B->counts.p, pm, B->stream);
+    e = point_order(c, S.P, S.lo, S.hi, B->sort.p, pm, B->stream);
     if (e == cudaSuccess)
       e = tc_launch_fused(S.plan, S.P, 5, c, S.cutoff, S.map, (const char*)B->krec.p + S.krec_off, S.rec_bytes, pm,
                           (const char*)B->coef.p + S.coef_off, S.rb, d_mo_vgl + S.out_off, (int*)B->loop_err.p,

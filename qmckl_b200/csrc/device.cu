@@ -346,7 +346,7 @@ struct DeviceState {
   bool fused = true;
   // per-K-block records of the fused kernel (rebuilt on basis or nuclear moves)
   DevBuf krec;
-  DevBuf order;      // point order of the fused kernel: keys[P], perm[P], cell counts
+  DevBuf order;      // point order: perm[P], the sort's scratch, the fused kernel's tile plan
   int rec_bytes = 0;
   uint64_t krec_basis_version = ~0ull, krec_nucl_version = ~0ull;
   // derivatives: AO Hessian and the MO VGL adjoint (FP64 coefficient [mo][ao],
@@ -863,6 +863,10 @@ qmckl_exit_code prepare_mixed(qmckl_context context, DeviceState* ds) {
   return QMCKL_SUCCESS;
 }
 
+// Point order of P points: perm[P], then the sort's scratch (256-byte aligned).
+size_t perm_bytes(int64_t P) { return (sizeof(int) * (size_t)P + 255) / 256 * 256; }
+size_t order_bytes(int64_t P) { return perm_bytes(P) + (point_order_bytes(P) + 255) / 256 * 256; }
+
 // Box of the nuclei, widened by 4 bohr: the grid of the spatial point order.
 void nucleus_box(const Context* ctx, double* lo, double* hi) {
   const int64_t N = ctx->nucleus.num;
@@ -962,17 +966,14 @@ qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, in
   const int64_t most = std::max<int64_t>(1, budget / (int64_t)f64_tile_bytes(comps, pts, A));
   const int64_t chunks = (tiles + most - 1) / most;
   const int64_t chunk = (tiles + chunks - 1) / chunks;
-  const size_t sort_bytes = sizeof(int) * 2 * (size_t)P + sizeof(unsigned int) * (kSortCells + 1);
-  rc = ensure(context, ds->order, sort_bytes, fname);
+  rc = ensure(context, ds->order, order_bytes(P), fname);
   if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, f64_tile_bytes(comps, pts, A) * (size_t)chunk, fname);
   if (rc != QMCKL_SUCCESS) return rc;
-  int* keys = (int*)ds->order.p;
-  int* perm = keys + P;
-  unsigned int* counts = (unsigned int*)(perm + P);
+  int* perm = (int*)ds->order.p;
   double lo[3], hi[3];
   nucleus_box(ctx, lo, hi);
   if (tiles > 1)
-    QB_CUDA(point_order(coord, P, lo, hi, keys, counts, perm, ds->stream, P), fname);
+    QB_CUDA(point_order(coord, P, lo, hi, (uint8_t*)ds->order.p + perm_bytes(P), perm, ds->stream, P), fname);
   else
     perm = nullptr;   // one tile: any order
   const F64Tiles t = f64_tiles_at(ds->f64_tiles.p, chunk, comps, pts, A);
@@ -1007,14 +1008,12 @@ qmckl_exit_code run_mo_mixed(qmckl_context context, DeviceState* ds, int64_t P, 
     if (ok && tc_fused_smem(ds->tc, comps, ds->rec_bytes) <= 232448) {
       // spatial order of the points, then the fused AO -> MO kernel (the AO
       // pieces never leave shared memory)
-      // scratch: keys[P], perm[P], cell counts, then the tile plan (256-byte aligned)
-      const size_t sort_bytes = (sizeof(int) * 2 * (size_t)P + sizeof(unsigned int) * (kSortCells + 1) + 255) / 256 * 256;
+      // scratch: the point order, then the tile plan (256-byte aligned)
+      const size_t sort_bytes = order_bytes(P);
       const size_t obytes = sort_bytes + tc_tile_plan_bytes(ds->tc, P, comps);
       qmckl_exit_code rc = ensure(context, ds->order, obytes, "qmckl_b200_mo_mixed");
       if (rc != QMCKL_SUCCESS) return rc;
-      int* keys = (int*)ds->order.p;
-      int* perm = keys + P;
-      unsigned int* counts = (unsigned int*)(perm + P);
+      int* perm = (int*)ds->order.p;
       void* tplan = (uint8_t*)ds->order.p + sort_bytes;
       double lo[3], hi[3];
       nucleus_box(ctx, lo, hi);
@@ -1031,7 +1030,8 @@ qmckl_exit_code run_mo_mixed(qmckl_context context, DeviceState* ds, int64_t P, 
       for (int64_t a = 0; a < P; a += step, ++slice) {
         const int64_t n = std::min(step, P - a);
         double* o = out + a * comps * M;
-        QB_CUDA(point_order(coord + a, n, lo, hi, keys, counts, perm, ds->stream, P), "qmckl_b200_mo_mixed");
+        QB_CUDA(point_order(coord + a, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(P), perm, ds->stream, P),
+                "qmckl_b200_mo_mixed");
         QB_CUDA(tc_run_fused(ds->T, ds->tc, n, comps, coord + a, cutoff_of(ctx), ds->tc_coef.p, ds->krec.p,
                              ds->rec_bytes, perm, rb, o, (int*)ds->tc_err.p, ds->stream, P, ds->kskip.p,
                              (unsigned long long*)ds->kstat.p, tplan),

@@ -570,110 +570,3 @@ cudaError_t tc_set_late_warps(unsigned int ns) {
 }
 
 }  // namespace qb
-
-// ---------------------------------------------------------------- point order
-//
-// Tiles of spatially close points share their zero AOs, which the producers
-// of the fused kernel skip a pair of AOs at a time.  Points are bucketed into
-// the cells of a 32^3 grid over the box of the nuclei (coordinates clamped),
-// ordered by Morton code.
-// The order within a cell does not affect any result: every output row is a
-// function of its own point only.
-namespace qb {
-namespace {
-
-__device__ __forceinline__ unsigned int spread5(unsigned int x) {   // 5 bits -> every third bit
-  x &= 31u;
-  x = (x | (x << 8)) & 0x0300F00Fu;
-  x = (x | (x << 4)) & 0x030C30C3u;
-  x = (x | (x << 2)) & 0x09249249u;
-  return x;
-}
-
-__global__ void point_keys_kernel(const double* __restrict__ coord, int64_t P, int64_t cstride, double3 origin,
-                                  double inv_cell, int* __restrict__ keys, unsigned int* __restrict__ counts) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (int64_t)gridDim.x * blockDim.x) {
-    int c[3];
-    const double o[3] = {origin.x, origin.y, origin.z};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double v = floor((coord[p + d * cstride] - o[d]) * inv_cell);
-      c[d] = (int)fmin(31.0, fmax(0.0, v));
-    }
-    const int key = (int)(spread5(c[0]) | (spread5(c[1]) << 1) | (spread5(c[2]) << 2));
-    keys[p] = key;
-    atomicAdd(&counts[key], 1u);
-  }
-}
-
-// exclusive scan of kSortCells counts in one CTA of 1024 threads: warp w
-// scans cells [1024 w, 1024 w + 1024) as 32 rows of 32 (coalesced loads and
-// stores, shuffles within a row, a carry from row to row), then the warps'
-// totals are scanned and added
-__global__ void __launch_bounds__(1024) scan_cells_kernel(unsigned int* counts) {
-  static_assert(kSortCells == 32 * 1024, "32 warps x 32 rows x 32 cells");
-  __shared__ unsigned int wbase[32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  unsigned int* c = counts + warp * 1024;
-  unsigned int v[32];
-  unsigned int carry = 0u;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const unsigned int x = c[32 * i + lane];
-    unsigned int y = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int t = __shfl_up_sync(0xffffffffu, y, o);
-      if (lane >= o) y += t;
-    }
-    v[i] = carry + y - x;
-    carry += __shfl_sync(0xffffffffu, y, 31);
-  }
-  if (lane == 0) wbase[warp] = carry;
-  __syncthreads();
-  if (warp == 0) {
-    const unsigned int x = wbase[lane];
-    unsigned int y = x;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned int t = __shfl_up_sync(0xffffffffu, y, o);
-      if (lane >= o) y += t;
-    }
-    wbase[lane] = y - x;
-  }
-  __syncthreads();
-  const unsigned int base = wbase[warp];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) c[32 * i + lane] = base + v[i];
-}
-
-__global__ void scatter_points_kernel(const int* __restrict__ keys, int64_t P, unsigned int* __restrict__ offsets,
-                                      int* __restrict__ perm) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < P; p += (int64_t)gridDim.x * blockDim.x) {
-    const unsigned int pos = atomicAdd(&offsets[keys[p]], 1u);
-    perm[pos] = (int)p;
-  }
-}
-
-}  // namespace
-
-cudaError_t point_order(const double* coord, int64_t point_num, const double* box_lo, const double* box_hi,
-                        int* keys, unsigned int* counts, int* perm, cudaStream_t s, int64_t cstride) {
-  if (cstride < point_num) cstride = point_num;
-  // 32 cells per axis over the box of the nuclei (cells at least 1 bohr wide)
-  double ext = 0.0;
-  for (int d = 0; d < 3; ++d) ext = std::max(ext, box_hi[d] - box_lo[d]);
-  const double cell = std::max(1.0, ext / 32.0);
-  const double3 origin = make_double3(box_lo[0], box_lo[1], box_lo[2]);
-  if (point_num <= 0) return cudaSuccess;
-  cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(unsigned int) * kSortCells, s);
-  if (e != cudaSuccess) return e;
-  const int grid = (int)std::min<int64_t>((point_num + 255) / 256, 148 * 8);
-  point_keys_kernel<<<grid, 256, 0, s>>>(coord, point_num, cstride, origin, 1.0 / cell, keys, counts);
-  scan_cells_kernel<<<1, 1024, 0, s>>>(counts);
-  scatter_points_kernel<<<grid, 256, 0, s>>>(keys, point_num, counts, perm);
-  count_launch(3);
-  return cudaGetLastError();
-}
-
-}  // namespace qb

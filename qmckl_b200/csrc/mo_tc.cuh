@@ -98,14 +98,14 @@ cudaError_t tc_launch_fused(const TcPlan& plan, int64_t point_num, int comps, co
 // in this process: producer warps holding a chunk of a skipped k-step sleep
 // `ns` nanoseconds before their stage wait (0: off, the kernel without it).
 cudaError_t tc_set_late_warps(unsigned int ns);
-// Spatial order of points (32^3 cells over [box_lo, box_hi], Morton order) by
-// a counting sort: perm[P]; keys[P] and counts[kSortCells + 1] are scratch.
-// cstride: distance between the x, y and z blocks of coord (default
-// point_num; larger for a slice of a bigger [3][N] array).  The fused
-// kernels take the same stride.
-constexpr int kSortCells = 1 << 15;
+// Spatial order of points (point_order.cu): perm[P] <- the points in Morton
+// order of 32^3 cells over [box_lo, box_hi], in their own order within a cell.
+// scratch: point_order_bytes(P) bytes, 256-byte aligned.  cstride: distance
+// between the x, y and z blocks of coord (default point_num; larger for a
+// slice of a bigger [3][N] array).  The fused kernels take the same stride.
+size_t point_order_bytes(int64_t point_num);
 cudaError_t point_order(const double* coord, int64_t point_num, const double* box_lo, const double* box_hi,
-                        int* keys, unsigned int* counts, int* perm, cudaStream_t s, int64_t cstride = -1);
+                        void* scratch, int* perm, cudaStream_t s, int64_t cstride = -1);
 // dynamic shared memory of the fused kernel (must stay <= 227 KB)
 size_t tc_fused_smem(const TcPlan& plan, int comps, int rec_bytes);
 

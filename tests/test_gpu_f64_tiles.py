@@ -4,7 +4,8 @@ of its tiles and of its dispatch, against the oracle (GPU).
 VGL tiles hold 32 points and value tiles 32 or, from 75,776 points on, 128;
 the contraction takes 80-column tiles once there are four CTAs per SM of them
 and narrower ones below; a tile's AO list is staged 1024 entries at a time;
-more than 1024 shells are numbered by another pass.  The bar is the parity
+more than 1024 shells are numbered by another pass; up to 4096 points are put
+in order by one CTA.  The bar is the parity
 bar of the FP64 form (1e-12, tests/conftest.py).
 """
 import numpy as np
@@ -48,7 +49,7 @@ def _device(ctx, pts, m, comps):
 
 
 @pytest.mark.parametrize("cid,P,m,comps", [
-    (0, 1, 1, 5), (0, 31, 33, 5), (0, 32, 64, 5), (0, 33, 81, 5), (0, 1300, 90, 5), (0, 9473, 90, 5),
+    (0, 1, 1, 5), (0, 31, 33, 5), (0, 32, 64, 5), (0, 33, 81, 5), (0, 1300, 90, 5), (0, 4096, 20, 5), (0, 4097, 20, 5), (0, 9473, 90, 5),
     (0, 1, 1, 1), (0, 33, 31, 1), (0, 4736, 65, 1), (0, 75775, 17, 1), (0, 75777, 81, 1),
     ("hl", 70, 120, 5), ("hl", 70, 101, 1), (1, 32, 160, 5), (4, 32, 350, 5), (4, 40, 33, 1)])
 def test_tiles(cid, P, m, comps):
