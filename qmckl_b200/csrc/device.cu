@@ -352,8 +352,7 @@ struct DeviceState {
   // derivatives: AO Hessian and the MO VGL adjoint (FP64 coefficient [mo][ao],
   // per-chunk coordinates, AO / pulled-back weight buffer, split-K partials)
   DevBuf ao_hessian;
-  uint64_t coef_rows_version = ~0ull;
-  DevBuf coef_rows, adj_coord, adj_buf, adj_part, adj_nucl;
+  DevBuf adj_coord, adj_buf, adj_part, adj_nucl;
   // mixed-form adjoint: bfloat16 pieces of the weights and of coefficient_t
   uint64_t adj_ct_version = ~0ull;
   DevBuf adj_wp, adj_ct;
@@ -1126,7 +1125,7 @@ void dev_detach(Context* ctx) {
   if (ds->stream) cudaStreamSynchronize(ds->stream);
   for (DevBuf* b : {&ds->tables, &ds->nucl, &ds->coord, &ds->prim_vgl, &ds->shell_vgl, &ds->ao_vgl, &ds->ao_value,
                     &ds->mo_vgl, &ds->mo_value, &ds->coef_t, &ds->tc_coef, &ds->tc_a, &ds->krec, &ds->order,
-                    &ds->ao_hessian, &ds->coef_rows, &ds->adj_coord, &ds->adj_buf, &ds->adj_part, &ds->adj_nucl,
+                    &ds->ao_hessian, &ds->adj_coord, &ds->adj_buf, &ds->adj_part, &ds->adj_nucl,
                     &ds->tc3_coef, &ds->env, &ds->nuc_ao, &ds->forces, &ds->adj_wp, &ds->adj_ct,
                     &ds->cusp, &ds->ao_masked, &ds->en_dist, &ds->mo_hessian, &ds->kskip, &ds->kstat,
                     &ds->tc_err, &ds->f64_sph, &ds->coef_f, &ds->f64_tiles})
@@ -1791,9 +1790,77 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
       QB_CUDA(tc_gemm_nt(ds->adj_wp.p, ldw, rows * ldw, rows, M, ds->adj_ct.p, ldw, A * ldw, A, (float*)buf, A, err,
                          s),
               fname);
-      QB_CUDA(launch_mo_adjoint_nuclear(ds->T, n, cc, n, cutoff, true, buf, gnucl,
+      QB_CUDA(launch_mo_adjoint_nuclear(ds->T, n, cc, n, cutoff, (const float*)buf, gnucl,
                                         d_grad_coord ? d_grad_coord + p0 : nullptr, P, s),
               fname);
+    }
+  }
+  return QMCKL_SUCCESS;
+}
+
+// FP64 adjoint over compact spatial tiles (f64_tiles.cu).  Per chunk of
+// tiles: the AOs and their lists; the weights in tile order; dL/dC as
+// per-tile products summed over the tiles in order; the weights pulled back to
+// the listed AOs, over the AO tile; the derivative kernel.  Only the AOs that
+// reach a tile take part.
+qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, const double* d_coord,
+                            const double* d_weight, double* d_grad_coef, double* d_grad_nucl, double* d_grad_coord) {
+  const char* fname = "qmckl_b200_mo_vgl_adjoint_device";
+  Context* ctx = ctx_of(context);
+  const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num, S = ctx->ao_basis.shell_num;
+  const double cutoff = cutoff_of(ctx);
+  cudaStream_t s = ds->stream;
+  const double* Ct = nullptr;
+  int64_t ldc = 0;
+  qmckl_exit_code rc = sync_f64_shells(context, ds);
+  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Ct, &ldc);
+  if (rc != QMCKL_SUCCESS) return rc;
+  const int64_t ldw = M + (M & 1);
+  const int pts = f64_tile_points(5, P);
+  const int64_t tiles = (P + pts - 1) / pts;
+  // per tile, each part a multiple of 16 bytes: AO tile with its list, live
+  // shells, list positions, weights, dL/dC products
+  const size_t b_ao = (f64_tile_bytes(5, pts, A) + 15) / 16 * 16, b_live = (sizeof(int2) * (size_t)S + 16) / 16 * 16,
+               b_inv = (sizeof(int) * (size_t)A + 15) / 16 * 16, b_n = 16, b_w = sizeof(double) * 5 * (size_t)pts * (size_t)ldw,
+               b_part = d_grad_coef ? sizeof(double) * (size_t)A * (size_t)ldw : 0;
+  const size_t per_tile = b_ao + b_live + b_inv + b_n + b_w + b_part;
+  const int64_t budget = (int64_t)4 << 30;
+  const int64_t most = std::max<int64_t>(1, budget / (int64_t)per_tile);
+  const int64_t chunks = (tiles + most - 1) / most;
+  const int64_t chunk = (tiles + chunks - 1) / chunks;
+  rc = ensure(context, ds->order, order_bytes(P), fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, per_tile * (size_t)chunk, fname);
+  if (rc != QMCKL_SUCCESS) return rc;
+  int* perm = (int*)ds->order.p;
+  double lo[3], hi[3];
+  nucleus_box(ctx, lo, hi);
+  if (tiles > 1)
+    QB_CUDA(point_order(d_coord, P, lo, hi, (uint8_t*)ds->order.p + perm_bytes(P), perm, s, P), fname);
+  else
+    perm = nullptr;
+  uint8_t* at = (uint8_t*)ds->f64_tiles.p;
+  double* part = (double*)at;
+  at += b_part * (size_t)chunk;
+  double* ws = (double*)at;
+  at += b_w * (size_t)chunk;
+  F64Tiles t = f64_tiles_at(at, chunk, 5, pts, A);
+  at += b_ao * (size_t)chunk;
+  t.adj.live = (int2*)at;
+  at += b_live * (size_t)chunk;
+  t.adj.nlive = (int*)at;
+  at += b_n * (size_t)chunk;
+  int* inv = (int*)at;
+  t.adj.inv = d_grad_coef ? inv : nullptr;
+  const F64Shell* sh = (const F64Shell*)ds->f64_sph.p;
+  for (int64_t t0 = 0; t0 < tiles; t0 += chunk) {
+    const int64_t n = std::min(chunk, tiles - t0);
+    if (d_grad_coef) QB_CUDA(cudaMemsetAsync(inv, 0xff, sizeof(int) * (size_t)(n * A), s), fname);
+    QB_CUDA(launch_ao_tiles(ds->T, P, 5, d_coord, P, perm, t0, n, sh, cutoff, true, nullptr, t, s), fname);
+    QB_CUDA(launch_weight_tiles(P, t0, n, d_weight, M, perm, ws, ldw, s), fname);
+    if (d_grad_coef) QB_CUDA(launch_adj_coef(n, A, M, t, ws, ldw, part, d_grad_coef, t0 > 0, s), fname);
+    if (d_grad_nucl || d_grad_coord) {
+      QB_CUDA(launch_adj_pullback(n, A, M, t, ws, ldw, Ct, ldc, s), fname);
+      QB_CUDA(launch_tile_deriv(ds->T, P, d_coord, P, perm, t0, n, sh, cutoff, t, d_grad_nucl, d_grad_coord, P, s), fname);
     }
   }
   return QMCKL_SUCCESS;
@@ -1817,53 +1884,13 @@ qmckl_exit_code qmckl_b200_mo_vgl_adjoint_device(qmckl_context context, const in
   DeviceState* ds = state(context);
   const int64_t P = point_num, A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num, N = ctx->nucleus.num;
   const bool mixed = use_mixed(ctx) || ctx->precision <= 23;
-  const double cutoff = cutoff_of(ctx);
   cudaStream_t s = ds->stream;
   if (d_grad_coef) QB_CUDA(cudaMemsetAsync(d_grad_coef, 0, sizeof(double) * M * A, s), fname);
   if (d_grad_nucl) QB_CUDA(cudaMemsetAsync(d_grad_nucl, 0, sizeof(double) * 3 * N, s), fname);
   if (d_grad_coord) QB_CUDA(cudaMemsetAsync(d_grad_coord, 0, sizeof(double) * 3 * P, s), fname);
   if (P == 0 || (!d_grad_coef && !d_grad_nucl && !d_grad_coord)) return QMCKL_SUCCESS;
   if (mixed) return adjoint_mixed(context, ds, P, d_coord, d_weight, d_grad_coef, d_grad_nucl, d_grad_coord);
-  // FP64 coefficient rows [mo][ao] for G = W C
-  if (ds->coef_rows_version != ctx->mo_basis.coef_version || !ds->coef_rows.p) {
-    rc = ensure(context, ds->coef_rows, sizeof(double) * M * A, fname);
-    if (rc != QMCKL_SUCCESS) return rc;
-    QB_CUDA(cudaMemcpyAsync(ds->coef_rows.p, ctx->mo_basis.coefficient.data(), sizeof(double) * M * A,
-                            cudaMemcpyHostToDevice, s), fname);
-    ds->coef_rows_version = ctx->mo_basis.coef_version;
-  }
-  const int64_t budget = (int64_t)2 << 30;
-  const int64_t chunk = std::min<int64_t>(P, std::max<int64_t>(64, budget / (int64_t)(40 * A)));
-  // split-K count: about two CTAs per SM for the (ao x mo) output tiles
-  const int64_t tiles = ((A + 127) / 128) * ((M + 79) / 80);
-  const int splits = (int)std::max<int64_t>(1, std::min<int64_t>(32, (2 * 148 + tiles - 1) / tiles));
-  rc = ensure(context, ds->adj_coord, sizeof(double) * 3 * chunk, fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_buf, sizeof(double) * 5 * chunk * A, fname);
-  if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_part, sizeof(double) * splits * A * M, fname);
-  if (rc == QMCKL_SUCCESS && !d_grad_nucl) rc = ensure(context, ds->adj_nucl, sizeof(double) * 3 * N, fname);
-  if (rc != QMCKL_SUCCESS) return rc;
-  double* gnucl = d_grad_nucl ? d_grad_nucl : (double*)ds->adj_nucl.p;
-  double* buf = (double*)ds->adj_buf.p;
-  double* cc = (double*)ds->adj_coord.p;
-  for (int64_t p0 = 0; p0 < P; p0 += chunk) {
-    const int64_t n = std::min<int64_t>(chunk, P - p0);
-    const double* w = d_weight + p0 * 5 * M;
-    QB_CUDA(cudaMemcpy2DAsync(cc, sizeof(double) * n, d_coord + p0, sizeof(double) * P, sizeof(double) * n, 3,
-                              cudaMemcpyDeviceToDevice, s), fname);
-    if (d_grad_coef) {
-      QB_CUDA(launch_ao_vgl_f64(ds->T, n, cc, cutoff, !mixed, buf, s), fname);
-      QB_CUDA(launch_gemm_f64_tn_split(A, M, 5 * n, buf, A, w, M, (double*)ds->adj_part.p, splits, s), fname);
-      QB_CUDA(launch_add_transposed((const double*)ds->adj_part.p, splits, A, M, d_grad_coef, true, s), fname);
-    }
-    if (d_grad_nucl || d_grad_coord) {
-      QB_CUDA(launch_gemm_f64(5 * n, A, M, w, M, (const double*)ds->coef_rows.p, A, buf, A, s), fname);
-      QB_CUDA(launch_mo_adjoint_nuclear(ds->T, n, cc, n, cutoff, mixed, buf, gnucl,
-                                        d_grad_coord ? d_grad_coord + p0 : nullptr, P, s),
-              fname);
-    }
-  }
-  // the AO scratch of the FP64 form was not touched; cached arrays stay valid
-  return QMCKL_SUCCESS;
+  return adjoint_f64(context, ds, P, d_coord, d_weight, d_grad_coef, d_grad_nucl, d_grad_coord);
 }
 
 }  // extern "C"

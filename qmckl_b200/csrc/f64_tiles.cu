@@ -135,7 +135,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
                 const int64_t tile0, const int shell_num, const F64Shell* __restrict__ sh,
                 const double2* __restrict__ prim, const double* __restrict__ factor, const double cutoff,
                 const bool dp_exp, const double* __restrict__ cusp_r, const int64_t kmax, double* __restrict__ ac,
-                int* __restrict__ klist, int* __restrict__ kcount) {
+                int* __restrict__ klist, int* __restrict__ kcount, const AdjTables adj) {
   constexpr int G = TP / 32;
   constexpr int LD = COMPS * TP + 4;
   static_assert(TP % 32 == 0 && G <= 4, "a tile is 1 to 4 warps of points");
@@ -289,8 +289,16 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
       const F64Shell S = sh[live[q] & 0xffffff];
       const int k = lpos[q];
       for (int i = 0; i < S.na; ++i) kl[k + i] = S.a0 + i;
+      if (adj.live != nullptr) {
+        adj.live[tile * shell_num + q] = make_int2(live[q] & 0xffffff, k);
+        if (adj.inv != nullptr)
+          for (int i = 0; i < S.na; ++i) adj.inv[tile * kmax + S.a0 + i] = k + i;
+      }
     }
-    if (tid == 0) kcount[tile] = nao;
+    if (tid == 0) {
+      kcount[tile] = nao;
+      if (adj.live != nullptr) adj.nlive[tile] = nlive;
+    }
   }
   double* __restrict__ act = ac + (size_t)tile * kmax * LD;
   const int units = nlive * G;
@@ -497,6 +505,242 @@ cudaError_t run_tile_gemm(int64_t P, int64_t tile0, int64_t ntiles, int64_t N, c
   return cudaGetLastError();
 }
 
+// ---------------------------------------------------------------- adjoint
+
+constexpr int kAdjPts = 32, kAdjRows = 5 * kAdjPts, kAdjLd = kAdjRows + 4;   // tiles of 32 points
+
+// Loss weights in tile order: ws[tile][c * 32 + p][ldw] = w[perm point][c][.]
+// (zero past the MOs and past the points); a warp per row.
+__global__ void __launch_bounds__(256)
+weight_tiles_kernel(const int64_t P, const int64_t tile0, const int64_t rows, const double* __restrict__ w,
+                    const int64_t M, const int* __restrict__ perm, double* __restrict__ ws, const int64_t ldw) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
+    const int64_t tile = r / kAdjRows;
+    const int pos = (int)(r - tile * kAdjRows), c = pos / kAdjPts;
+    const int64_t q = (tile0 + tile) * kAdjPts + pos % kAdjPts;
+    double* o = ws + r * ldw;
+    if (q < P) {
+      const double* src = w + ((perm ? (int64_t)perm[q] : q) * 5 + c) * M;
+      for (int64_t n = lane; n < ldw; n += 32) o[n] = n < M ? src[n] : 0.0;
+    } else {
+      for (int64_t n = lane; n < ldw; n += 32) o[n] = 0.0;
+    }
+  }
+}
+
+// The two contractions of the adjoint over a tile's AO list, 32 MF list rows by
+// 80 columns per CTA (8 warps as 4 x 2), 16-step k in STG stages of 16-byte
+// cp.async, two CTAs per SM; bound by the FP64 tensor pipe as the forward.
+//   COEF: part[tile][m][n] = sum over the tile's positions of ac[m][pos] *
+//         ws[pos][n], the tile's share of dL/dC (columns: MOs)
+//   else: ac[m][pos] = sum over MOs of Ct[list[m]][mo] * ws[pos][mo], the
+//         weights pulled back to the AOs (columns: positions; overwrites ac)
+// The 8-row and 8-column blocks are dealt to the warps in turn and blocks past
+// the list or the columns are skipped.  Tiles of 32 points, although their
+// products are short (160 rows): tiles of 128 points keep 31% of the AOs of
+// the 2000-AO molecule against 25%, and with their dead 32-point groups
+// skipped the warps wait for one another (0.68 and 0.64 ms against 0.56 and
+// 0.57 = 30 TFLOP/s on 20,352 points; as dense products over all AOs they
+// took 3.3 and 2.2 ms).
+template <bool COEF, int MF, int STG>
+__global__ void __launch_bounds__(256, 2)
+adj_gemm_kernel(double* __restrict__ ac, const int* __restrict__ klist, const int* __restrict__ kcount,
+                const int64_t kmax, const int64_t M, const double* __restrict__ ws, const int64_t ldw,
+                const double* __restrict__ Ct, const int64_t ldc, double* __restrict__ part) {
+  constexpr int BM = 32 * MF, NT = 5, BN = 80, LDR = BKT + 4, LDB = BN + 4;
+  constexpr int B_STAGE = COEF ? BKT * LDB : BN * LDR;
+  extern __shared__ __align__(16) double smem[];
+  double* As = smem;                          // [STG][BM][LDR]
+  double* Bs = smem + STG * BM * LDR;        // COEF: [STG][BKT][LDB], else [STG][BN][LDR]
+  const int64_t tile = blockIdx.z;
+  const int nk = kcount[tile];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int turn = (int)(blockIdx.y + blockIdx.z);
+  const int wm = ((warp >> 1) + turn) & 3, wn = (warp + turn) & 1;
+  const int g = lane >> 2, t = lane & 3;
+  const int n0 = (int)blockIdx.x * BN;
+  const int K = COEF ? kAdjRows : (int)M;
+  const int ncol = COEF ? (int)M : kAdjRows;
+  const int ktiles = (K + BKT - 1) / BKT;
+  const int nj = (min(BN / 8, (ncol - n0 + 7) / 8) - wn + 1) / 2;     // column blocks wn, wn + 2, ...
+  const double* wt = ws + (size_t)tile * kAdjRows * ldw;
+  for (int m0 = (int)blockIdx.y * BM; m0 < nk; m0 += (int)gridDim.y * BM) {
+    const int ni = (min(4 * MF, (nk - m0 + 7) / 8) - wm + 3) / 4;           // row blocks wm, wm + 4, ...
+    // the MF A rows this thread copies a 16-byte piece of
+    const int a_r = tid >> 3, a_c = (tid & 7) * 2;
+    const double* arow[MF];
+#pragma unroll
+    for (int i = 0; i < MF; ++i) {
+      const int m = m0 + a_r + 32 * i;
+      arow[i] = m >= nk ? nullptr
+                : COEF  ? ac + ((size_t)tile * kmax + m) * kAdjLd + a_c
+                        : Ct + (int64_t)klist[tile * kmax + m] * ldc + a_c;
+    }
+    double acc[MF][NT][2];
+#pragma unroll
+    for (int i = 0; i < MF; ++i)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    auto load = [&](int kt, int st) {
+      const int k0 = kt * BKT;
+      double* as = As + st * BM * LDR + a_r * LDR + a_c;
+      const bool ka = k0 + a_c < K;   // pairs: the pad of an odd row length is zero
+#pragma unroll
+      for (int i = 0; i < MF; ++i) {
+        const bool ok = ka && arow[i] != nullptr;
+        cp16(as + 32 * i * LDR, ok ? arow[i] + k0 : ws, ok ? 16 : 0);
+      }
+      double* bs = Bs + st * B_STAGE;
+      if constexpr (COEF) {
+#pragma unroll
+        for (int i = 0; i < BKT / 8; ++i) {
+          const int row = warp + 8 * i;
+          const double* src = wt + (int64_t)(k0 + row) * ldw + n0;
+#pragma unroll
+          for (int h = 0; h < (BN / 2 + 31) / 32; ++h) {
+            const int c = lane + 32 * h;
+            const bool ok = n0 + 2 * c < (int)ldw;
+            if (2 * c < BN) cp16(bs + row * LDB + 2 * c, ok ? src + 2 * c : ws, ok ? 16 : 0);
+          }
+        }
+      } else {
+        for (int r = a_r; r < BN; r += 32) {
+          const bool ok = ka && n0 + r < ncol;
+          cp16(bs + r * LDR + a_c, ok ? wt + (int64_t)(n0 + r) * ldw + k0 + a_c : ws, ok ? 16 : 0);
+        }
+      }
+    };
+#pragma unroll
+    for (int s = 0; s < STG - 1; ++s) {
+      if (s < ktiles) load(s, s);
+      cp_commit_t();
+    }
+    int st = 0;
+    for (int kt = 0; kt < ktiles; ++kt) {
+      cp_wait_t<STG - 2>();
+      __syncthreads();
+      if (kt + STG - 1 < ktiles) load(kt + STG - 1, st == 0 ? STG - 1 : st - 1);
+      cp_commit_t();
+      const double* as = As + st * BM * LDR + (wm * 8 + g) * LDR + t;
+      const double* bs = COEF ? Bs + st * B_STAGE + t * LDB + wn * 8 + g : Bs + st * B_STAGE + (wn * 8 + g) * LDR + t;
+      st = st + 1 == STG ? 0 : st + 1;
+#pragma unroll
+      for (int kk = 0; kk < BKT; kk += 4) {
+        double bf[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) bf[j] = COEF ? bs[kk * LDB + j * 16] : bs[j * 16 * LDR + kk];
+#pragma unroll
+        for (int i = 0; i < MF; ++i)
+          if (i < ni) {   // uniform in the warp
+            const double af = as[i * 32 * LDR + kk];
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+              if (j < nj) dmma_t(acc[i][j][0], acc[i][j][1], af, bf[j]);
+          }
+      }
+    }
+    cp_wait_t<0>();
+    __syncthreads();   // the stages are refilled for the next rows
+#pragma unroll
+    for (int i = 0; i < MF; ++i) {
+      const int m = m0 + (4 * i + wm) * 8 + g;
+      if (m >= nk) continue;
+      double* o = COEF ? part + ((size_t)tile * kmax + m) * ldw : ac + ((size_t)tile * kmax + m) * kAdjLd;
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const int n = n0 + (wn + 2 * j) * 8 + 2 * t;
+        if (n < (COEF ? (int)ldw : ncol)) *reinterpret_cast<double2*>(o + n) = make_double2(acc[i][j][0], acc[i][j][1]);
+      }
+    }
+  }
+}
+
+// grad[n][k] (+)= sum over the tiles, in order, of part[tile][inv[tile][k]][n]
+// (inv < 0: AO k is not in the tile's list).  A warp per AO and 64 MOs, with
+// the list positions of the next 32 tiles in flight beside eight rows; 16 AOs
+// x 64 MOs per CTA, transposed through shared memory.
+__global__ void __launch_bounds__(512)
+sum_tiles_kernel(const double* __restrict__ part, const int* __restrict__ inv, const int64_t ntiles, const int64_t kmax,
+                 const int64_t A, const int64_t M, const int64_t ldw, double* __restrict__ grad,
+                 const bool accumulate) {
+  __shared__ double tr[64][17];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t k = (int64_t)blockIdx.x * 16 + warp, n = (int64_t)blockIdx.y * 64 + 2 * lane;
+  double2 v = make_double2(0.0, 0.0);
+  if (k < A) {
+    int next = lane < ntiles ? inv[lane * kmax + k] : -1;
+    for (int64_t t0 = 0; t0 < ntiles; t0 += 32) {
+      const int at = next;
+      next = t0 + 32 + lane < ntiles ? inv[(t0 + 32 + lane) * kmax + k] : -1;
+      unsigned int m = __ballot_sync(0xffffffffu, at >= 0);
+      while (m) {
+        double2 x[8];
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+          x[h] = make_double2(0.0, 0.0);
+          if (m) {
+            const int b = __ffs(m) - 1;
+            m &= m - 1;
+            const int row = __shfl_sync(0xffffffffu, at, b);
+            if (n < ldw) x[h] = *reinterpret_cast<const double2*>(part + ((size_t)(t0 + b) * kmax + row) * ldw + n);
+          }
+        }
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+          v.x += x[h].x;
+          v.y += x[h].y;
+        }
+      }
+    }
+  }
+  tr[2 * lane][warp] = v.x;
+  tr[2 * lane + 1][warp] = v.y;
+  __syncthreads();
+  for (int i = threadIdx.x; i < 64 * 16; i += 512) {
+    const int64_t n2 = (int64_t)blockIdx.y * 64 + i / 16, k2 = (int64_t)blockIdx.x * 16 + i % 16;
+    if (n2 < M && k2 < A) {
+      double* o = grad + n2 * A + k2;
+      *o = accumulate ? *o + tr[i / 16][i % 16] : tr[i / 16][i % 16];
+    }
+  }
+}
+
+template <bool COEF, int MF, int STG>
+cudaError_t run_adj_gemm(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws, int64_t ldw,
+                         const double* Ct, int64_t ldc, double* part, cudaStream_t s) {
+  constexpr int BM = 32 * MF, BN = 80;
+  const size_t smem = sizeof(double) * STG * (BM * (BKT + 4) + (COEF ? BKT * (BN + 4) : BN * (BKT + 4)));
+  auto kern = adj_gemm_kernel<COEF, MF, STG>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int64_t ncol = COEF ? M : kAdjRows;
+  // a tile's list holds a quarter to a half of the AOs: a CTA takes row block
+  // after row block beyond half of them
+  const int64_t gy = (ao_num + 2 * BM - 1) / (2 * BM);
+  for (int64_t z0 = 0; z0 < ntiles; z0 += 65535) {   // grid.z limit
+    const int64_t nz = std::min<int64_t>(65535, ntiles - z0);
+    dim3 grid((unsigned)((ncol + BN - 1) / BN), (unsigned)std::min<int64_t>(65535, gy), (unsigned)nz);
+    kern<<<grid, 256, smem, s>>>(t.ac + (size_t)z0 * ao_num * kAdjLd, t.klist + z0 * ao_num, t.kcount + z0, ao_num, M,
+                                 ws + (size_t)z0 * kAdjRows * ldw, ldw, Ct, ldc,
+                                 COEF ? part + (size_t)z0 * ao_num * ldw : nullptr);
+    count_launch();
+  }
+  return cudaGetLastError();
+}
+
+// Blocks of 128 list rows when they give about a CTA per SM (lists of a
+// quarter of the AOs), else of 32: 10 tiles of a 500-AO molecule 17 and 12
+// us against 56 and 30; 32 tiles of a 3750-AO one 157 and 156 us with 128,
+// 189 and 169 with 32.
+template <bool COEF>
+cudaError_t pick_adj_gemm(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws, int64_t ldw,
+                          const double* Ct, int64_t ldc, double* part, cudaStream_t s) {
+  const int64_t ctas = ntiles * (((COEF ? M : kAdjRows) + 79) / 80) * std::max<int64_t>(1, ao_num / 512);
+  return ctas < 148 ? run_adj_gemm<COEF, 1, 5>(ntiles, ao_num, M, t, ws, ldw, Ct, ldc, part, s)
+                    : run_adj_gemm<COEF, 4, 3>(ntiles, ao_num, M, t, ws, ldw, Ct, ldc, part, s);
+}
+
 }  // namespace
 
 // VGL tiles of 32 points (one warp of points, 160 contraction rows).  Value
@@ -510,7 +754,7 @@ size_t f64_tile_bytes(int comps, int pts, int64_t ao_num) {
 
 F64Tiles f64_tiles_at(void* scratch, int64_t ntiles, int comps, int pts, int64_t ao_num) {
   const size_t ld = (size_t)comps * pts + 4;
-  F64Tiles t;
+  F64Tiles t{};
   t.pts = pts;
   t.ac = (double*)scratch;
   t.klist = (int*)(t.ac + ld * (size_t)ao_num * (size_t)ntiles);
@@ -530,10 +774,10 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1));
   if (e != cudaSuccess) return e;
   // few tiles: several CTAs share one, so that its shells are spread over SMs
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, 8 * 148 / ntiles));
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
   kern<<<dim3((unsigned)ntiles, (unsigned)parts), kAoThreads, sm, s>>>(
       P, coord, cstride, perm, tile0, T.shell_num, sh, T.coef_ac, T.ao_factor, cutoff, dp_exp, cusp_r, T.ao_num, t.ac,
-      t.klist, t.kcount);
+      t.klist, t.kcount, t.adj);
   count_launch();
   return cudaGetLastError();
 }
@@ -557,6 +801,35 @@ cudaError_t launch_tile_gemm(int64_t P, int comps, int64_t tile0, int64_t ntiles
     return go(run_tile_gemm<1, 32, 4, 1, 4, 1, 6>);
   }
   return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_weight_tiles(int64_t P, int64_t tile0, int64_t ntiles, const double* w, int64_t M, const int* perm,
+                                double* ws, int64_t ldw, cudaStream_t s) {
+  if (ntiles <= 0) return cudaSuccess;
+  const int64_t rows = ntiles * kAdjRows;
+  const unsigned grid = (unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 32);
+  weight_tiles_kernel<<<grid, 256, 0, s>>>(P, tile0, rows, w, M, perm, ws, ldw);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws, int64_t ldw,
+                            double* part, double* grad, bool accumulate, cudaStream_t s) {
+  if (ntiles <= 0 || M <= 0) return cudaSuccess;
+  if (t.pts != kAdjPts) return cudaErrorInvalidValue;
+  cudaError_t e = pick_adj_gemm<true>(ntiles, ao_num, M, t, ws, ldw, nullptr, 0, part, s);
+  if (e != cudaSuccess) return e;
+  dim3 grid((unsigned)((ao_num + 15) / 16), (unsigned)((M + 63) / 64));
+  sum_tiles_kernel<<<grid, 512, 0, s>>>(part, t.adj.inv, ntiles, ao_num, ao_num, M, ldw, grad, accumulate);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_adj_pullback(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws,
+                                int64_t ldw, const double* Ct, int64_t ldc, cudaStream_t s) {
+  if (ntiles <= 0 || M <= 0) return cudaSuccess;
+  if (t.pts != kAdjPts) return cudaErrorInvalidValue;
+  return pick_adj_gemm<false>(ntiles, ao_num, M, t, ws, ldw, Ct, ldc, nullptr, s);
 }
 
 }  // namespace qb

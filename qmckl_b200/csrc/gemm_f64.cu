@@ -1,13 +1,7 @@
-// FP64 MO contraction: C[M][N] = A[M][K] * B[K][N] (row-major).
+// Dense FP64 GEMM: C[M][N] = A[M][K] * B[K][N] (row-major), the MO Hessian's
+// contraction of AO Hessian rows with coefficient_t (org/qmckl_mo.org:2428-2600).
 //
-// For MO VGL, A is ao_vgl viewed as a (5*point_num) x ao_num matrix, B is
-// coefficient_t [ao][mo] and C is mo_vgl viewed as (5*point_num) x mo_num; for
-// MO value the same with ao_value / mo_value.  This is the dense form of
-// qmckl_compute_mo_basis_mo_vgl_hpc (org/qmckl_mo.org:2015-2163): the
-// reference skips AOs whose value is exactly zero, whose products are exact
-// zeros, so only the summation order differs.
-//
-// The FP64 form runs on the FP64 tensor pipe (mma.sync m8n8k4 f64, the only
+// It runs on the FP64 tensor pipe (mma.sync m8n8k4 f64, the only
 // FP64 MMA on sm_100a; tcgen05 has no FP64 kind).  CTA tile 128 x (8*NT*2),
 // BK = 16, 8 warps as 4 (M) x 2 (N), each warp 32 x 8*NT, operands staged in
 // shared memory by a 3-stage cp.async pipeline with zero-filled edges.
@@ -41,35 +35,19 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-// TA: A is stored transposed (element (m, k) at A[k * lda + m]); its shared
-// tile is then kept k-major ([BK][BM + 4]).  Split K (TA only): CTA z of the
-// grid covers k in [z * k_split, (z + 1) * k_split) and writes C + z * c_split.
-template <int NT, int VA, int VB, bool TA>
+template <int NT, int VA, int VB>
 __global__ void __launch_bounds__(256)
-dgemm_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A_, int64_t lda,
-             const double* __restrict__ B_, int64_t ldb, double* __restrict__ C_, int64_t ldc, int64_t k_split,
-             int64_t c_split) {
+dgemm_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A, int64_t lda,
+             const double* __restrict__ B, int64_t ldb, double* __restrict__ C, int64_t ldc) {
   constexpr int BN = 16 * NT;
   constexpr int LDB_S = BN + 4;
-  constexpr int LDT = BM + 4;                      // row stride of the k-major A tile (TA)
   extern __shared__ __align__(16) double smem[];
-  double* As = smem;                               // [STAGES][BM][LDA_S] or [STAGES][BK][LDT]
+  double* As = smem;                               // [STAGES][BM][LDA_S]
   double* Bs = smem + STAGES * BM * LDA_S;         // [STAGES][BK][LDB_S]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp & 3, wn = warp >> 2;
   const int g = lane >> 2, t = lane & 3;
   const int64_t n0 = (int64_t)blockIdx.x * BN;
-  const double* __restrict__ A = A_;
-  const double* __restrict__ B = B_;
-  double* __restrict__ C = C_;
-  if constexpr (TA) {   // split K (used with the transposed form only)
-    const int64_t kz0 = (int64_t)blockIdx.z * k_split;
-    // an empty K range (last splits of a short K) still writes its zero slice
-    K = kz0 >= K ? 0 : ((K - kz0) < k_split ? (K - kz0) : k_split);
-    A = A_ + kz0 * lda;
-    B = B_ + kz0 * ldb;
-    C = C_ + (int64_t)blockIdx.z * c_split;
-  }
   const int ktiles = (int)((K + BK - 1) / BK);
 
   for (int64_t mt = blockIdx.y; mt * BM < M; mt += gridDim.y) {
@@ -86,30 +64,16 @@ dgemm_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A_, int
       double* bs = Bs + st * BK * LDB_S;
       // A tile: BM x BK
       constexpr int ACH = BM * BK / VA;
-      if constexpr (TA) {
 #pragma unroll
-        for (int i = 0; i < ACH / 256; ++i) {
-          const int c = tid + i * 256;
-          const int kr = c / (BM / VA), mc = (c % (BM / VA)) * VA;
-          const int64_t gm = m0 + mc, gk = k0 + kr;
-          int bytes = 0;
-          if (gm < M && gk < K) bytes = (int)((M - gm) < VA ? (M - gm) : VA) * 8;
-          const double* src = bytes ? A + gk * lda + gm : A;
-          if (VA == 2) cp_async16(as + kr * LDT + mc, src, bytes);
-          else cp_async8(as + kr * LDT + mc, src, bytes);
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < ACH / 256; ++i) {
-          const int c = tid + i * 256;
-          const int row = c / (BK / VA), col = (c % (BK / VA)) * VA;
-          const int64_t gm = m0 + row, gk = k0 + col;
-          int bytes = 0;
-          if (gm < M && gk < K) bytes = (int)((K - gk) < VA ? (K - gk) : VA) * 8;
-          const double* src = bytes ? A + gm * lda + gk : A;
-          if (VA == 2) cp_async16(as + row * LDA_S + col, src, bytes);
-          else cp_async8(as + row * LDA_S + col, src, bytes);
-        }
+      for (int i = 0; i < ACH / 256; ++i) {
+        const int c = tid + i * 256;
+        const int row = c / (BK / VA), col = (c % (BK / VA)) * VA;
+        const int64_t gm = m0 + row, gk = k0 + col;
+        int bytes = 0;
+        if (gm < M && gk < K) bytes = (int)((K - gk) < VA ? (K - gk) : VA) * 8;
+        const double* src = bytes ? A + gm * lda + gk : A;
+        if (VA == 2) cp_async16(as + row * LDA_S + col, src, bytes);
+        else cp_async8(as + row * LDA_S + col, src, bytes);
       }
       // B tile: BK x BN
       constexpr int BCH = BK * BN / VB;
@@ -141,8 +105,7 @@ dgemm_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A_, int
       for (int kk = 0; kk < BK; kk += 4) {
         double af[4], bf[NT];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          af[i] = TA ? as[(kk + t) * LDT + wm * 32 + i * 8 + g] : as[(wm * 32 + i * 8 + g) * LDA_S + kk + t];
+        for (int i = 0; i < 4; ++i) af[i] = as[(wm * 32 + i * 8 + g) * LDA_S + kk + t];
 #pragma unroll
         for (int j = 0; j < NT; ++j) bf[j] = bs[(kk + t) * LDB_S + j * 8 + g];
 #pragma unroll
@@ -173,42 +136,39 @@ dgemm_kernel(int64_t M, int64_t N, int64_t K, const double* __restrict__ A_, int
   }
 }
 
-template <int NT, int VA, int VB, bool TA>
+template <int NT, int VA, int VB>
 cudaError_t run(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
-                int64_t ldb, double* C, int64_t ldc, int splits, cudaStream_t s) {
+                int64_t ldb, double* C, int64_t ldc, cudaStream_t s) {
   constexpr int BN = 16 * NT;
   const size_t smem = sizeof(double) * STAGES * (BM * LDA_S + BK * (BN + 4));
-  auto kern = dgemm_kernel<NT, VA, VB, TA>;
+  auto kern = dgemm_kernel<NT, VA, VB>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int64_t mt = (M + BM - 1) / BM;
-  const int64_t k_split = ((K + splits - 1) / splits + BK - 1) / BK * BK;
-  dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)std::min<int64_t>(mt, 65535), (unsigned)splits);
-  kern<<<grid, 256, smem, s>>>(M, N, K, A, lda, B, ldb, C, ldc, k_split, M * ldc);
+  dim3 grid((unsigned)((N + BN - 1) / BN), (unsigned)std::min<int64_t>(mt, 65535));
+  kern<<<grid, 256, smem, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
   count_launch();
   return cudaGetLastError();
 }
 
-template <int NT, bool TA>
+template <int NT>
 cudaError_t run_nt(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
-                   int64_t ldb, double* C, int64_t ldc, int splits, cudaStream_t s) {
+                   int64_t ldb, double* C, int64_t ldc, cudaStream_t s) {
   const bool va = (lda % 2 == 0) && ((uintptr_t)A % 16 == 0);
   const bool vb = (ldb % 2 == 0) && ((uintptr_t)B % 16 == 0);
-  if (va && vb) return run<NT, 2, 2, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
-  if (va) return run<NT, 2, 1, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
-  if (vb) return run<NT, 1, 2, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
-  return run<NT, 1, 1, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
+  if (va && vb) return run<NT, 2, 2>(M, N, K, A, lda, B, ldb, C, ldc, s);
+  if (va) return run<NT, 2, 1>(M, N, K, A, lda, B, ldb, C, ldc, s);
+  if (vb) return run<NT, 1, 2>(M, N, K, A, lda, B, ldb, C, ldc, s);
+  return run<NT, 1, 1>(M, N, K, A, lda, B, ldb, C, ldc, s);
 }
 
-template <bool TA>
 cudaError_t run_any(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B, int64_t ldb,
-                    double* C, int64_t ldc, int splits, cudaStream_t s) {
+                    double* C, int64_t ldc, cudaStream_t s) {
   if (M <= 0 || N <= 0) return cudaSuccess;
-  if (!TA && splits != 1) return cudaErrorInvalidValue;
   // pick the N tile (64 or 80 columns) that wastes fewer padded columns
   const int64_t w64 = ((N + 63) / 64) * 64 - N, w80 = ((N + 79) / 80) * 80 - N;
-  if (w80 < w64) return run_nt<5, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
-  return run_nt<4, TA>(M, N, K, A, lda, B, ldb, C, ldc, splits, s);
+  if (w80 < w64) return run_nt<5>(M, N, K, A, lda, B, ldb, C, ldc, s);
+  return run_nt<4>(M, N, K, A, lda, B, ldb, C, ldc, s);
 }
 
 // out[n][m] (+)= sum_z part[z][m][n], through 32 x 32 shared tiles
@@ -237,13 +197,7 @@ __global__ void add_transposed_kernel(const double* __restrict__ part, int split
 
 cudaError_t launch_gemm_f64(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda,
                             const double* B, int64_t ldb, double* C, int64_t ldc, cudaStream_t s) {
-  return run_any<false>(M, N, K, A, lda, B, ldb, C, ldc, 1, s);
-}
-
-cudaError_t launch_gemm_f64_tn_split(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
-                                     int64_t ldb, double* part, int splits, cudaStream_t s) {
-  if (splits < 1) return cudaErrorInvalidValue;
-  return run_any<true>(M, N, K, A, lda, B, ldb, part, N, splits, s);
+  return run_any(M, N, K, A, lda, B, ldb, C, ldc, s);
 }
 
 cudaError_t launch_add_transposed(const double* part, int splits, int64_t M, int64_t N, double* out, bool accumulate,

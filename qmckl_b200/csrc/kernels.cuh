@@ -130,11 +130,20 @@ struct F64Shell {
 // Compact tiles of pts = f64_tile_points points each, f64_tile_bytes per
 // tile: ac[tile][ao_num][comps * pts + 4] (the first kcount[tile] rows hold
 // the tile's live AOs klist[tile][.]).
+// For the adjoint also: inv[tile][ao_num], the list position of each AO
+// (preset to -1; may be null); live[tile][shell_num], the live shells (shell,
+// first list position), nlive[tile] of them.
+struct AdjTables {
+  int* inv;
+  int2* live;
+  int* nlive;
+};
 struct F64Tiles {
   int pts;
   double* ac;
   int* klist;
   int* kcount;
+  AdjTables adj;
 };
 int f64_tile_points(int comps, int64_t P);
 size_t f64_tile_bytes(int comps, int pts, int64_t ao_num);
@@ -150,21 +159,33 @@ cudaError_t launch_tile_gemm(int64_t P, int comps, int64_t tile0, int64_t ntiles
                              const F64Tiles& t, const int* perm, const double* Bt, int64_t ldb, double* C,
                              cudaStream_t s);
 
-// Split-K FP64 GEMM with A transposed: part[z][m][n] = sum over the z-th K
-// range of A[k][m] * B[k][n] (A element (m, k) at A[k * lda + m]), for
-// z < splits; part is [splits][M][N].
-cudaError_t launch_gemm_f64_tn_split(int64_t M, int64_t N, int64_t K, const double* A, int64_t lda, const double* B,
-                                     int64_t ldb, double* part, int splits, cudaStream_t s);
+// FP64 adjoint of the MO VGL over compact VGL tiles (f64_tiles.cu,
+// adjoint.cu) with their AdjTables.
+// Weights in tile order: ws[tile][c * 32 + p][ldw], ldw even.
+cudaError_t launch_weight_tiles(int64_t P, int64_t tile0, int64_t ntiles, const double* w, int64_t M, const int* perm,
+                                double* ws, int64_t ldw, cudaStream_t s);
+// grad[mo][ao] (+)= AO^T W of the tiles; part [ntiles][ao_num][ldw].
+cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws, int64_t ldw,
+                            double* part, double* grad, bool accumulate, cudaStream_t s);
+// t.ac <- W C, the weights pulled back to the tiles' AOs (Ct: coefficient_t
+// with ldc even, zero past the MOs).
+cudaError_t launch_adj_pullback(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws,
+                                int64_t ldw, const double* Ct, int64_t ldc, cudaStream_t s);
+// grad_nucl [nucl][3] -= and grad_coord [3][gstride] (zeroed before) +=, either
+// may be null, from the pulled-back weights in t.ac.
+cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,
+                              int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const F64Tiles& t,
+                              double* grad_nucl, double* grad_coord, int64_t gstride, cudaStream_t s);
+
 // out[n][m] = (out[n][m] +) sum_z part[z][m][n]  (fixed summation order)
 cudaError_t launch_add_transposed(const double* part, int splits, int64_t M, int64_t N, double* out, bool accumulate,
                                   cudaStream_t s);
 
 // Derivative kernels (adjoint.cu).  ao_hessian: [3][point_num][4][ao]
-// (coord [3][point_num]).  Adjoint: G [point_num][5][ao]; grad_nucl
-// [nucl][3] -= and grad_coord [3][gstride] += (may be null); coord
-// [3][cstride].  `mixed` selects FP32 exponentials where a r^2 <= 30; for
-// the adjoint it also means G in FP32 (float*, else double*) and FP32
-// per-AO derivative arithmetic.
+// (coord [3][point_num]), `mixed` selects FP32 exponentials where a r^2 <= 30.
+// Mixed-form adjoint: G [point_num][5][ao] in FP32; grad_nucl [nucl][3] -=
+// and grad_coord [3][gstride] += (may be null); coord [3][cstride]; FP32
+// exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic.
 cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const double* coord, double cutoff, bool mixed,
                               double* ao_hessian, cudaStream_t s, const double* cusp_r = nullptr);
 // Orbital forces (adjoint.cu): which = 0 forces_mo_value, 1 forces_mo_g,
@@ -174,7 +195,7 @@ cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const doubl
 cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, const int2* nuc_ao, const double* X,
                           const double* Ct, double* out, cudaStream_t s);
 cudaError_t launch_mo_adjoint_nuclear(const DevTables& T, int64_t point_num, const double* coord, int64_t cstride,
-                                      double cutoff, bool mixed, const void* G, double* grad_nucl,
-                                      double* grad_coord, int64_t gstride, cudaStream_t s);
+                                      double cutoff, const float* G, double* grad_nucl, double* grad_coord,
+                                      int64_t gstride, cudaStream_t s);
 
 }  // namespace qb

@@ -86,3 +86,46 @@ def test_nan_point_stays_alone():
     assert parity_error(got[keep], ref[keep]) < TOL
     assert (got_far[17] == 0.0).all()
     assert parity_error(got_far[keep], ref[keep]) < TOL
+
+
+@pytest.mark.parametrize("cid,P,m", [(0, 1, 3), (0, 32, 90), (0, 33, 81), (0, 100, 17), ("hl", 40, 101), (1, 50, 33)])
+def test_adjoint_tiles(cid, P, m):
+    """dL/dC, dL/dR and dL/dr over the tiles, against the oracle (the bar of test_gpu_adjoint.py)."""
+    d = _molecule(cid, m, 300 + P)
+    pts = _points(d, P, 400 + P)
+    w = np.random.default_rng(500 + P).standard_normal((P, 5, m))
+    ctx = make_context(d, points=False, form=pq.FORM_FP64)
+    t = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")  # noqa: E731
+    c, dw = t(pts.T), t(w)
+    nan = float("nan")
+    gc, gn, gr = (torch.full(s, nan, dtype=torch.float64, device="cuda")
+                  for s in ((m, d["ao_num"]), (d["nucl_num"], 3), (3, P)))
+    torch.cuda.synchronize()
+    try:
+        pq.b200_mo_vgl_adjoint_device(ctx, P, c.data_ptr(), dw.data_ptr(), gc.data_ptr(), gn.data_ptr(), gr.data_ptr())
+        pq.b200_synchronize(ctx)
+    finally:
+        pq.context_destroy(ctx)
+    ref = O.mo_vgl_adjoint(O.Basis(d), pts, d["nucl_coord"], d["mo_coef"], w)
+    for got, want in zip((gc, gn, gr.T), ref):
+        assert np.abs(got.cpu().numpy() - want).max() <= 1e-10 * np.abs(want).max()
+
+
+def test_adjoint_coefficients_repeat():
+    """dL/dC is summed in a fixed order: the same bits in every run."""
+    d = _molecule(0, 90, 8)
+    pts = _points(d, 5000, 9)
+    w = torch.randn((5000, 5, 90), dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    c = torch.tensor(np.ascontiguousarray(pts.T), dtype=torch.float64, device="cuda")
+    ctx = make_context(d, points=False, form=pq.FORM_FP64)
+    out = []
+    torch.cuda.synchronize()
+    try:
+        for _ in range(3):
+            g = torch.empty((90, d["ao_num"]), dtype=torch.float64, device="cuda")
+            pq.b200_mo_vgl_adjoint_device(ctx, 5000, c.data_ptr(), w.data_ptr(), g.data_ptr(), 0, 0)
+            pq.b200_synchronize(ctx)
+            out.append(g)
+    finally:
+        pq.context_destroy(ctx)
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
