@@ -1,5 +1,5 @@
-// Derivative kernels of the AO VGL: the AO Hessian getter and the adjoint of
-// MO VGL with respect to the nuclear and point coordinates.
+// Derivative kernels of the AO VGL: the AO Hessian getter, the adjoint of MO
+// VGL with respect to the nuclear and point coordinates, the orbital forces.
 //
 // Quantities (derivatives with respect to the point coordinates r; an AO
 // centred on nucleus A depends on r - R_A, so d/dR_A = -d/dr):
@@ -18,18 +18,11 @@
 // r^2 > cutoff * range, primitives sorted by exponent with a break at
 // a r^2 > cutoff, AO skipped when its contracted radial value is zero.
 //
-// Work decomposition: one warp per (point, nucleus block), as in the forward
-// AO kernel: lanes stage the block's displacements and radial derivative sets
-// in shared memory, then sweep the block's contiguous AO range.
-//   MODE_HESSIAN  writes ao_hessian[3][point][4][ao] (coalesced rows).
-//   MODE_ADJOINT  (mixed form) reads G[point][5][ao] = (W . C)[point][comp][ao], the loss
-//                 weights pulled back through the MO coefficients, and forms
-//                 q_d = G0 d_d chi + sum_e G_{1+e} H_ed + G4 T_d per AO.  A
-//                 segmented warp reduction over the (contiguous) AOs of each
-//                 nucleus feeds per-CTA shared accumulators of dL/dR (one
-//                 device atomic per nucleus and CTA at the end); the sum over
-//                 all AOs gives dL/dr of the point.
-// The FP64 adjoint works on compact tiles instead (tile_deriv_kernel).
+// The AO Hessian takes one warp per (point, nucleus block), as the forward AO
+// kernel; the adjoint works on compact tiles (tile_deriv_kernel): with the
+// loss weights pulled back through the MO coefficients, G = W . C, it forms
+// q_d = G0 d_d chi + sum_e G_{1+e} H_ed + G4 T_d per AO; -q summed over a
+// nucleus's AOs and the points is dL/dR, q summed over all AOs dL/dr.
 #include <algorithm>
 #include <type_traits>
 
@@ -40,7 +33,6 @@ namespace {
 
 constexpr int kWarpsD = 8;
 constexpr double kShiftD = 1.e-20;
-constexpr int MODE_HESSIAN = 0, MODE_ADJOINT = 1;
 
 struct DerivSmem {
   double rad[kBlockSlots][4];   // R, R1, R2, R3 of the block's shells
@@ -162,158 +154,49 @@ __device__ __forceinline__ void ao_derivs(int code, F f, const F (&v)[3], const 
   }
 }
 
-// MODE_HESSIAN: out = ao_hessian[3][point_num][4][ao] (point_num points from
-//   coord [3][cstride], cstride >= point_num).
-// MODE_ADJOINT: G = [point_num][5][ao]; grad_nucl [nucl][3] -= sum q (per-CTA
-//   shared accumulators when use_smem, else device atomics); grad_coord
-//   ([3][gstride], may be null) += sum q.
-// MIXED: FP32 exponentials where a r^2 <= 30; in MODE_ADJOINT also G in FP32
-//   and the per-AO derivative arithmetic in FP32 (displacements, r^2, radial
-//   sums and the cancelling radial combinations in FP64; q summed in FP64).
-template <int MODE, bool MIXED>
+// AO Hessian: out = ao_hessian[3][point_num][4][ao].  MIXED: FP32
+// exponentials where a r^2 <= 30.
+template <bool MIXED>
 __global__ void __launch_bounds__(kWarpsD * 32)
-deriv_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord, const int64_t cstride,
-             const double cutoff, double* __restrict__ out, const void* __restrict__ Gv,
-             double* __restrict__ grad_nucl, double* __restrict__ grad_coord, const int64_t gstride,
-             const bool use_smem, const double* __restrict__ cusp_r) {
-  using F = typename std::conditional<MIXED && MODE == MODE_ADJOINT, float, double>::type;
-  const F* __restrict__ G = (const F*)Gv;
+hessian_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord, const double cutoff,
+               double* __restrict__ out, const double* __restrict__ cusp_r) {
   __shared__ DerivSmem smem[kWarpsD];
-  extern __shared__ double sacc[];   // [nucl][3] (MODE_ADJOINT with use_smem)
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   DerivSmem& sm = smem[warp];
   const int64_t A = T.ao_num;
-  if (MODE == MODE_ADJOINT && use_smem) {
-    for (int i = threadIdx.x; i < 3 * T.nucl_num; i += blockDim.x) sacc[i] = 0.0;
-    __syncthreads();
-  }
   const int64_t stride = (int64_t)gridDim.x * kWarpsD;
   // one warp per point, through its nucleus blocks (as the FP64 AO kernel)
   for (int64_t p = (int64_t)blockIdx.x * kWarpsD + warp; p < point_num; p += stride) {
-   double pg[3] = {0., 0., 0.};
-   for (int b = 0; b < T.nblock; ++b) {
-    const int4 blk = T.block[b];
-    const int2 slots = T.block_slots[b];
-    stage_deriv<MIXED>(T, sm, blk, slots, coord[p], coord[p + cstride], coord[p + 2 * cstride], cutoff, lane);
-    for (int k0 = blk.z; k0 < blk.w; k0 += 32) {
-      const int k = k0 + lane;
-      const bool valid = k < blk.w;
-      int nl = kBlockNuc;   // past-the-end lanes form their own (last) segment
-      F g[3] = {F(0), F(0), F(0)}, H[3][3] = {{F(0), F(0), F(0)}, {F(0), F(0), F(0)}, {F(0), F(0), F(0)}},
-        Tl[3] = {F(0), F(0), F(0)};
-      if (valid) {
+    for (int b = 0; b < T.nblock; ++b) {
+      const int4 blk = T.block[b];
+      const int2 slots = T.block_slots[b];
+      stage_deriv<MIXED>(T, sm, blk, slots, coord[p], coord[p + point_num], coord[p + 2 * point_num], cutoff, lane);
+      for (int k = blk.z + lane; k < blk.w; k += 32) {
         const int code = T.ao_code[k];
-        const int slot = (code >> 16) & 255;
-        nl = (code >> 24) & 31;
+        const int slot = (code >> 16) & 255, nl = (code >> 24) & 31;
         const double r2 = sm.nuc[nl][3];
         const double* Rs = sm.rad[slot];
+        double g[3], H[3][3] = {{0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}}, Tl[3] = {0., 0., 0.};
         if (r2 >= 0.0 && Rs[0] != 0.0 && !cusp_masked(cusp_r, (code >> 12) & 15, blk.x + nl, r2, false)) {
           const double lapR = 4.0 * r2 * Rs[2] + 6.0 * Rs[1];
           const double k3 = 20.0 * Rs[2] + 8.0 * r2 * Rs[3];
-          const F v[3] = {(F)sm.nuc[nl][0], (F)sm.nuc[nl][1], (F)sm.nuc[nl][2]};
-          const F R[3] = {(F)Rs[0], (F)Rs[1], (F)Rs[2]};
-          ao_derivs<F>(code, (F)T.ao_factor[k], v, R, (F)lapR, (F)k3, g, H, Tl);
+          const double v[3] = {sm.nuc[nl][0], sm.nuc[nl][1], sm.nuc[nl][2]};
+          const double R[3] = {Rs[0], Rs[1], Rs[2]};
+          ao_derivs<double>(code, T.ao_factor[k], v, R, lapR, k3, g, H, Tl);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          double* o = out + ((int64_t)i * point_num + p) * 4 * A;
+          o[k] = H[i][0];
+          o[A + k] = H[i][1];
+          o[2 * A + k] = H[i][2];
+          o[3 * A + k] = Tl[i];
         }
       }
-      if (MODE == MODE_HESSIAN) {
-        if (valid) {
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            double* o = out + ((int64_t)i * point_num + p) * 4 * A;
-            o[k] = H[i][0];
-            o[A + k] = H[i][1];
-            o[2 * A + k] = H[i][2];
-            o[3 * A + k] = Tl[i];
-          }
-        }
-      } else {
-        double q[3] = {0., 0., 0.};
-        if (valid) {
-          const F* gr = G + p * 5 * A + k;
-          const F G0 = gr[0], G1 = gr[A], G2 = gr[2 * A], G3 = gr[3 * A], G4 = gr[4 * A];
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            q[d] = (double)(G0 * g[d] + G1 * H[0][d] + G2 * H[1][d] + G3 * H[2][d] + G4 * Tl[d]);
-        }
-#pragma unroll
-        for (int d = 0; d < 3; ++d) pg[d] += q[d];
-        // segmented sum over lanes of the same nucleus (AOs of a nucleus are
-        // contiguous, so segments are runs of lanes): the first lane of each
-        // run ends up with the run's sum
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-          const int ko = __shfl_down_sync(0xffffffffu, nl, off);
-          double o[3];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) o[d] = __shfl_down_sync(0xffffffffu, q[d], off);
-          if (lane + off < 32 && ko == nl) {
-#pragma unroll
-            for (int d = 0; d < 3; ++d) q[d] += o[d];
-          }
-        }
-        const int kprev = __shfl_up_sync(0xffffffffu, nl, 1);
-        if ((lane == 0 || kprev != nl) && nl < kBlockNuc) {
-          const int n = blk.x + nl;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            if (use_smem) atomicAdd(&sacc[n * 3 + d], q[d]);
-            else if (grad_nucl != nullptr) atomicAdd(&grad_nucl[n * 3 + d], -q[d]);
-          }
-        }
-      }
+      __syncwarp();
     }
-    __syncwarp();
-   }
-    if (MODE == MODE_ADJOINT && grad_coord != nullptr) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        double s = pg[d];
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        pg[d] = s;
-      }
-      if (lane == 0) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) atomicAdd(&grad_coord[p + d * gstride], pg[d]);
-      }
-    }
-    __syncwarp();
   }
-  if (MODE == MODE_ADJOINT && use_smem && grad_nucl != nullptr) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < 3 * T.nucl_num; i += blockDim.x)
-      if (sacc[i] != 0.0) atomicAdd(&grad_nucl[i], -sacc[i]);
-  }
-}
-
-template <int MODE>
-cudaError_t launch_deriv(const DevTables& T, int64_t point_num, const double* coord, int64_t cstride, double cutoff,
-                         bool mixed, double* out, const void* G, double* grad_nucl, double* grad_coord,
-                         int64_t gstride, cudaStream_t s, const double* cusp_r = nullptr) {
-  if (point_num <= 0) return cudaSuccess;
-  const int grid = (int)std::min<int64_t>((point_num + kWarpsD - 1) / kWarpsD, 148 * 8);   // warps = points
-  size_t dyn = 0;
-  bool use_smem = false;
-  if (MODE == MODE_ADJOINT) {
-    dyn = sizeof(double) * 3 * (size_t)T.nucl_num;
-    use_smem = dyn <= 64 * 1024;
-    if (!use_smem) dyn = 0;
-  }
-  cudaError_t e = cudaSuccess;
-  if (mixed || MODE == MODE_ADJOINT) {   // the FP64 adjoint: tile_deriv_kernel
-    auto k = deriv_kernel<MODE, true>;
-    if (dyn > 48 * 1024) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-    if (e != cudaSuccess) return e;
-    k<<<grid, kWarpsD * 32, dyn, s>>>(T, point_num, coord, cstride, cutoff, out, G, grad_nucl, grad_coord, gstride,
-                                      use_smem, cusp_r);
-  } else if constexpr (MODE == MODE_HESSIAN) {
-    auto k = deriv_kernel<MODE, false>;
-    k<<<grid, kWarpsD * 32, dyn, s>>>(T, point_num, coord, cstride, cutoff, out, G, grad_nucl, grad_coord, gstride,
-                                      use_smem, cusp_r);
-  }
-  count_launch();
-  return cudaGetLastError();
 }
 
 // One AO of the FP64 adjoint, exponents known at compile time: with the
@@ -391,21 +274,29 @@ __device__ __forceinline__ void adj_shell(const ShellRad& S, const double (&xp)[
   }
 }
 
-// FP64 adjoint over compact tiles: a CTA per tile (gridDim.y of them when
+// The adjoint over compact tiles: a CTA per tile (gridDim.y of them when
 // there are few tiles), lanes are points, the warps take contiguous runs of
 // the tile's live shells.  The pulled-back weights G of the tile are read
 // along the points; q of a point is kept in the lane over the warp's shells
 // and summed over the warps in order (grad_coord is stored by a CTA that owns
 // its points, added to by one that shares them), q of a nucleus is summed
-// over the run of its shells and the lanes and added by one atomic.  0.14 ms on 20,352
+// over the run of its shells and the lanes and added by one atomic.  0.13 ms on 20,352
 // points of the 2000-AO molecule, bound by the latency of its FP64 chains (a
 // warp per point over all AOs, with the AO derivatives formed first, 1.43 ms).
-__global__ void __launch_bounds__(256)
+// gc: G[tile][m][LD], FP64 with LD = 164.  MIXED: G in FP32 with LD = 160, FP32
+// exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic
+// (displacements, r^2, radial sums and the cancelling radial combinations in
+// FP64; q summed in FP64); 0.18 ms, against 0.93 with a warp per point over all
+// AOs.  Two or three CTAs per tile below 900 tiles: 0.24 and 0.14 ms with one.
+template <bool MIXED>
+__global__ void __launch_bounds__(256, MIXED ? 3 : 2)
 tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__ coord, const int64_t cstride,
                   const int* __restrict__ perm, const int64_t tile0, const F64Shell* __restrict__ sh,
-                  const double cutoff, const double* __restrict__ gc, const AdjTables adj, const int64_t kmax,
+                  const double cutoff, const void* __restrict__ gcv, const AdjTables adj, const int64_t kmax,
                   double* __restrict__ grad_nucl, double* __restrict__ grad_coord, const int64_t gstride) {
-  constexpr int TP = 32, LD = 5 * TP + 4, NW = 8;
+  using F = typename std::conditional<MIXED, float, double>::type;
+  constexpr int TP = 32, LD = 5 * TP + (MIXED ? 0 : 4), NW = 8;
+  const F* __restrict__ gc = (const F*)gcv;
   __shared__ double sq[NW][3][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t tile = blockIdx.x;
@@ -416,7 +307,7 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
   const int n = adj.nlive[tile];
   const int part = (int)blockIdx.y * NW + warp, parts = (int)gridDim.y * NW;
   const int e0 = (int)((int64_t)n * part / parts), e1 = (int)((int64_t)n * (part + 1) / parts);
-  const double* gt = gc + (size_t)tile * kmax * LD + lane;
+  const F* gt = gc + (size_t)tile * kmax * LD + lane;
   double pq[3] = {0., 0., 0.}, nq[3] = {0., 0., 0.};
   int nucl = -1;
   auto flush = [&]() {
@@ -449,7 +340,8 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
         const double2 ac = T.coef_ac[j];
         const double ar2 = ac.x * r2;
         if (ar2 > cutoff) break;   // primitives sorted by exponent
-        const double ce = ac.y * exp(-ar2);
+        const double e = MIXED && ar2 <= 30.0 ? (double)expf(-(float)ar2) : exp(-ar2);
+        const double ce = ac.y * e;
         a0 += ce;
         a1 -= ac.x * ce;
         a2 += ac.x * ac.x * ce;
@@ -464,28 +356,34 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
     R.k3 = 20.0 * a2 + 8.0 * r2 * a3;
 #pragma unroll
     for (int d = 0; d < 3; ++d) R.Rd[d] = 2.0 * R.v[d] * a1;
-    const double* gr = gt + (size_t)le.y * LD;
+    const F* gr = gt + (size_t)le.y * LD;
     const double* fac = T.ao_factor + S.a0;
     double q[3] = {0., 0., 0.};
-    if (S.l <= 3) {
-      const double x = R.v[0], y = R.v[1], z = R.v[2];
-      const double xp[4] = {1.0, x, x * x, x * (x * x)}, yp[4] = {1.0, y, y * y, y * (y * y)},
-                   zp[4] = {1.0, z, z * z, z * (z * z)};
-      switch (S.l) {
-        case 0: adj_shell<0, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
-        case 1: adj_shell<1, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
-        case 2: adj_shell<2, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
-        default: adj_shell<3, 0>(R, xp, yp, zp, gr, LD, TP, fac, q);
+    bool any_l = true;
+    if constexpr (!MIXED) {
+      if (S.l <= 3) {
+        const double x = R.v[0], y = R.v[1], z = R.v[2];
+        const double xp[4] = {1.0, x, x * x, x * (x * x)}, yp[4] = {1.0, y, y * y, y * (y * y)},
+                     zp[4] = {1.0, z, z * z, z * (z * z)};
+        switch (S.l) {
+          case 0: adj_shell<0, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
+          case 1: adj_shell<1, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
+          case 2: adj_shell<2, 0>(R, xp, yp, zp, gr, LD, TP, fac, q); break;
+          default: adj_shell<3, 0>(R, xp, yp, zp, gr, LD, TP, fac, q);
+        }
+        any_l = false;
       }
-    } else {
-      const double R3[3] = {a0, a1, a2};
+    }
+    if (any_l) {
+      const F v[3] = {(F)R.v[0], (F)R.v[1], (F)R.v[2]}, R3[3] = {(F)a0, (F)a1, (F)a2};
       for (int i = 0; i < S.na; ++i) {
-        double g[3], H[3][3], Tl[3];
-        ao_derivs<double>(T.ao_code[S.a0 + i], fac[i], R.v, R3, R.lapR, R.k3, g, H, Tl);
-        const double* p = gr + i * LD;
+        F g[3], H[3][3], Tl[3];
+        ao_derivs<F>(T.ao_code[S.a0 + i], (F)fac[i], v, R3, (F)R.lapR, (F)R.k3, g, H, Tl);
+        const F* p = gr + i * LD;
+        const F G0 = p[0], G1 = p[TP], G2 = p[2 * TP], G3 = p[3 * TP], G4 = p[4 * TP];
 #pragma unroll
         for (int d = 0; d < 3; ++d)
-          q[d] += p[0] * g[d] + p[TP] * H[0][d] + p[2 * TP] * H[1][d] + p[3 * TP] * H[2][d] + p[4 * TP] * Tl[d];
+          q[d] += (double)(G0 * g[d] + G1 * H[0][d] + G2 * H[1][d] + G3 * H[2][d] + G4 * Tl[d]);
       }
     }
 #pragma unroll
@@ -584,25 +482,23 @@ cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, con
 
 cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const double* coord, double cutoff, bool mixed,
                               double* ao_hessian, cudaStream_t s, const double* cusp_r) {
-  return launch_deriv<MODE_HESSIAN>(T, point_num, coord, point_num, cutoff, mixed, ao_hessian, nullptr, nullptr,
-                                    nullptr, 0, s, cusp_r);
-}
-
-cudaError_t launch_mo_adjoint_nuclear(const DevTables& T, int64_t point_num, const double* coord, int64_t cstride,
-                                      double cutoff, const float* G, double* grad_nucl, double* grad_coord,
-                                      int64_t gstride, cudaStream_t s) {
-  return launch_deriv<MODE_ADJOINT>(T, point_num, coord, cstride, cutoff, true, nullptr, G, grad_nucl, grad_coord,
-                                    gstride, s);
+  if (point_num <= 0) return cudaSuccess;
+  const int grid = (int)std::min<int64_t>((point_num + kWarpsD - 1) / kWarpsD, 148 * 8);   // warps = points
+  auto k = mixed ? hessian_kernel<true> : hessian_kernel<false>;
+  k<<<grid, kWarpsD * 32, 0, s>>>(T, point_num, coord, cutoff, ao_hessian, cusp_r);
+  count_launch();
+  return cudaGetLastError();
 }
 
 cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,
-                              int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const F64Tiles& t,
-                              double* grad_nucl, double* grad_coord, int64_t gstride, cudaStream_t s) {
+                              int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const AdjTables& adj,
+                              const void* g, bool mixed, double* grad_nucl, double* grad_coord, int64_t gstride,
+                              cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
-  if (t.pts != 32) return cudaErrorInvalidValue;
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, 2 * 148 / ntiles));
-  tile_deriv_kernel<<<dim3((unsigned)ntiles, (unsigned)parts), 256, 0, s>>>(
-      T, P, coord, cstride, perm, tile0, sh, cutoff, t.ac, t.adj, T.ao_num, grad_nucl, grad_coord, gstride);
+  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, (6 * 148 + ntiles - 1) / ntiles));
+  auto k = mixed ? tile_deriv_kernel<true> : tile_deriv_kernel<false>;
+  k<<<dim3((unsigned)ntiles, (unsigned)parts), 256, 0, s>>>(T, P, coord, cstride, perm, tile0, sh, cutoff, g, adj, T.ao_num,
+                                                            grad_nucl, grad_coord, gstride);
   count_launch();
   return cudaGetLastError();
 }

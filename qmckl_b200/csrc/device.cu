@@ -352,10 +352,10 @@ struct DeviceState {
   // derivatives: AO Hessian and the MO VGL adjoint (FP64 coefficient [mo][ao],
   // per-chunk coordinates, AO / pulled-back weight buffer, split-K partials)
   DevBuf ao_hessian;
-  DevBuf adj_coord, adj_buf, adj_part, adj_nucl;
+  DevBuf adj_coord, adj_buf, adj_part;
   // mixed-form adjoint: bfloat16 pieces of the weights and of coefficient_t
   uint64_t adj_ct_version = ~0ull;
-  DevBuf adj_wp, adj_ct;
+  DevBuf adj_wp, adj_wt, adj_ct;
   // cusp adjustment: radii [nucl] followed by the cubics' parameters
   // [nucl][4][mo]; AO arrays with the left-out AOs zeroed, which feed only the
   // MO step; point-nucleus distances; MO Hessian
@@ -1125,8 +1125,8 @@ void dev_detach(Context* ctx) {
   if (ds->stream) cudaStreamSynchronize(ds->stream);
   for (DevBuf* b : {&ds->tables, &ds->nucl, &ds->coord, &ds->prim_vgl, &ds->shell_vgl, &ds->ao_vgl, &ds->ao_value,
                     &ds->mo_vgl, &ds->mo_value, &ds->coef_t, &ds->tc_coef, &ds->tc_a, &ds->krec, &ds->order,
-                    &ds->ao_hessian, &ds->adj_coord, &ds->adj_buf, &ds->adj_part, &ds->adj_nucl,
-                    &ds->tc3_coef, &ds->env, &ds->nuc_ao, &ds->forces, &ds->adj_wp, &ds->adj_ct,
+                    &ds->ao_hessian, &ds->adj_coord, &ds->adj_buf, &ds->adj_part,
+                    &ds->tc3_coef, &ds->env, &ds->nuc_ao, &ds->forces, &ds->adj_wp, &ds->adj_wt, &ds->adj_ct,
                     &ds->cusp, &ds->ao_masked, &ds->en_dist, &ds->mo_hessian, &ds->kskip, &ds->kstat,
                     &ds->tc_err, &ds->f64_sph, &ds->coef_f, &ds->f64_tiles})
     release(*b);
@@ -1724,24 +1724,26 @@ namespace {
 // entry with 2048 rows, 7.0e-7 with 4096 and 1.7e-6 with 16384.
 constexpr int kAdjointSliceRows = 2048;
 
-// Mixed-form adjoint: the two contractions on the tensor cores.  Per chunk
-// of points: the weights W[(p,c)][mo] as 3 bfloat16 pieces; the AOs in FP64
-// arithmetic (FP32 exponentials where a r^2 <= 30, as in the derivative
-// kernel) stored as 3 bfloat16 pieces of rows p*5 + c; dC += AO^T W by the
-// split-K TN kernel, the partials summed in a fixed order into the [mo][ao]
-// layout; G = W C^T (FP32) from the pieces of coefficient_t; then the
-// derivative kernel in its mixed form.  Synchronizes once at the end to read
-// the kernels' error word.
+// Mixed-form adjoint: the two contractions on the tensor cores.  Per chunk of
+// points: the weights W[(p,c)][mo] as 3 bfloat16 pieces, in the points' order
+// and in the order of spatial tiles of 32 points; the AOs in FP64 arithmetic
+// (FP32 exponentials where a r^2 <= 30, as in the derivative kernel) stored as
+// 3 bfloat16 pieces of rows p*5 + c; dC += AO^T W by the split-K TN kernel, the
+// partials summed in a fixed order into the [mo][ao] layout; the tiles' lists
+// of AOs that reach them (f64_tiles.cu), the weights pulled back to those AOs
+// only, G = W C^T (FP32) from the pieces of coefficient_t, and the derivative
+// kernel in its mixed form over them.
 qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P, const double* d_coord,
                               const double* d_weight, double* d_grad_coef, double* d_grad_nucl, double* d_grad_coord) {
   const char* fname = "qmckl_b200_mo_vgl_adjoint_device";
   Context* ctx = ctx_of(context);
-  const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num, N = ctx->nucleus.num;
+  const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num, S = ctx->ao_basis.shell_num;
   const double cutoff = cutoff_of(ctx);
   cudaStream_t s = ds->stream;
   const int64_t ldw = (M + 7) / 8 * 8, lda = (A + 7) / 8 * 8;
   const int kps = kAdjointSliceRows / 32;
   qmckl_exit_code rc = sync_coef(context, ds);
+  if (rc == QMCKL_SUCCESS) rc = sync_f64_shells(context, ds);
   if (rc != QMCKL_SUCCESS) return rc;
   if (ds->adj_ct_version != ctx->mo_basis.coef_version || !ds->adj_ct.p) {
     rc = ensure(context, ds->adj_ct, sizeof(uint16_t) * 3 * A * ldw, fname);
@@ -1749,34 +1751,56 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
     QB_CUDA(tc_split_rows((const double*)ds->coef_t.p, A, (int)M, M, ds->adj_ct.p, (int)ldw, A * ldw, s), fname);
     ds->adj_ct_version = ctx->mo_basis.coef_version;
   }
+  const bool points = d_grad_nucl || d_grad_coord;
   const int64_t budget = (int64_t)2 << 30;
   const int64_t row_bytes = std::max<int64_t>(20 * A, 30 * lda);   // G (FP32) or the AO pieces, per point
   const int64_t max_chunk = std::min<int64_t>(P, std::max<int64_t>(64, budget / row_bytes));
   const int64_t nchunks = (P + max_chunk - 1) / max_chunk;
   const int64_t chunk = (P + nchunks - 1) / nchunks;   // equal chunks keep every launch full
   const int splits = tc_tn_splits(5 * chunk, kps);
+  const int64_t ctiles = (chunk + 31) / 32;
+  const size_t buf_bytes = std::max<size_t>((size_t)(30 * lda) * (size_t)chunk, sizeof(float) * 160 * (size_t)A * (size_t)ctiles);
+  const size_t b_live = (sizeof(int2) * (size_t)S * (size_t)ctiles + 15) / 16 * 16;
   rc = ensure(context, ds->adj_coord, sizeof(double) * 3 * chunk, fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_buf, (size_t)row_bytes * chunk, fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_wp, sizeof(uint16_t) * 3 * 5 * chunk * ldw, fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_buf, buf_bytes, fname);
+  if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_wp, sizeof(uint16_t) * 3 * 5 * chunk * ldw, fname);
+  if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->adj_wt, sizeof(uint16_t) * 3 * 160 * ctiles * ldw, fname);
+  if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->order, order_bytes(chunk), fname);
+  if (rc == QMCKL_SUCCESS && points)
+    rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 2), fname);
   if (rc == QMCKL_SUCCESS && ds->tc_err.p == nullptr) {
     rc = ensure(context, ds->tc_err, sizeof(int), fname);
     if (rc == QMCKL_SUCCESS) QB_CUDA(cudaMemsetAsync(ds->tc_err.p, 0, sizeof(int), s), fname);
   }
   if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_part, sizeof(double) * splits * A * M, fname);
-  if (rc == QMCKL_SUCCESS && !d_grad_nucl) rc = ensure(context, ds->adj_nucl, sizeof(double) * 3 * N, fname);
   if (rc != QMCKL_SUCCESS) return rc;
-  double* gnucl = d_grad_nucl ? d_grad_nucl : (double*)ds->adj_nucl.p;
   void* buf = ds->adj_buf.p;
   double* cc = (double*)ds->adj_coord.p;
+  F64Tiles t{};
+  t.pts = 32;
+  t.adj.live = (int2*)ds->f64_tiles.p;
+  t.klist = (int*)((uint8_t*)ds->f64_tiles.p + b_live);
+  t.kcount = t.klist + ctiles * A;
+  t.adj.nlive = t.kcount + ctiles;
+  const F64Shell* sh = (const F64Shell*)ds->f64_sph.p;
+  double lo[3], hi[3];
+  nucleus_box(ctx, lo, hi);
   // a bounded wait that gives up is left in the context's error word for its
   // next synchronization point (qmckl_b200_synchronize, a host getter)
   int* err = (int*)ds->tc_err.p;
   for (int64_t p0 = 0; p0 < P; p0 += chunk) {
-    const int64_t n = std::min<int64_t>(chunk, P - p0), rows = 5 * n;
+    const int64_t n = std::min<int64_t>(chunk, P - p0), rows = 5 * n, tiles = (n + 31) / 32;
     const double* w = d_weight + p0 * 5 * M;
     QB_CUDA(cudaMemcpy2DAsync(cc, sizeof(double) * n, d_coord + p0, sizeof(double) * P, sizeof(double) * n, 3,
                               cudaMemcpyDeviceToDevice, s), fname);
-    QB_CUDA(tc_split_rows(w, rows, (int)M, M, ds->adj_wp.p, (int)ldw, rows * ldw, s), fname);
+    int* perm = nullptr;
+    if (points && tiles > 1) {
+      perm = (int*)ds->order.p;
+      QB_CUDA(point_order(cc, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(n), perm, s, n), fname);
+    }
+    QB_CUDA(tc_split_weights(w, n, (int)M, perm, (int)ldw, d_grad_coef ? ds->adj_wp.p : nullptr,
+                             points ? ds->adj_wt.p : nullptr, s),
+            fname);
     if (d_grad_coef) {
       QB_CUDA(launch_ao_vgl_pieces(ds->T, n, cc, cutoff, false, buf, lda, rows * lda, s), fname);
       QB_CUDA(tc_gemm_tn_split(buf, lda, rows * lda, A, ds->adj_wp.p, ldw, rows * ldw, (int)M, rows, kps,
@@ -1786,12 +1810,12 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
                                     s),
               fname);
     }
-    if (d_grad_nucl || d_grad_coord) {
-      QB_CUDA(tc_gemm_nt(ds->adj_wp.p, ldw, rows * ldw, rows, M, ds->adj_ct.p, ldw, A * ldw, A, (float*)buf, A, err,
-                         s),
+    if (points) {
+      QB_CUDA(launch_ao_tiles(ds->T, n, 5, cc, n, perm, 0, tiles, sh, cutoff, false, nullptr, t, s), fname);
+      QB_CUDA(tc_pullback(ds->adj_wt.p, (int)ldw, tiles, (int)M, ds->adj_ct.p, A, t.klist, t.kcount, (float*)buf, err, s),
               fname);
-      QB_CUDA(launch_mo_adjoint_nuclear(ds->T, n, cc, n, cutoff, (const float*)buf, gnucl,
-                                        d_grad_coord ? d_grad_coord + p0 : nullptr, P, s),
+      QB_CUDA(launch_tile_deriv(ds->T, n, cc, n, perm, 0, tiles, sh, cutoff, t.adj, buf, true, d_grad_nucl,
+                                d_grad_coord ? d_grad_coord + p0 : nullptr, P, s),
               fname);
     }
   }
@@ -1860,7 +1884,9 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
     if (d_grad_coef) QB_CUDA(launch_adj_coef(n, A, M, t, ws, ldw, part, d_grad_coef, t0 > 0, s), fname);
     if (d_grad_nucl || d_grad_coord) {
       QB_CUDA(launch_adj_pullback(n, A, M, t, ws, ldw, Ct, ldc, s), fname);
-      QB_CUDA(launch_tile_deriv(ds->T, P, d_coord, P, perm, t0, n, sh, cutoff, t, d_grad_nucl, d_grad_coord, P, s), fname);
+      QB_CUDA(launch_tile_deriv(ds->T, P, d_coord, P, perm, t0, n, sh, cutoff, t.adj, t.ac, false, d_grad_nucl,
+                                d_grad_coord, P, s),
+              fname);
     }
   }
   return QMCKL_SUCCESS;

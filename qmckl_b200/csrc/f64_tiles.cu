@@ -300,6 +300,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
       if (adj.live != nullptr) adj.nlive[tile] = nlive;
     }
   }
+  if (ac == nullptr) return;   // the lists only
   double* __restrict__ act = ac + (size_t)tile * kmax * LD;
   const int units = nlive * G;
   for (;;) {
@@ -774,7 +775,7 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1));
   if (e != cudaSuccess) return e;
   // few tiles: several CTAs share one, so that its shells are spread over SMs
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
+  const int parts = t.ac == nullptr ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
   kern<<<dim3((unsigned)ntiles, (unsigned)parts), kAoThreads, sm, s>>>(
       P, coord, cstride, perm, tile0, T.shell_num, sh, T.coef_ac, T.ao_factor, cutoff, dp_exp, cusp_r, T.ao_num, t.ac,
       t.klist, t.kcount, t.adj);

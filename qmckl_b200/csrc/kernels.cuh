@@ -148,7 +148,8 @@ struct F64Tiles {
 int f64_tile_points(int comps, int64_t P);
 size_t f64_tile_bytes(int comps, int pts, int64_t ao_num);
 F64Tiles f64_tiles_at(void* scratch, int64_t ntiles, int comps, int pts, int64_t ao_num);
-// The AO tiles [tile0, tile0 + ntiles) of the points in the order perm
+// The AO tiles (or, with t.ac null, only their lists) [tile0, tile0 + ntiles) of
+// the points in the order perm
 // (null: as they are), coord [3][cstride]; cusp_r as in launch_ao_vgl_f64.
 cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const double* coord, int64_t cstride,
                             const int* perm, int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff,
@@ -172,10 +173,13 @@ cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64
 cudaError_t launch_adj_pullback(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws,
                                 int64_t ldw, const double* Ct, int64_t ldc, cudaStream_t s);
 // grad_nucl [nucl][3] -= and grad_coord [3][gstride] (zeroed before) +=, either
-// may be null, from the pulled-back weights in t.ac.
+// may be null, from the pulled-back weights g of the tiles: FP64
+// [tile][ao_num][164], or (mixed) FP32 [tile][ao_num][160] with FP32
+// exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic.
 cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,
-                              int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const F64Tiles& t,
-                              double* grad_nucl, double* grad_coord, int64_t gstride, cudaStream_t s);
+                              int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const AdjTables& adj,
+                              const void* g, bool mixed, double* grad_nucl, double* grad_coord, int64_t gstride,
+                              cudaStream_t s);
 
 // out[n][m] = (out[n][m] +) sum_z part[z][m][n]  (fixed summation order)
 cudaError_t launch_add_transposed(const double* part, int splits, int64_t M, int64_t N, double* out, bool accumulate,
@@ -183,9 +187,6 @@ cudaError_t launch_add_transposed(const double* part, int splits, int64_t M, int
 
 // Derivative kernels (adjoint.cu).  ao_hessian: [3][point_num][4][ao]
 // (coord [3][point_num]), `mixed` selects FP32 exponentials where a r^2 <= 30.
-// Mixed-form adjoint: G [point_num][5][ao] in FP32; grad_nucl [nucl][3] -=
-// and grad_coord [3][gstride] += (may be null); coord [3][cstride]; FP32
-// exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic.
 cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const double* coord, double cutoff, bool mixed,
                               double* ao_hessian, cudaStream_t s, const double* cusp_r = nullptr);
 // Orbital forces (adjoint.cu): which = 0 forces_mo_value, 1 forces_mo_g,
@@ -194,8 +195,5 @@ cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const doubl
 // nuc_ao[a] = AO range of nucleus a.
 cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, const int2* nuc_ao, const double* X,
                           const double* Ct, double* out, cudaStream_t s);
-cudaError_t launch_mo_adjoint_nuclear(const DevTables& T, int64_t point_num, const double* coord, int64_t cstride,
-                                      double cutoff, const float* G, double* grad_nucl, double* grad_coord,
-                                      int64_t gstride, cudaStream_t s);
 
 }  // namespace qb

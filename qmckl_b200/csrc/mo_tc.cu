@@ -54,15 +54,11 @@ constexpr int kThreads = 32 * (kEpiWarps + 2);
 
 // ------------------------------------------------------------ GEMM kernel
 
-// TWO_ACC: one accumulator for the leading product and one for the
-// corrections (short K: the split of the leading product over two halves of
-// K is not needed), so that a 128-column tile needs 256 TMEM columns and two
-// CTAs share an SM.
-template <int PIECES, int STAGES, typename OutT = double, bool TWO_ACC = false>
-__global__ void __launch_bounds__(kThreads, TWO_ACC ? 2 : 1)
+template <int PIECES, int STAGES>
+__global__ void __launch_bounds__(kThreads, 1)
 tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const int64_t M, const int n_out, const int n_tile, const int kblocks, const int comps,
-               const double* __restrict__ scales, OutT* __restrict__ out, const int64_t ldo,
+               const double* __restrict__ scales, double* __restrict__ out, const int64_t ldo,
                int* __restrict__ err) {
   constexpr int NPROD = PIECES == 3 ? 6 : 3;
   constexpr int A_TILE = BM * BK * 2;             // bytes of one A piece tile
@@ -83,7 +79,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   const int n0 = blockIdx.y * n_tile;
   // three accumulators of n_tile columns: A1*C1 (first half of K), A1*C1
   // (second half), corrections
-  constexpr int NACC = TWO_ACC ? 2 : 3;
+  constexpr int NACC = 3;
   uint32_t tmem_cols = 32;
   while ((int)tmem_cols < NACC * n_tile) tmem_cols <<= 1;
 
@@ -145,7 +141,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t a_addr = base + ia * A_TILE + kk * UMMA_K * 2;
             const uint32_t b_addr = base + PIECES * A_TILE + ib * B_TILE + kk * UMMA_K * 2;
             const bool lead = (t == NPROD - 1);                 // A1*C1
-            const bool second = !TWO_ACC && lead && (2 * kb >= kblocks);
+            const bool second = lead && (2 * kb >= kblocks);
             const uint32_t d = tmem + (uint32_t)((lead ? (second ? 1 : 0) : NACC - 1) * n_tile);
             const bool first_use = lead ? (second ? (kb == (kblocks + 1) / 2 && kk == 0) : (kb == 0 && kk == 0))
                                         : (kb == 0 && kk == 0 && t == 0);
@@ -166,17 +162,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // warp's 16-byte stores fall on distinct banks) and each row leaves in
     // one bulk copy; otherwise each warp writes its rows through a small
     // staging buffer.
-    constexpr int kPadT = 16 / (int)sizeof(OutT);
-    const int ldst = n_tile + kPadT;
+    const int ldst = n_tile + 2;
     const int ncols = n_out - n0 < n_tile ? n_out - n0 : n_tile;
-    const bool bulk = (size_t)BM * ldst * sizeof(OutT) <= (size_t)STAGES * STAGE &&
-                      ((size_t)ncols * sizeof(OutT)) % 16 == 0 && ((size_t)ldo * sizeof(OutT)) % 16 == 0 &&
+    const bool bulk = (size_t)BM * ldst * sizeof(double) <= (size_t)STAGES * STAGE && ncols % 2 == 0 && ldo % 2 == 0 &&
                       (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     if (bulk) {
-      OutT* stg = (OutT*)smem;
+      double* stg = (double*)smem;
       const int r = warp * 32 + lane;   // this thread's TMEM lane = tile row
       const int64_t row = m0 + r;
-      const bool has_second = !TWO_ACC && kblocks >= 2;
+      const bool has_second = kblocks >= 2;
       if (ok) {
         for (int c0 = 0; c0 < n_tile; c0 += 16) {
           uint32_t r0[16], r1[16], r2[16];
@@ -184,7 +178,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           tmem_ld16(ta, r0);
           if (has_second) tmem_ld16(ta + (uint32_t)n_tile, r1);
           tmem_ld16(ta + (uint32_t)((NACC - 1) * n_tile), r2);
-          OutT vals[16];
+          double vals[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             double v = (double)__uint_as_float(r0[j]) + (double)__uint_as_float(r2[j]);
@@ -193,34 +187,27 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
               const int col = n0 + c0 + j;
               v *= scales[(int)(row % comps)] * (col < n_out ? scales[kScaleCols + col] : 1.0);
             }
-            vals[j] = (OutT)v;
+            vals[j] = v;
           }
           uint4* dst = reinterpret_cast<uint4*>(stg + (size_t)r * ldst + c0);
-          if constexpr (sizeof(OutT) == 4) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              dst[q] = make_uint4(__float_as_uint(vals[4 * q]), __float_as_uint(vals[4 * q + 1]),
-                                  __float_as_uint(vals[4 * q + 2]), __float_as_uint(vals[4 * q + 3]));
-          } else {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-              const unsigned long long a = __double_as_longlong(vals[2 * q]), b = __double_as_longlong(vals[2 * q + 1]);
-              dst[q] = make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
-            }
+          for (int q = 0; q < 8; ++q) {
+            const unsigned long long a = __double_as_longlong(vals[2 * q]), b = __double_as_longlong(vals[2 * q + 1]);
+            dst[q] = make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
           }
         }
       }
       fence_async_smem();
       named_bar_sync(1, kEpiWarps * 32);   // all epilogue warps arrive, whatever their `ok`
       if (ok && row < M) {
-        bulk_store(out + row * ldo + n0, stg + (size_t)r * ldst, (uint32_t)(ncols * sizeof(OutT)));
+        bulk_store(out + row * ldo + n0, stg + (size_t)r * ldst, (uint32_t)(ncols * sizeof(double)));
         bulk_commit();
         bulk_wait_read();
       }
     } else if (ok) {
       double* stage = (double*)smem + warp * 32 * 16;     // [32 rows][16 cols] per warp; stages are idle now
       const int row_base = warp * 32;
-      const bool has_second = !TWO_ACC && kblocks >= 2;
+      const bool has_second = kblocks >= 2;
       for (int c0 = 0; c0 < n_tile; c0 += 16) {
         uint32_t r0[16], r1[16], r2[16];
         const uint32_t ta = tmem + ((uint32_t)row_base << 16) + (uint32_t)c0;
@@ -244,7 +231,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             double v = stage[rr * 16 + ((cc + rr) & 15)];
             // float16 operands carry power-of-two component and MO scales
             if constexpr (PIECES == 2) v *= scales[(int)(row % comps)] * scales[kScaleCols + col];
-            out[row * ldo + col] = (OutT)v;
+            out[row * ldo + col] = v;
           }
         }
         __syncwarp();
@@ -415,6 +402,222 @@ tc_gemm_mn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   if (warp == kEpiWarps + 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols));
+  }
+}
+
+// ------------------------------------------------------------ pulled-back weights
+//
+// gc[tile][m][pos] = sum over the MOs of C[list[m]][mo] * W[tile][pos][mo] for
+// the AOs of each tile's list (f64_tiles.cu), FP32: the weights of 32 points
+// pulled back to the AOs that reach them, 25% of all AOs on the 2000-AO
+// molecule.  M = 128 list entries (rows of the coefficient pieces, gathered by
+// the list with 16-byte cp.async into the swizzled tile), N = the tile's 160
+// positions (weight pieces in tile order, by TMA), K = the MOs; the six split
+// products of tc_gemm_kernel in its order, so that every element is the one
+// of the product over all AOs.  Warps 0..3 load the A tiles and run the
+// epilogue, warp 4 loads the B tiles, warp 5 issues the MMAs; two stages.
+// 0.155 ms on 20,352 points (all AOs of every point: 0.59 ms).
+constexpr int kPbCols = 160;            // positions of a tile
+constexpr int kPbStages = 2;
+constexpr int kPbA = 3 * BM * BK * 2, kPbB = 3 * kPbCols * BK * 2, kPbStage = kPbA + kPbB;
+
+__global__ void __launch_bounds__(kThreads, 1)
+tc_pullback_kernel(const __grid_constant__ CUtensorMap tmW, const uint16_t* __restrict__ ct, const int ldw,
+                   const int64_t ct_pstride, const int K, const int* __restrict__ klist, const int* __restrict__ kcount,
+                   const int64_t kmax, float* __restrict__ gc, int* __restrict__ err) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (tcx::smem_addr(smem_raw) & 1023u)) & 1023u);
+  uint64_t* fullA = (uint64_t*)(smem + kPbStages * kPbStage);
+  uint64_t* fullB = fullA + kPbStages;
+  uint64_t* empty = fullB + kPbStages;
+  uint64_t* acc_full = empty + kPbStages;
+  uint64_t* drained = acc_full + 1;   // the staged rows of a row block have left
+  uint32_t* tmem_slot = (uint32_t*)(drained + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int64_t tile = blockIdx.y;
+  const int nk = kcount[tile];
+  const int kblocks = (K + BK - 1) / BK;
+  constexpr uint32_t kCols = 512;   // two accumulators of 160 columns
+  if (tid == 0) {
+    for (int s = 0; s < kPbStages; ++s) {
+      mbar_init(&fullA[s], kEpiWarps * 32);
+      mbar_init(&fullB[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    mbar_init(drained, kEpiWarps * 32);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == kEpiWarps + 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                 "r"(kCols));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  // every role walks the same sequence of (row block, K block) steps g
+  if (warp == kEpiWarps) {
+    if (lane == 0) {
+      int g = 0;
+      bool ok = true;
+      for (int m0 = (int)blockIdx.x * BM; m0 < nk && ok; m0 += (int)gridDim.x * BM)
+        for (int kb = 0; kb < kblocks; ++kb, ++g) {
+          const int s = g % kPbStages;
+          if (!mbar_wait(&empty[s], ((uint32_t)(g / kPbStages) & 1u) ^ 1u, err, 21)) {
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(&fullB[s], (uint32_t)kPbB);
+          for (int q = 0; q < 3; ++q)
+            tma_load_3d(smem + s * kPbStage + kPbA + q * (kPbB / 3), &tmW, &fullB[s], kb * BK, (int)(tile * kPbCols), q);
+        }
+    }
+  } else if (warp == kEpiWarps + 1) {
+    if (lane == 0) {
+      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPbCols >> 3) << 17) |
+                             ((uint32_t)(BM >> 4) << 24);
+      constexpr int pw[6] = {2, 1, 0, 1, 0, 0}, pc[6] = {0, 1, 2, 0, 1, 0};   // weight and coefficient pieces
+      int g = 0;
+      bool ok = true;
+      for (int m0 = (int)blockIdx.x * BM; m0 < nk && ok; m0 += (int)gridDim.x * BM) {
+        for (int kb = 0; kb < kblocks; ++kb, ++g) {
+          const int s = g % kPbStages;
+          const uint32_t phase = (uint32_t)(g / kPbStages) & 1u;
+          if (!mbar_wait(&fullB[s], phase, err, 22) || !mbar_wait(&fullA[s], phase, err, 23)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t base = smem_addr(smem + s * kPbStage);
+          for (int kk = 0; kk < BK / UMMA_K && kb * BK + kk * UMMA_K < K; ++kk) {
+#pragma unroll
+            for (int t = 0; t < 6; ++t) {
+              const uint32_t a_addr = base + pc[t] * (kPbA / 3) + kk * UMMA_K * 2;
+              const uint32_t b_addr = base + kPbA + pw[t] * (kPbB / 3) + kk * UMMA_K * 2;
+              const bool lead = t == 5;
+              const bool first = kb == 0 && kk == 0 && (lead || t == 0);
+              umma_bf16(tmem + (lead ? 0u : (uint32_t)kPbCols), smem_desc(a_addr), smem_desc(b_addr), idesc,
+                        first ? 0u : 1u);
+            }
+          }
+          umma_commit(&empty[s]);
+        }
+        if (ok) umma_commit(acc_full);
+      }
+    }
+  } else {
+    int g = 0, round = 0;
+    bool ok = true;
+    for (int m0 = (int)blockIdx.x * BM; m0 < nk && ok; m0 += (int)gridDim.x * BM, ++round) {
+      // rows (tid >> 3) + 16 i of the A tile, 16-byte piece tid & 7
+      int row_ao[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int m = m0 + (tid >> 3) + 16 * i;
+        row_ao[i] = m < nk ? klist[tile * kmax + m] : -1;
+      }
+      for (int kb = 0; kb < kblocks; ++kb, ++g) {
+        const int s = g % kPbStages;
+        bool go = mbar_wait(&empty[s], ((uint32_t)(g / kPbStages) & 1u) ^ 1u, err, 24);
+        if (kb == 0 && round > 0) go = go && mbar_wait(drained, (uint32_t)(round - 1) & 1u, err, 26);
+        go = __all_sync(0xffffffffu, go);
+        if (!go) {
+          ok = false;
+          break;
+        }
+        const int c = tid & 7, col = kb * BK + c * 8;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = (tid >> 3) + 16 * i;
+          const bool in = row_ao[i] >= 0 && col < ldw;
+          const uint16_t* src = in ? ct + (int64_t)row_ao[i] * ldw + col : ct;
+          const uint32_t dst = smem_addr(smem + s * kPbStage) + (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
+#pragma unroll
+          for (int q = 0; q < 3; ++q)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst + q * (kPbA / 3)),
+                         "l"(src + (in ? q * ct_pstride : 0)), "r"(in ? 16 : 0));
+        }
+        asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
+        fence_async_smem();
+        tc_fence_before();   // after the previous row block's accumulator reads
+        mbar_arrive(&fullA[s]);
+      }
+      if (!ok) break;
+      ok = mbar_wait(acc_full, (uint32_t)round & 1u, err, 25);
+      ok = __all_sync(0xffffffffu, ok && *(volatile int*)err == 0);
+      tc_fence_after();
+      // rows 0..63 are staged in the A tiles of stage 0, rows 64..127 in those
+      // of stage 1 (all MMAs are done; the B tiles may already be loading)
+      constexpr int ldst = kPbCols + 4;
+      const int r = warp * 32 + lane;
+      float* stg = (float*)(smem + (r >> 6) * kPbStage) + (r & 63) * ldst;
+      if (ok) {
+        for (int c0 = 0; c0 < kPbCols; c0 += 16) {
+          uint32_t r0[16], r2[16];
+          const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+          tmem_ld16(ta, r0);
+          tmem_ld16(ta + (uint32_t)kPbCols, r2);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            float v[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h)
+              v[h] = (float)((double)__uint_as_float(r0[4 * q + h]) + (double)__uint_as_float(r2[4 * q + h]));
+            *reinterpret_cast<float4*>(stg + c0 + 4 * q) = make_float4(v[0], v[1], v[2], v[3]);
+          }
+        }
+      }
+      fence_async_smem();
+      if (ok && m0 + r < nk) {
+        bulk_store(gc + ((size_t)tile * kmax + m0 + r) * kPbCols, stg, kPbCols * 4u);
+        bulk_commit();
+        bulk_wait_read();
+      }
+      mbar_arrive(drained);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kEpiWarps + 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols));
+  }
+}
+
+// Weight rows w[(p, c)][M] as 3 bfloat16 pieces, in the points' order
+// (rows, for dL/dC) and in tile order (tiled [tile][c * 32 + p], zero past the
+// points; for the pulled-back weights).  Either may be null.  A thread per 8
+// columns of a tile-order row.
+__global__ void __launch_bounds__(256)
+split_weights_kernel(const double* __restrict__ w, const int64_t P, const int M, const int* __restrict__ perm,
+                     const int64_t tiles, const int ldw, uint16_t* __restrict__ rows, uint16_t* __restrict__ tiled) {
+  const int cw = ldw / 8;
+  const int64_t total = tiles * kPbCols * cw, rstride = P * 5 * ldw, tstride = tiles * kPbCols * ldw;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t tr = i / cw;
+    const int c8 = (int)(i - tr * cw) * 8;
+    const int64_t tile = tr / kPbCols;
+    const int pos = (int)(tr - tile * kPbCols), c = pos >> 5;
+    const int64_t q = tile * 32 + (pos & 31);
+    uint16_t pc[3][8];
+    int64_t row = -1;
+    if (q < P) row = (perm ? (int64_t)perm[q] : q) * 5 + c;
+#pragma unroll
+    for (int h = 0; h < 8; ++h) {
+      uint16_t o[3];
+      split3_bf16(row >= 0 && c8 + h < M ? w[row * M + c8 + h] : 0.0, o);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) pc[k][h] = o[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const uint4 v = *reinterpret_cast<const uint4*>(pc[k]);
+      if (rows != nullptr && row >= 0) *reinterpret_cast<uint4*>(rows + k * rstride + row * ldw + c8) = v;
+      if (tiled != nullptr) *reinterpret_cast<uint4*>(tiled + k * tstride + tr * ldw + c8) = v;
+    }
   }
 }
 
@@ -597,13 +800,13 @@ int sm_count() {
   return sms;
 }
 
-template <int PIECES, int STAGES, typename OutT = double, bool TWO_ACC = false>
+template <int PIECES, int STAGES>
 cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int64_t M, int n_out, int n_tile, int n_tiles,
-                        int kblocks, int comps, const double* scales, OutT* out, int64_t ldo, int* err,
+                        int kblocks, int comps, const double* scales, double* out, int64_t ldo, int* err,
                         cudaStream_t s) {
   const size_t stage = (size_t)PIECES * (BM * BK * 2 + (size_t)n_tile * BK * 2);
   const size_t smem = 1024 + STAGES * stage + (2 * STAGES + 1) * 8 + 16;
-  auto kern = tc_gemm_kernel<PIECES, STAGES, OutT, TWO_ACC>;
+  auto kern = tc_gemm_kernel<PIECES, STAGES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)n_tiles);
@@ -814,7 +1017,7 @@ cudaError_t tc_prime_unfused() {
   cudaFuncAttributes a;
   cudaError_t e = cudaFuncGetAttributes(&a, ao_split_kernel<3, 5>);
   if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, ao_split_kernel<3, 1>);
-  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, tc_gemm_kernel<3, 2, double, false>);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, tc_gemm_kernel<3, 2>);
   return e;
 }
 
@@ -890,20 +1093,41 @@ cudaError_t tc_gemm_tn_split(const void* x, int64_t ldx, int64_t x_pstride, int6
   return cudaGetLastError();
 }
 
-cudaError_t tc_gemm_nt(const void* x, int64_t ldx, int64_t x_pstride, int64_t rows, int64_t k, const void* y,
-                       int64_t ldy, int64_t y_pstride, int64_t n, float* out, int64_t ldo, int* err, cudaStream_t s) {
-  if (rows <= 0 || n <= 0) return cudaSuccess;
-  if (ldx % 8 != 0 || ldy % 8 != 0 || x_pstride % 8 != 0 || y_pstride % 8 != 0) return cudaErrorInvalidValue;
-  // 128-column MO tiles, one stage, two accumulators: ~99 KB of shared
-  // memory and 256 TMEM columns, two CTAs per SM (one's epilogue overlaps
-  // the other's loads and MMAs); K (the MO count) is short
-  const int n_tile = 128;
-  const int n_tiles = (int)((n + n_tile - 1) / n_tile);
-  CUtensorMap tx, ty;
-  if (!make_map(&tx, x, k, rows, ldx, 3, x_pstride, BM)) return cudaErrorInvalidValue;
-  if (!make_map(&ty, y, k, n, ldy, 3, y_pstride, n_tile)) return cudaErrorInvalidValue;
-  const int kblocks = (int)((k + BK - 1) / BK);
-  return launch_gemm<3, 1, float, true>(tx, ty, rows, (int)n, n_tile, n_tiles, kblocks, 1, nullptr, out, ldo, err, s);
+cudaError_t tc_split_weights(const double* w, int64_t P, int M, const int* perm, int ldw, void* rows, void* tiled,
+                             cudaStream_t s) {
+  if (P <= 0) return cudaSuccess;
+  if (ldw < M || ldw % 8 != 0) return cudaErrorInvalidValue;
+  const int64_t tiles = (P + 31) / 32;
+  const int64_t total = tiles * kPbCols * (ldw / 8);
+  const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 16);
+  split_weights_kernel<<<grid, 256, 0, s>>>(w, P, M, perm, tiles, ldw, (uint16_t*)rows, (uint16_t*)tiled);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t tc_pullback(const void* tiled, int ldw, int64_t tiles, int M, const void* ct, int64_t ao_num,
+                        const int* klist, const int* kcount, float* gc, int* err, cudaStream_t s) {
+  if (tiles <= 0 || M <= 0) return cudaSuccess;
+  if (ldw % 8 != 0 || err == nullptr) return cudaErrorInvalidValue;
+  CUtensorMap tw;
+  if (!make_map(&tw, tiled, M, tiles * kPbCols, ldw, 3, tiles * kPbCols * ldw, kPbCols)) return cudaErrorInvalidValue;
+  const size_t smem = 1024 + kPbStages * (size_t)kPbStage + (3 * kPbStages + 2) * 8 + 16;
+  cudaError_t e = cudaFuncSetAttribute(tc_pullback_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  // one CTA per SM: a CTA per tile once the tiles fill the SMs twice, else one
+  // per row block of half the AOs
+  const int64_t gx = tiles >= 2 * sm_count() ? 1 : std::max<int64_t>(1, (ao_num + 2 * BM - 1) / (2 * BM));
+  for (int64_t t0 = 0; t0 < tiles; t0 += 65535) {   // grid.y limit
+    const int64_t n = std::min<int64_t>(65535, tiles - t0);
+    if (t0 > 0 && !make_map(&tw, (const uint16_t*)tiled + t0 * kPbCols * ldw, M, n * kPbCols, ldw, 3,
+                            tiles * kPbCols * ldw, kPbCols))
+      return cudaErrorInvalidValue;
+    tc_pullback_kernel<<<dim3((unsigned)gx, (unsigned)n), kThreads, smem, s>>>(
+        tw, (const uint16_t*)ct, ldw, ao_num * ldw, M, klist + t0 * ao_num, kcount + t0, ao_num,
+        gc + (size_t)t0 * ao_num * kPbCols, err);
+    count_launch();
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace qb

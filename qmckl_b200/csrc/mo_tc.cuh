@@ -123,7 +123,14 @@ cudaError_t tc_run_scratch(const DevTables& T, const TcPlan& plan, int64_t point
 //   tc_gemm_tn_split : part[z][a][b] = sum over the rows of K slice z of
 //                   X[r][a] Y[r][b], z < tc_tn_splits(rows, kps); slices of
 //                   kps * 32 rows (the caller sums the partials)
-//   tc_gemm_nt    : out[r][j] (FP32, pitch ldo) = sum_k X[r][k] Y[j][k]
+//   tc_split_weights : FP64 weights w[(p, c)][M] -> pieces of rows [3][5 P][ldw]
+//                   and of tile-order rows [3][tiles * 160][ldw] (tiles of 32
+//                   points in the order perm, row c * 32 + p, zero past the
+//                   points); either may be null
+//   tc_pullback   : gc[tile][m][160] (FP32) = sum over the MOs of
+//                   C[klist[tile][m]][mo] * W[tile][pos][mo], m < kcount[tile],
+//                   from tile-order weight pieces and the pieces ct [3][ao][ldw]
+//                   of coefficient_t (klist, gc rows: ao_num per tile)
 // err: a device error word set by a timed-out barrier wait.
 cudaError_t tc_split_rows(const double* x, int64_t rows, int cols, int64_t ldx, void* pieces, int ldp,
                           int64_t pstride, cudaStream_t s);
@@ -131,8 +138,10 @@ int tc_tn_splits(int64_t rows, int kps);
 cudaError_t tc_gemm_tn_split(const void* x, int64_t ldx, int64_t x_pstride, int64_t a_num, const void* y, int64_t ldy,
                              int64_t y_pstride, int b_num, int64_t rows, int kps, double* part, int* err,
                              cudaStream_t s);
-cudaError_t tc_gemm_nt(const void* x, int64_t ldx, int64_t x_pstride, int64_t rows, int64_t k, const void* y,
-                       int64_t ldy, int64_t y_pstride, int64_t n, float* out, int64_t ldo, int* err, cudaStream_t s);
+cudaError_t tc_split_weights(const double* w, int64_t P, int M, const int* perm, int ldw, void* rows, void* tiled,
+                             cudaStream_t s);
+cudaError_t tc_pullback(const void* tiled, int ldw, int64_t tiles, int M, const void* ct, int64_t ao_num,
+                        const int* klist, const int* kcount, float* gc, int* err, cudaStream_t s);
 
 // What the fixed-scratch entry point needs from a context whose basis and
 // coefficient pieces are already on the device (device.cu).

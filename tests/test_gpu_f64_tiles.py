@@ -111,6 +111,30 @@ def test_adjoint_tiles(cid, P, m):
         assert np.abs(got.cpu().numpy() - want).max() <= 1e-10 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("cid,P,m", [(0, 1, 3), (0, 32, 64), (0, 33, 81), (0, 100, 17), ("hl", 40, 101), (1, 50, 161),
+                                     (0, 12000, 20)])
+def test_mixed_adjoint_tiles(cid, P, m):
+    """The mixed adjoint's pulled-back weights over the tiles' AO lists, at the edges of their row blocks (128), K
+    blocks (64 MOs) and tiles: against the FP64 form, within the mixed adjoint's bound (test_gpu_adjoint.py)."""
+    d = _molecule(cid, m, 600 + P)
+    pts = _points(d, P, 700 + P)
+    t = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")  # noqa: E731
+    c, dw = t(pts.T), t(np.random.default_rng(800 + P).standard_normal((P, 5, m)))
+    res = []
+    for form in (pq.FORM_FP64, pq.FORM_MIXED):
+        ctx = make_context(d, points=False, form=form)
+        gn, gr = (torch.full(s, float("nan"), dtype=torch.float64, device="cuda") for s in ((d["nucl_num"], 3), (3, P)))
+        torch.cuda.synchronize()
+        try:
+            pq.b200_mo_vgl_adjoint_device(ctx, P, c.data_ptr(), dw.data_ptr(), 0, gn.data_ptr(), gr.data_ptr())
+            pq.b200_synchronize(ctx)
+        finally:
+            pq.context_destroy(ctx)
+        res.append((gn, gr))
+    for ref, got in zip(*res):
+        assert float((got - ref).abs().max()) <= 1e-6 * float(ref.abs().max())
+
+
 def test_adjoint_coefficients_repeat():
     """dL/dC is summed in a fixed order: the same bits in every run."""
     d = _molecule(0, 90, 8)
