@@ -1,5 +1,5 @@
-// Derivative kernels of the AO VGL: the AO Hessian getter, the adjoint of MO
-// VGL with respect to the nuclear and point coordinates, the orbital forces.
+// The adjoint of MO VGL with respect to the nuclear and point coordinates, and
+// the orbital forces.
 //
 // Quantities (derivatives with respect to the point coordinates r; an AO
 // centred on nucleus A depends on r - R_A, so d/dR_A = -d/dr):
@@ -18,186 +18,18 @@
 // r^2 > cutoff * range, primitives sorted by exponent with a break at
 // a r^2 > cutoff, AO skipped when its contracted radial value is zero.
 //
-// The AO Hessian takes one warp per (point, nucleus block), as the forward AO
-// kernel; the adjoint works on compact tiles (tile_deriv_kernel): with the
+// The adjoint works on compact tiles (tile_deriv_kernel): with the
 // loss weights pulled back through the MO coefficients, G = W . C, it forms
 // q_d = G0 d_d chi + sum_e G_{1+e} H_ed + G4 T_d per AO; -q summed over a
 // nucleus's AOs and the points is dL/dR, q summed over all AOs dL/dr.
 #include <algorithm>
 #include <type_traits>
 
+#include "ao_derivs.cuh"
 #include "kernels.cuh"
 
 namespace qb {
 namespace {
-
-constexpr int kWarpsD = 8;
-constexpr double kShiftD = 1.e-20;
-
-struct DerivSmem {
-  double rad[kBlockSlots][4];   // R, R1, R2, R3 of the block's shells
-  double nuc[kBlockNuc][4];     // displacement, r^2 (negative when screened out)
-  uint8_t act[kBlockSlots];     // the shells whose nucleus is in range
-};
-
-// x^a and its first three derivatives (Leibniz, one factor x at a time)
-template <typename F>
-__device__ __forceinline__ void pow_derivs(F x, int a, F (&q)[4]) {
-  if (a <= 3) {
-    // without branches (lanes of a warp hold different exponents): with
-    // f_i = x for i <= a, 1 otherwise, x^a = f1 f2 f3, and the derivatives
-    // a x^(a-1), a (a-1) x^(a-2), a (a-1) (a-2) vanish where they must
-    const F f1 = a >= 1 ? x : F(1), f2 = a >= 2 ? x : F(1), f3 = a >= 3 ? x : F(1);
-    const F fa = F(a);
-    q[2] = fa * (fa - F(1)) * f3;
-    q[1] = fa * (f2 * f3);
-    q[0] = f1 * (f2 * f3);
-    q[3] = fa * (fa - F(1)) * (fa - F(2));
-    return;
-  }
-  q[0] = F(1); q[1] = F(0); q[2] = F(0); q[3] = F(0);
-  for (int i = 0; i < a; ++i) {
-    q[3] = q[3] * x + F(3) * q[2];
-    q[2] = q[2] * x + F(2) * q[1];
-    q[1] = q[1] * x + q[0];
-    q[0] = q[0] * x;
-  }
-}
-
-template <bool MIXED>
-__device__ __forceinline__ void stage_deriv(const DevTables& T, DerivSmem& sm, const int4 blk, const int2 slots,
-                                            double px, double py, double pz, double cutoff, int lane) {
-  const int nn = blk.y - blk.x;
-  if (lane < nn) {
-    const int n = blk.x + lane;
-    const int N = T.nucl_num;
-    const double x = px - T.nucl_coord[n];
-    const double y = py - T.nucl_coord[n + N];
-    const double z = pz - T.nucl_coord[n + 2 * N];
-    const double r2 = x * x + y * y + z * z;
-    const bool in = !(r2 > cutoff * T.nucleus_range[n]);
-    sm.nuc[lane][0] = x;
-    sm.nuc[lane][1] = y;
-    sm.nuc[lane][2] = z;
-    sm.nuc[lane][3] = in ? r2 : -1.0;
-  }
-  __syncwarp();
-  // shells of screened-out nuclei are not staged (the AO loop tests the nucleus first)
-  const int nlive = pack_live_slots(T.slot_nuc, blk.x, slots, sm.nuc, sm.act, lane);
-  for (int i = lane; i < nlive; i += 32) {
-    const int ls = sm.act[i];
-    const int s = slots.x + ls;
-    const int nucl = T.slot_nuc[s];
-    const double r2 = sm.nuc[nucl - blk.x][3];
-    double acc[4] = {0., 0., 0., 0.};
-    {
-      const int2 cr = T.slot_coef[s];
-      const int p0 = T.nuc_prim_start[nucl];
-      for (int j = cr.x; j < cr.y; ++j) {
-        const double a = T.expo[p0 + T.coef_prim[j]];
-        const double ar2 = a * r2;
-        if (ar2 > cutoff) break;   // primitives sorted by exponent
-        const double e = (MIXED && ar2 <= 30.0) ? (double)expf(-(float)ar2) : exp(-ar2);
-        const double ce = T.coef_val[j] * e;
-        acc[0] += ce;
-        acc[1] -= a * ce;
-        acc[2] += a * a * ce;
-        acc[3] -= a * a * a * ce;
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) sm.rad[ls][c] = acc[c];
-  }
-  __syncwarp();
-}
-
-// Hessian H[d][e] and gradient of the Laplacian T[d] of one AO (times its
-// factor f), plus its gradient g[d], in arithmetic F.  The radial
-// combinations that cancel near their zeros, lap R = 4 s R2 + 6 R1 and
-// k3 = 20 R2 + 8 s R3, come in formed in FP64.
-template <typename F>
-__device__ __forceinline__ void ao_derivs(int code, F f, const F (&v)[3], const F (&R)[3], F lapR, F k3,
-                                          F (&g)[3], F (&H)[3][3], F (&Tl)[3]) {
-  const int ax = code & 15, by = (code >> 4) & 15, cz = (code >> 8) & 15, l = (code >> 12) & 15;
-  F X[4], Y[4], Z[4];
-  pow_derivs<F>(v[0], ax, X);
-  pow_derivs<F>(v[1], by, Y);
-  pow_derivs<F>(v[2], cz, Z);
-  const F P = X[0] * Y[0] * Z[0] + (l >= 1 ? F(kShiftD) : F(0));
-  const F Pd[3] = {X[1] * Y[0] * Z[0], X[0] * Y[1] * Z[0], X[0] * Y[0] * Z[1]};
-  F Pdd[3][3];
-  Pdd[0][0] = X[2] * Y[0] * Z[0];
-  Pdd[1][1] = X[0] * Y[2] * Z[0];
-  Pdd[2][2] = X[0] * Y[0] * Z[2];
-  Pdd[0][1] = Pdd[1][0] = X[1] * Y[1] * Z[0];
-  Pdd[0][2] = Pdd[2][0] = X[1] * Y[0] * Z[1];
-  Pdd[1][2] = Pdd[2][1] = X[0] * Y[1] * Z[1];
-  const F lapP = Pdd[0][0] + Pdd[1][1] + Pdd[2][2];
-  const F dlapP[3] = {X[3] * Y[0] * Z[0] + X[1] * Y[2] * Z[0] + X[1] * Y[0] * Z[2],
-                      X[2] * Y[1] * Z[0] + X[0] * Y[3] * Z[0] + X[0] * Y[1] * Z[2],
-                      X[2] * Y[0] * Z[1] + X[0] * Y[2] * Z[1] + X[0] * Y[0] * Z[3]};
-  const F Rd[3] = {F(2) * v[0] * R[1], F(2) * v[1] * R[1], F(2) * v[2] * R[1]};
-  F Rdd[3][3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d)
-#pragma unroll
-    for (int e = 0; e < 3; ++e) Rdd[d][e] = F(4) * v[d] * v[e] * R[2] + (d == e ? F(2) * R[1] : F(0));
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    g[d] = f * (Pd[d] * R[0] + P * Rd[d]);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) H[d][e] = f * (Pdd[d][e] * R[0] + Pd[d] * Rd[e] + Pd[e] * Rd[d] + P * Rdd[d][e]);
-    F t = F(0);
-#pragma unroll
-    for (int e = 0; e < 3; ++e) t += Pdd[d][e] * Rd[e] + Pd[e] * Rdd[d][e];
-    Tl[d] = f * (dlapP[d] * R[0] + lapP * Rd[d] + F(2) * t + Pd[d] * lapR + P * v[d] * k3);
-  }
-}
-
-// AO Hessian: out = ao_hessian[3][point_num][4][ao].  MIXED: FP32
-// exponentials where a r^2 <= 30.
-template <bool MIXED>
-__global__ void __launch_bounds__(kWarpsD * 32)
-hessian_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord, const double cutoff,
-               double* __restrict__ out, const double* __restrict__ cusp_r) {
-  __shared__ DerivSmem smem[kWarpsD];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  DerivSmem& sm = smem[warp];
-  const int64_t A = T.ao_num;
-  const int64_t stride = (int64_t)gridDim.x * kWarpsD;
-  // one warp per point, through its nucleus blocks (as the FP64 AO kernel)
-  for (int64_t p = (int64_t)blockIdx.x * kWarpsD + warp; p < point_num; p += stride) {
-    for (int b = 0; b < T.nblock; ++b) {
-      const int4 blk = T.block[b];
-      const int2 slots = T.block_slots[b];
-      stage_deriv<MIXED>(T, sm, blk, slots, coord[p], coord[p + point_num], coord[p + 2 * point_num], cutoff, lane);
-      for (int k = blk.z + lane; k < blk.w; k += 32) {
-        const int code = T.ao_code[k];
-        const int slot = (code >> 16) & 255, nl = (code >> 24) & 31;
-        const double r2 = sm.nuc[nl][3];
-        const double* Rs = sm.rad[slot];
-        double g[3], H[3][3] = {{0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}}, Tl[3] = {0., 0., 0.};
-        if (r2 >= 0.0 && Rs[0] != 0.0 && !cusp_masked(cusp_r, (code >> 12) & 15, blk.x + nl, r2, false)) {
-          const double lapR = 4.0 * r2 * Rs[2] + 6.0 * Rs[1];
-          const double k3 = 20.0 * Rs[2] + 8.0 * r2 * Rs[3];
-          const double v[3] = {sm.nuc[nl][0], sm.nuc[nl][1], sm.nuc[nl][2]};
-          const double R[3] = {Rs[0], Rs[1], Rs[2]};
-          ao_derivs<double>(code, T.ao_factor[k], v, R, lapR, k3, g, H, Tl);
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          double* o = out + ((int64_t)i * point_num + p) * 4 * A;
-          o[k] = H[i][0];
-          o[A + k] = H[i][1];
-          o[2 * A + k] = H[i][2];
-          o[3 * A + k] = Tl[i];
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
 
 // One AO of the FP64 adjoint, exponents known at compile time: with the
 // pulled-back weights (G0, g = G1..G3, G4) and P's derivatives,
@@ -476,16 +308,6 @@ cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, con
     case 3: forces_ao_kernel<<<grid, 256, 0, s>>>(P, A, N, nuc_ao, X, out); break;
     default: return cudaErrorInvalidValue;
   }
-  count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const double* coord, double cutoff, bool mixed,
-                              double* ao_hessian, cudaStream_t s, const double* cusp_r) {
-  if (point_num <= 0) return cudaSuccess;
-  const int grid = (int)std::min<int64_t>((point_num + kWarpsD - 1) / kWarpsD, 148 * 8);   // warps = points
-  auto k = mixed ? hessian_kernel<true> : hessian_kernel<false>;
-  k<<<grid, kWarpsD * 32, 0, s>>>(T, point_num, coord, cutoff, ao_hessian, cusp_r);
   count_launch();
   return cudaGetLastError();
 }

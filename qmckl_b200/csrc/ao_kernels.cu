@@ -1,5 +1,4 @@
-// AO kernels: FP64 AO VGL / AO value, the primitive and shell VGL getters, and
-// the mixed-precision AO VGL kernel that feeds the tensor-core MO contraction.
+// AO kernels: FP64 AO VGL / AO value, the primitive and shell VGL getters.
 //
 // Arithmetic follows the reference's production kernel
 // qmckl_compute_ao_vgl_hpc_gaussian (org/qmckl_ao.org:8601-8973):
@@ -18,10 +17,9 @@
 // radial VGL of the block's shells into shared memory, then sweep the block's
 // contiguous AO range with consecutive lanes on consecutive AOs, so every
 // store of ao_vgl[point][comp][k] is a 256-byte coalesced row segment.
-#include <cuda_bf16.h>
+#include <algorithm>
 
 #include "kernels.cuh"
-#include "split.cuh"
 
 namespace qb {
 
@@ -136,15 +134,12 @@ __device__ __forceinline__ void stage_block(const DevTables& T, WarpSmem& sm, co
   __syncwarp();
 }
 
-// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1).  SPLIT: each value
-// stored as 3 bfloat16 pieces (split.cuh) at pieces[q * pstride + row * lda
-// + ao], rows p * COMPS + c, instead of FP64 in `out`.
-template <int COMPS, bool SPLIT = false>
+// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1).
+template <int COMPS>
 __global__ void __launch_bounds__(kWarps * 32)
 ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord,
               const double cutoff, const bool dp_exp, double* __restrict__ out,
-              uint16_t* __restrict__ pieces = nullptr, const int64_t lda = 0, const int64_t pstride = 0,
-              const double* __restrict__ cusp_r = nullptr) {
+              const double* __restrict__ cusp_r) {
   __shared__ WarpSmem smem[kWarps];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -161,12 +156,11 @@ ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restri
     const double px = coord[p], py = coord[p + point_num], pz = coord[p + 2 * point_num];
     stage_block<COMPS>(T, sm, blk, slots, px, py, pz, cutoff, dp_exp, lane);
     double* __restrict__ row = out + p * COMPS * A;
-    // The lanes' 32-AO groups start on a 128-byte boundary of the output
-    // (64 bytes of the bfloat16 pieces): a group that straddles it writes
-    // partial sectors and ~20% fewer bytes per second (2.87 ms against 2.37
-    // for the 13 GB of the config-1 molecule's AO VGL, stores alone).
-    const int sh = SPLIT ? (int)((reinterpret_cast<uintptr_t>(pieces + p * COMPS * lda + blk.z) >> 1) & 31)
-                         : (int)((reinterpret_cast<uintptr_t>(row + blk.z) >> 3) & 15);
+    // The lanes' 32-AO groups start on a 128-byte boundary of the output: a
+    // group that straddles it writes partial sectors and ~20% fewer bytes per
+    // second (2.87 ms against 2.37 for the 13 GB of the config-1 molecule's AO
+    // VGL, stores alone).
+    const int sh = (int)((reinterpret_cast<uintptr_t>(row + blk.z) >> 3) & 15);
     for (int k = blk.z - sh + lane; k < blk.w; k += 32) {
       if (k < blk.z) continue;
       const int code = T.ao_code[k];
@@ -208,25 +202,13 @@ ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restri
           }
         }
       }
-      if constexpr (SPLIT) {
-#pragma unroll
-        for (int c = 0; c < COMPS; ++c) {
-          uint16_t pc[3];
-          split3_bf16(v[c], pc);
-          uint16_t* dst = pieces + (p * COMPS + c) * lda + k;
-          dst[0] = pc[0];
-          dst[pstride] = pc[1];
-          dst[2 * pstride] = pc[2];
-        }
-      } else {
-        // streaming stores: the array is written once and not read back here
-        __stcs(&row[k], v[0]);
-        if (COMPS == 5) {
-          __stcs(&row[A + k], v[1]);
-          __stcs(&row[2 * A + k], v[2]);
-          __stcs(&row[3 * A + k], v[3]);
-          __stcs(&row[4 * A + k], v[4]);
-        }
+      // streaming stores: the array is written once and not read back here
+      __stcs(&row[k], v[0]);
+      if (COMPS == 5) {
+        __stcs(&row[A + k], v[1]);
+        __stcs(&row[2 * A + k], v[2]);
+        __stcs(&row[3 * A + k], v[3]);
+        __stcs(&row[4 * A + k], v[4]);
       }
     }
     __syncwarp();
@@ -321,18 +303,7 @@ cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const doubl
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
   const int grid = grid_for(point_num);   // one warp per point
-  ao_f64_kernel<5><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_vgl, nullptr, 0, 0, cusp_r);
-  count_launch();
-  return cudaGetLastError();
-}
-
-cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const double* coord, double cutoff,
-                                 bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s) {
-  if (point_num <= 0) return cudaSuccess;
-  if (lda < T.ao_num || lda % 8 != 0 || pstride % 8 != 0) return cudaErrorInvalidValue;
-  const int grid = grid_for(point_num);   // one warp per point
-  ao_f64_kernel<5, true><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, nullptr,
-                                                      (uint16_t*)pieces, lda, pstride);
+  ao_f64_kernel<5><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_vgl, cusp_r);
   count_launch();
   return cudaGetLastError();
 }
@@ -341,8 +312,7 @@ cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const dou
                                 double cutoff, bool dp_exp, double* ao_value, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
   const int grid = grid_for(point_num);   // one warp per point
-  ao_f64_kernel<1><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_value, nullptr, 0, 0,
-                                                cusp_r);
+  ao_f64_kernel<1><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_value, cusp_r);
   count_launch();
   return cudaGetLastError();
 }

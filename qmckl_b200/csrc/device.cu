@@ -376,6 +376,7 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
+  AoRowTables rows{};   // in f64_sph: the shell records and the segments of the AO array kernels
 };
 
 namespace {
@@ -715,6 +716,87 @@ qmckl_exit_code copy_out(qmckl_context context, DeviceState* ds, double* host, c
 
 DeviceState* state(qmckl_context context) { return ctx_of(context)->extra; }
 
+// The per-shell records of the FP64 tile and AO array kernels (basis order),
+// and the AO array kernels' segments.
+qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
+  const char* fname = "qmckl_b200_mo_fp64";
+  Context* ctx = ctx_of(context);
+  const AoBasisRec& B = ctx->ao_basis;
+  const AoDerived& d = B.d;
+  const int64_t A = B.ao_num, S = B.shell_num, N = ctx->nucleus.num;
+  const double cutoff = cutoff_of(ctx);
+  if (ds->f64_sph.p && ds->f64_sph_basis == B.basis_version && ds->f64_sph_nucl == ctx->nucleus.coord_version &&
+      ds->f64_sph_cutoff == cutoff)
+    return QMCKL_SUCCESS;
+  std::vector<F64Shell> sh((size_t)S);
+  for (int64_t m = 0; m < N; ++m)
+    for (int64_t s = B.nucleus_index[m]; s < B.nucleus_index[m] + B.nucleus_shell_num[m]; ++s) {
+      F64Shell& e = sh[(size_t)s];
+      const int l = B.shell_ang_mom[s];
+      const int64_t a0 = d.ao_index[s];
+      e.x = ctx->nucleus.coord[m];
+      e.y = ctx->nucleus.coord[m + N];
+      e.z = ctx->nucleus.coord[m + 2 * N];
+      e.r2max = shell_r2max(ctx, (int)s, (int)m, cutoff);
+      e.crange = cutoff * d.nucleus_range[m];
+      e.a0 = (int32_t)a0;
+      e.na = (int32_t)std::max<int64_t>(0, std::min<int64_t>((int64_t)(l + 1) * (l + 2) / 2, A - a0));
+      e.cb = d.shell_coef_start[s];
+      e.ce = d.shell_coef_start[s + 1];
+      e.l = l;
+      e.nucl = (int32_t)m;
+    }
+  std::vector<int2> segs;
+  size_t at[2];
+  for (int m = 0; m < 2; ++m) {
+    AoSegments& g = ds->rows.seg[m];
+    const int64_t w = g.width = ao_segment_width(m, A);
+    g.nseg = (int)((A + w - 1) / w);
+    at[m] = segs.size();
+    int64_t s0 = 0;
+    for (int64_t a0 = 0; a0 < A; a0 += w) {
+      while (s0 < S && sh[(size_t)s0].a0 + sh[(size_t)s0].na <= a0) ++s0;
+      int64_t s1 = s0;
+      while (s1 < S && sh[(size_t)s1].a0 < a0 + w) ++s1;
+      segs.push_back(make_int2((int)s0, (int)s1));
+    }
+    g.run_shells.assign((size_t)g.nseg + 1, 0);
+    for (int n = 1; n <= g.nseg; ++n)
+      for (int i = 0; i + n <= g.nseg; ++i)
+        g.run_shells[n] = std::max(g.run_shells[n], segs[at[m] + i + n - 1].y - segs[at[m] + i].x);
+  }
+  const size_t sb = sizeof(F64Shell) * (size_t)S;
+  qmckl_exit_code rc = ensure(context, ds->f64_sph, sb + sizeof(int2) * segs.size(), fname);
+  if (rc != QMCKL_SUCCESS) return rc;
+  QB_CUDA(cudaMemcpy(ds->f64_sph.p, sh.data(), sb, cudaMemcpyHostToDevice), fname);
+  QB_CUDA(cudaMemcpy((uint8_t*)ds->f64_sph.p + sb, segs.data(), sizeof(int2) * segs.size(), cudaMemcpyHostToDevice),
+          fname);
+  ds->rows.sh = (const F64Shell*)ds->f64_sph.p;
+  for (int m = 0; m < 2; ++m) ds->rows.seg[m].seg = (const int2*)((uint8_t*)ds->f64_sph.p + sb) + at[m];
+  ds->f64_sph_basis = B.basis_version;
+  ds->f64_sph_nucl = ctx->nucleus.coord_version;
+  ds->f64_sph_cutoff = cutoff;
+  return QMCKL_SUCCESS;
+}
+
+// Point order of P points: perm[P], then the sort's scratch (256-byte aligned).
+size_t perm_bytes(int64_t P) { return (sizeof(int) * (size_t)P + 255) / 256 * 256; }
+size_t order_bytes(int64_t P) { return perm_bytes(P) + (point_order_bytes(P) + 255) / 256 * 256; }
+
+// Box of the nuclei, widened by 4 bohr: the grid of the spatial point order.
+void nucleus_box(const Context* ctx, double* lo, double* hi) {
+  const int64_t N = ctx->nucleus.num;
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = 1e300;
+    hi[d] = -1e300;
+  }
+  for (int64_t n = 0; n < N; ++n)
+    for (int d = 0; d < 3; ++d) {
+      lo[d] = std::min(lo[d], ctx->nucleus.coord[n + d * N] - 4.0);
+      hi[d] = std::max(hi[d], ctx->nucleus.coord[n + d * N] + 4.0);
+    }
+}
+
 // ---- compute steps on the device (no date logic) ----
 
 // cusp_r (optional): zero the AOs that the cusp adjustment leaves out of the
@@ -732,6 +814,16 @@ qmckl_exit_code run_ao_value(qmckl_context context, DeviceState* ds, int64_t P, 
   Context* ctx = ctx_of(context);
   QB_CUDA(launch_ao_value_f64(ds->T, P, coord, cutoff_of(ctx), ctx->precision > 23, out, ds->stream, cusp_r),
           "qmckl_b200_ao_value");
+  return QMCKL_SUCCESS;
+}
+
+qmckl_exit_code run_ao_hessian(qmckl_context context, DeviceState* ds, int64_t P, const double* coord, double* out,
+                               const double* cusp_r = nullptr) {
+  Context* ctx = ctx_of(context);
+  qmckl_exit_code rc = sync_f64_shells(context, ds);
+  if (rc != QMCKL_SUCCESS) return rc;
+  QB_CUDA(launch_ao_hessian(ds->T, ds->rows, P, coord, cutoff_of(ctx), ctx->precision <= 23, out, ds->stream, cusp_r),
+          "qmckl_b200_ao_hessian");
   return QMCKL_SUCCESS;
 }
 
@@ -859,62 +951,6 @@ qmckl_exit_code prepare_mixed(qmckl_context context, DeviceState* ds) {
     ds->env_inv_log2q = il;
     ds->env_basis_version = ctx->ao_basis.basis_version;
   }
-  return QMCKL_SUCCESS;
-}
-
-// Point order of P points: perm[P], then the sort's scratch (256-byte aligned).
-size_t perm_bytes(int64_t P) { return (sizeof(int) * (size_t)P + 255) / 256 * 256; }
-size_t order_bytes(int64_t P) { return perm_bytes(P) + (point_order_bytes(P) + 255) / 256 * 256; }
-
-// Box of the nuclei, widened by 4 bohr: the grid of the spatial point order.
-void nucleus_box(const Context* ctx, double* lo, double* hi) {
-  const int64_t N = ctx->nucleus.num;
-  for (int d = 0; d < 3; ++d) {
-    lo[d] = 1e300;
-    hi[d] = -1e300;
-  }
-  for (int64_t n = 0; n < N; ++n)
-    for (int d = 0; d < 3; ++d) {
-      lo[d] = std::min(lo[d], ctx->nucleus.coord[n + d * N] - 4.0);
-      hi[d] = std::max(hi[d], ctx->nucleus.coord[n + d * N] + 4.0);
-    }
-}
-
-// The per-shell records of the FP64 tile kernels (basis order).
-qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
-  const char* fname = "qmckl_b200_mo_fp64";
-  Context* ctx = ctx_of(context);
-  const AoBasisRec& B = ctx->ao_basis;
-  const AoDerived& d = B.d;
-  const int64_t A = B.ao_num, S = B.shell_num, N = ctx->nucleus.num;
-  const double cutoff = cutoff_of(ctx);
-  if (ds->f64_sph.p && ds->f64_sph_basis == B.basis_version && ds->f64_sph_nucl == ctx->nucleus.coord_version &&
-      ds->f64_sph_cutoff == cutoff)
-    return QMCKL_SUCCESS;
-  std::vector<F64Shell> sh((size_t)S);
-  for (int64_t m = 0; m < N; ++m)
-    for (int64_t s = B.nucleus_index[m]; s < B.nucleus_index[m] + B.nucleus_shell_num[m]; ++s) {
-      F64Shell& e = sh[(size_t)s];
-      const int l = B.shell_ang_mom[s];
-      const int64_t a0 = d.ao_index[s];
-      e.x = ctx->nucleus.coord[m];
-      e.y = ctx->nucleus.coord[m + N];
-      e.z = ctx->nucleus.coord[m + 2 * N];
-      e.r2max = shell_r2max(ctx, (int)s, (int)m, cutoff);
-      e.crange = cutoff * d.nucleus_range[m];
-      e.a0 = (int32_t)a0;
-      e.na = (int32_t)std::max<int64_t>(0, std::min<int64_t>((int64_t)(l + 1) * (l + 2) / 2, A - a0));
-      e.cb = d.shell_coef_start[s];
-      e.ce = d.shell_coef_start[s + 1];
-      e.l = l;
-      e.nucl = (int32_t)m;
-    }
-  qmckl_exit_code rc = ensure(context, ds->f64_sph, sizeof(F64Shell) * (size_t)S, fname);
-  if (rc != QMCKL_SUCCESS) return rc;
-  QB_CUDA(cudaMemcpy(ds->f64_sph.p, sh.data(), sizeof(F64Shell) * (size_t)S, cudaMemcpyHostToDevice), fname);
-  ds->f64_sph_basis = B.basis_version;
-  ds->f64_sph_nucl = ctx->nucleus.coord_version;
-  ds->f64_sph_cutoff = cutoff;
   return QMCKL_SUCCESS;
 }
 
@@ -1288,9 +1324,8 @@ qmckl_exit_code dev_provide_ao_hessian(qmckl_context context, double* host_out) 
     if (rc != QMCKL_SUCCESS) return rc;
     rc = ensure(context, ds->ao_hessian, bytes, "qmckl_provide_ao_basis_ao_hessian");
     if (rc != QMCKL_SUCCESS) return rc;
-    QB_CUDA(launch_ao_hessian(ds->T, P, (const double*)ds->coord.p, cutoff_of(ctx), ctx->precision <= 23,
-                              (double*)ds->ao_hessian.p, ds->stream),
-            "qmckl_provide_ao_basis_ao_hessian");
+    rc = run_ao_hessian(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_hessian.p);
+    if (rc != QMCKL_SUCCESS) return rc;
     ctx->ao_basis.ao_hessian_date = ctx->date;
   }
   return copy_out(context, ds, host_out, ds->ao_hessian.p, bytes, "qmckl_get_ao_basis_ao_hessian");
@@ -1429,9 +1464,8 @@ qmckl_exit_code dev_provide_mo_hessian(qmckl_context context, double* host_out) 
     if (cr != nullptr) {
       rc = ensure(context, ds->ao_masked, sizeof(double) * 12 * A * P, fname);
       if (rc != QMCKL_SUCCESS) return rc;
-      QB_CUDA(launch_ao_hessian(ds->T, P, (const double*)ds->coord.p, cutoff_of(ctx), ctx->precision <= 23,
-                                (double*)ds->ao_masked.p, ds->stream, cr),
-              fname);
+      rc = run_ao_hessian(context, ds, P, (const double*)ds->coord.p, (double*)ds->ao_masked.p, cr);
+      if (rc != QMCKL_SUCCESS) return rc;
       H = (const double*)ds->ao_masked.p;
     } else {
       rc = dev_provide_ao_hessian(context, nullptr);
@@ -1697,10 +1731,7 @@ qmckl_exit_code qmckl_b200_ao_hessian_device(qmckl_context context, const int64_
       device_entry(context, "qmckl_b200_ao_hessian_device", point_num, d_coord, d_ao_hessian, false);
   if (rc != QMCKL_SUCCESS) return rc;
   Context* ctx = ctx_of(context);
-  QB_CUDA(launch_ao_hessian(state(context)->T, point_num, d_coord, cutoff_of(ctx), ctx->precision <= 23, d_ao_hessian,
-                            state(context)->stream),
-          "qmckl_b200_ao_hessian_device");
-  return QMCKL_SUCCESS;
+  return run_ao_hessian(context, state(context), point_num, d_coord, d_ao_hessian);
 }
 
 // Adjoint of MO VGL.  With L = sum_{p,c,i} W[p][c][i] mo_vgl[p][c][i]:
@@ -1765,7 +1796,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_buf, buf_bytes, fname);
   if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_wp, sizeof(uint16_t) * 3 * 5 * chunk * ldw, fname);
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->adj_wt, sizeof(uint16_t) * 3 * 160 * ctiles * ldw, fname);
-  if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->order, order_bytes(chunk), fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->order, order_bytes(chunk), fname);
   if (rc == QMCKL_SUCCESS && points)
     rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 2), fname);
   if (rc == QMCKL_SUCCESS && ds->tc_err.p == nullptr) {
@@ -1794,7 +1825,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
     QB_CUDA(cudaMemcpy2DAsync(cc, sizeof(double) * n, d_coord + p0, sizeof(double) * P, sizeof(double) * n, 3,
                               cudaMemcpyDeviceToDevice, s), fname);
     int* perm = nullptr;
-    if (points && tiles > 1) {
+    if (tiles > 1) {
       perm = (int*)ds->order.p;
       QB_CUDA(point_order(cc, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(n), perm, s, n), fname);
     }
@@ -1802,7 +1833,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
                              points ? ds->adj_wt.p : nullptr, s),
             fname);
     if (d_grad_coef) {
-      QB_CUDA(launch_ao_vgl_pieces(ds->T, n, cc, cutoff, false, buf, lda, rows * lda, s), fname);
+      QB_CUDA(launch_ao_vgl_pieces(ds->T, ds->rows, n, cc, perm, cutoff, false, buf, lda, rows * lda, s), fname);
       QB_CUDA(tc_gemm_tn_split(buf, lda, rows * lda, A, ds->adj_wp.p, ldw, rows * ldw, (int)M, rows, kps,
                                (double*)ds->adj_part.p, err, s),
               fname);

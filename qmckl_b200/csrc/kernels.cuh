@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <vector>
 
 namespace qb {
 
@@ -82,13 +83,36 @@ __device__ __forceinline__ int pack_live_slots(const int32_t* __restrict__ slot_
 cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const double* coord,
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s,
                               const double* cusp_r = nullptr);
-// The same FP64 AO VGL stored as 3 bfloat16 pieces (split.cuh) of rows
-// p*5 + c: pieces[q * pstride + row * lda + ao] (lda, pstride multiples of 8).
-cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const double* coord, double cutoff,
-                                 bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s);
 cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const double* coord,
                                 double cutoff, bool dp_exp, double* ao_value, cudaStream_t s,
                                 const double* cusp_r = nullptr);
+// AO arrays through row images (ao_rows.cu).  The tables of its kernels: the
+// shell records, and for each array (0 Hessian, 1 bfloat16 pieces) segments of
+// ao_segment_width(array, ao_num) AOs with the shells [seg.x, seg.y) that have
+// AOs in each; run_shells[n]: the most shells that n segments in a row span.
+struct F64Shell;
+struct AoSegments {
+  const int2* seg;
+  int nseg, width;
+  std::vector<int> run_shells;
+};
+struct AoRowTables {
+  const F64Shell* sh;
+  AoSegments seg[2];
+};
+int ao_segment_width(int array, int64_t ao_num);
+// ao_hessian [3][point_num][4][ao]; `mixed`: FP32 exponentials where a r^2 <= 30.
+cudaError_t launch_ao_hessian(const DevTables& T, const AoRowTables& R, int64_t point_num, const double* coord,
+                              double cutoff, bool mixed, double* ao_hessian, cudaStream_t s,
+                              const double* cusp_r = nullptr);
+// The FP64 AO VGL (FP32 exponentials unless dp_exp) as 3 bfloat16 pieces
+// (split.cuh) of rows p*5 + c: pieces[q * pstride + row * lda + ao] (lda,
+// pstride multiples of 8, lda less than 8 past the AOs, 16-byte aligned; the
+// columns past the AOs are zeroed).  perm: the order in which the points are
+// taken (null: as they are; it decides the speed only).
+cudaError_t launch_ao_vgl_pieces(const DevTables& T, const AoRowTables& R, int64_t point_num, const double* coord,
+                                 const int* perm, double cutoff, bool dp_exp, void* pieces, int64_t lda, int64_t pstride,
+                                 cudaStream_t s);
 // Cusp adjustment (cusp.cu, org/qmckl_mo.org:2807-2860, 3099-3185,
 // 2629-2697): adds, for every nucleus closer to a point than its radius, the
 // cubic c0 + c1 r + c2 r^2 + c3 r^3 (prm [nucl][4][mo]) to the point's MO
@@ -185,10 +209,6 @@ cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord
 cudaError_t launch_add_transposed(const double* part, int splits, int64_t M, int64_t N, double* out, bool accumulate,
                                   cudaStream_t s);
 
-// Derivative kernels (adjoint.cu).  ao_hessian: [3][point_num][4][ao]
-// (coord [3][point_num]), `mixed` selects FP32 exponentials where a r^2 <= 30.
-cudaError_t launch_ao_hessian(const DevTables& T, int64_t point_num, const double* coord, double cutoff, bool mixed,
-                              double* ao_hessian, cudaStream_t s, const double* cusp_r = nullptr);
 // Orbital forces (adjoint.cu): which = 0 forces_mo_value, 1 forces_mo_g,
 // 2 forces_mo_l (from X = ao_vgl for 0, ao_hessian for 1 and 2, and
 // Ct = coefficient_t [ao][mo]), 3 forces_ao_value (from X = ao_vgl).
