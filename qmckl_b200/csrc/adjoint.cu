@@ -136,7 +136,8 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
   const bool in = qi < P;
   const int64_t pi = in ? (perm ? (int64_t)perm[qi] : qi) : 0;
   const double px = in ? coord[pi] : 0.0, py = in ? coord[pi + cstride] : 0.0, pz = in ? coord[pi + 2 * cstride] : 0.0;
-  const int n = adj.nlive[tile];
+  // with shells of l >= 4, T.shell_parts entries per shell share its AOs
+  const int n = adj.nlive[tile] * T.shell_parts;
   const int part = (int)blockIdx.y * NW + warp, parts = (int)gridDim.y * NW;
   const int e0 = (int)((int64_t)n * part / parts), e1 = (int)((int64_t)n * (part + 1) / parts);
   const F* gt = gc + (size_t)tile * kmax * LD + lane;
@@ -155,8 +156,10 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
     nq[0] = nq[1] = nq[2] = 0.0;
   };
   for (int e = e0; e < e1; ++e) {
-    const int2 le = adj.live[tile * T.shell_num + e];
+    const int2 le = adj.live[tile * T.shell_num + e / T.shell_parts];
     const F64Shell S = sh[le.x];
+    const int sp = e % T.shell_parts;
+    if (sp > 0 && S.l < 4) continue;
     if (S.nucl != nucl) {
       flush();
       nucl = S.nucl;
@@ -208,7 +211,8 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
     }
     if (any_l) {
       const F v[3] = {(F)R.v[0], (F)R.v[1], (F)R.v[2]}, R3[3] = {(F)a0, (F)a1, (F)a2};
-      for (int i = 0; i < S.na; ++i) {
+      const int i0 = S.l < 4 ? 0 : S.na * sp / T.shell_parts, i1 = S.l < 4 ? S.na : S.na * (sp + 1) / T.shell_parts;
+      for (int i = i0; i < i1; ++i) {
         F g[3], H[3][3], Tl[3];
         ao_derivs<F>(T.ao_code[S.a0 + i], (F)fac[i], v, R3, (F)R.lapR, (F)R.k3, g, H, Tl);
         const F* p = gr + i * LD;

@@ -1,5 +1,5 @@
 // Second and third derivatives of one AO, shared by the AO Hessian
-// (ao_rows.cu) and the adjoint (adjoint.cu).
+// (ao_hessian.cu) and the adjoint (adjoint.cu).
 #pragma once
 
 #include <cuda_runtime.h>

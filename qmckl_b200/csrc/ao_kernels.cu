@@ -1,4 +1,5 @@
-// AO kernels: FP64 AO VGL / AO value, the primitive and shell VGL getters.
+// AO kernels: FP64 AO VGL / AO value, the primitive and shell VGL getters, and
+// the mixed-precision AO VGL kernel that feeds the tensor-core MO contraction.
 //
 // Arithmetic follows the reference's production kernel
 // qmckl_compute_ao_vgl_hpc_gaussian (org/qmckl_ao.org:8601-8973):
@@ -17,9 +18,12 @@
 // radial VGL of the block's shells into shared memory, then sweep the block's
 // contiguous AO range with consecutive lanes on consecutive AOs, so every
 // store of ao_vgl[point][comp][k] is a 256-byte coalesced row segment.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "split.cuh"
 
 namespace qb {
 
@@ -134,33 +138,37 @@ __device__ __forceinline__ void stage_block(const DevTables& T, WarpSmem& sm, co
   __syncwarp();
 }
 
-// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1).
-template <int COMPS>
+// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1), a warp per (point,
+// gridDim.y'th of the nucleus blocks).  SPLIT: each value
+// stored as 3 bfloat16 pieces (split.cuh) at pieces[q * pstride + row * lda
+// + ao], rows p * COMPS + c, instead of FP64 in `out`.
+template <int COMPS, bool SPLIT = false>
 __global__ void __launch_bounds__(kWarps * 32)
 ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord,
               const double cutoff, const bool dp_exp, double* __restrict__ out,
-              const double* __restrict__ cusp_r) {
+              uint16_t* __restrict__ pieces = nullptr, const int64_t lda = 0, const int64_t pstride = 0,
+              const double* __restrict__ cusp_r = nullptr) {
   __shared__ WarpSmem smem[kWarps];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   WarpSmem& sm = smem[warp];
   const int64_t A = T.ao_num;
   const int64_t stride = (int64_t)gridDim.x * kWarps;
-  // one warp per point, through its nucleus blocks in order: the point's
-  // rows are written in sequence (faster than spreading a point's blocks
-  // over warps: 2.9 against 3.1 ms on the config-1 molecule)
+  const int b0 = (int)((int64_t)T.nblock * blockIdx.y / gridDim.y);
+  const int b1 = (int)((int64_t)T.nblock * (blockIdx.y + 1) / gridDim.y);
   for (int64_t p = (int64_t)blockIdx.x * kWarps + warp; p < point_num; p += stride)
-  for (int b = 0; b < T.nblock; ++b) {
+  for (int b = b0; b < b1; ++b) {
     const int4 blk = T.block[b];
     const int2 slots = T.block_slots[b];
     const double px = coord[p], py = coord[p + point_num], pz = coord[p + 2 * point_num];
     stage_block<COMPS>(T, sm, blk, slots, px, py, pz, cutoff, dp_exp, lane);
     double* __restrict__ row = out + p * COMPS * A;
-    // The lanes' 32-AO groups start on a 128-byte boundary of the output: a
-    // group that straddles it writes partial sectors and ~20% fewer bytes per
-    // second (2.87 ms against 2.37 for the 13 GB of the config-1 molecule's AO
-    // VGL, stores alone).
-    const int sh = (int)((reinterpret_cast<uintptr_t>(row + blk.z) >> 3) & 15);
+    // The lanes' 32-AO groups start on a 128-byte boundary of the output
+    // (64 bytes of the bfloat16 pieces): a group that straddles it writes
+    // partial sectors and ~20% fewer bytes per second (2.87 ms against 2.37
+    // for the 13 GB of the config-1 molecule's AO VGL, stores alone).
+    const int sh = SPLIT ? (int)((reinterpret_cast<uintptr_t>(pieces + p * COMPS * lda + blk.z) >> 1) & 31)
+                         : (int)((reinterpret_cast<uintptr_t>(row + blk.z) >> 3) & 15);
     for (int k = blk.z - sh + lane; k < blk.w; k += 32) {
       if (k < blk.z) continue;
       const int code = T.ao_code[k];
@@ -202,13 +210,25 @@ ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restri
           }
         }
       }
-      // streaming stores: the array is written once and not read back here
-      __stcs(&row[k], v[0]);
-      if (COMPS == 5) {
-        __stcs(&row[A + k], v[1]);
-        __stcs(&row[2 * A + k], v[2]);
-        __stcs(&row[3 * A + k], v[3]);
-        __stcs(&row[4 * A + k], v[4]);
+      if constexpr (SPLIT) {
+#pragma unroll
+        for (int c = 0; c < COMPS; ++c) {
+          uint16_t pc[3];
+          split3_bf16(v[c], pc);
+          uint16_t* dst = pieces + (p * COMPS + c) * lda + k;
+          dst[0] = pc[0];
+          dst[pstride] = pc[1];
+          dst[2 * pstride] = pc[2];
+        }
+      } else {
+        // streaming stores: the array is written once and not read back here
+        __stcs(&row[k], v[0]);
+        if (COMPS == 5) {
+          __stcs(&row[A + k], v[1]);
+          __stcs(&row[2 * A + k], v[2]);
+          __stcs(&row[3 * A + k], v[3]);
+          __stcs(&row[4 * A + k], v[4]);
+        }
       }
     }
     __syncwarp();
@@ -288,13 +308,15 @@ __global__ void shell_vgl_kernel(const DevTables T, const int64_t point_num,
   }
 }
 
-int grid_for(int64_t items_per_warp_unit) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t want = (items_per_warp_unit + kWarps - 1) / kWarps;
-  const int64_t cap = (int64_t)sms * 8;
-  return (int)(want < cap ? (want > 0 ? want : 1) : cap);
+// A warp per point, through its nucleus blocks in order: the point's rows are
+// written in sequence (2.9 against 3.1 ms with a point's blocks spread over
+// warps, on the config-1 molecule).  Points too few to fill the chip (8 CTAs
+// per SM) have their blocks spread all the same: 100 points x 5000 AOs, the
+// pieces, 15 us against 169 us.
+dim3 ao_grid(const DevTables& T, int64_t points) {
+  const int64_t want = (points + kWarps - 1) / kWarps, cap = 148 * 8;
+  const int64_t split = std::min<int64_t>(std::max(1, T.nblock), std::max<int64_t>(1, cap / want));
+  return dim3((unsigned)std::min(want, cap), (unsigned)split);
 }
 
 }  // namespace
@@ -302,8 +324,17 @@ int grid_for(int64_t items_per_warp_unit) {
 cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const double* coord,
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
-  const int grid = grid_for(point_num);   // one warp per point
-  ao_f64_kernel<5><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_vgl, cusp_r);
+  ao_f64_kernel<5><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_vgl, nullptr, 0, 0, cusp_r);
+  count_launch();
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const double* coord, double cutoff,
+                                 bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s) {
+  if (point_num <= 0) return cudaSuccess;
+  if (lda < T.ao_num || lda % 8 != 0 || pstride % 8 != 0) return cudaErrorInvalidValue;
+  ao_f64_kernel<5, true><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, nullptr,
+                                                      (uint16_t*)pieces, lda, pstride);
   count_launch();
   return cudaGetLastError();
 }
@@ -311,8 +342,8 @@ cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const doubl
 cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const double* coord,
                                 double cutoff, bool dp_exp, double* ao_value, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
-  const int grid = grid_for(point_num);   // one warp per point
-  ao_f64_kernel<1><<<grid, kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_value, cusp_r);
+  ao_f64_kernel<1><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_value, nullptr, 0, 0,
+                                                cusp_r);
   count_launch();
   return cudaGetLastError();
 }

@@ -376,7 +376,7 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
-  AoRowTables rows{};   // in f64_sph: the shell records and the segments of the AO array kernels
+  AoSegments hess{};   // in f64_sph: the shell records and the segments of the AO Hessian
 };
 
 namespace {
@@ -592,6 +592,7 @@ qmckl_exit_code upload_tables(qmckl_context context, DeviceState* ds) {
   T.shell_num = (int32_t)S;
   T.prim_num = (int32_t)Pn;
   T.ao_num = (int32_t)A;
+  T.shell_parts = *std::max_element(B.shell_ang_mom.begin(), B.shell_ang_mom.end()) >= 4 ? 4 : 1;
   T.nblock = (int32_t)blocks.size();
   T.nslot = (int32_t)slot_nuc.size();
   T.nucleus_range = (const double*)(base + o_range);
@@ -716,8 +717,8 @@ qmckl_exit_code copy_out(qmckl_context context, DeviceState* ds, double* host, c
 
 DeviceState* state(qmckl_context context) { return ctx_of(context)->extra; }
 
-// The per-shell records of the FP64 tile and AO array kernels (basis order),
-// and the AO array kernels' segments.
+// The per-shell records of the FP64 tile kernels and of the AO Hessian (basis
+// order), and the latter's segments.
 qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
   const char* fname = "qmckl_b200_mo_fp64";
   Context* ctx = ctx_of(context);
@@ -746,33 +747,27 @@ qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
       e.l = l;
       e.nucl = (int32_t)m;
     }
+  AoSegments g{};
+  g.width = hessian_segment_width(A);
   std::vector<int2> segs;
-  size_t at[2];
-  for (int m = 0; m < 2; ++m) {
-    AoSegments& g = ds->rows.seg[m];
-    const int64_t w = g.width = ao_segment_width(m, A);
-    g.nseg = (int)((A + w - 1) / w);
-    at[m] = segs.size();
-    int64_t s0 = 0;
-    for (int64_t a0 = 0; a0 < A; a0 += w) {
-      while (s0 < S && sh[(size_t)s0].a0 + sh[(size_t)s0].na <= a0) ++s0;
-      int64_t s1 = s0;
-      while (s1 < S && sh[(size_t)s1].a0 < a0 + w) ++s1;
-      segs.push_back(make_int2((int)s0, (int)s1));
-    }
-    g.run_shells.assign((size_t)g.nseg + 1, 0);
-    for (int n = 1; n <= g.nseg; ++n)
-      for (int i = 0; i + n <= g.nseg; ++i)
-        g.run_shells[n] = std::max(g.run_shells[n], segs[at[m] + i + n - 1].y - segs[at[m] + i].x);
+  int64_t s0 = 0;
+  for (int64_t a0 = 0; a0 < A; a0 += g.width) {
+    while (s0 < S && sh[(size_t)s0].a0 + sh[(size_t)s0].na <= a0) ++s0;
+    int64_t s1 = s0;
+    while (s1 < S && sh[(size_t)s1].a0 < a0 + g.width) ++s1;
+    segs.push_back(make_int2((int)s0, (int)s1));
+    g.max_shells = std::max(g.max_shells, (int)(s1 - s0));
   }
+  g.nseg = (int)segs.size();
   const size_t sb = sizeof(F64Shell) * (size_t)S;
   qmckl_exit_code rc = ensure(context, ds->f64_sph, sb + sizeof(int2) * segs.size(), fname);
   if (rc != QMCKL_SUCCESS) return rc;
   QB_CUDA(cudaMemcpy(ds->f64_sph.p, sh.data(), sb, cudaMemcpyHostToDevice), fname);
   QB_CUDA(cudaMemcpy((uint8_t*)ds->f64_sph.p + sb, segs.data(), sizeof(int2) * segs.size(), cudaMemcpyHostToDevice),
           fname);
-  ds->rows.sh = (const F64Shell*)ds->f64_sph.p;
-  for (int m = 0; m < 2; ++m) ds->rows.seg[m].seg = (const int2*)((uint8_t*)ds->f64_sph.p + sb) + at[m];
+  g.sh = (const F64Shell*)ds->f64_sph.p;
+  g.seg = (const int2*)((uint8_t*)ds->f64_sph.p + sb);
+  ds->hess = g;
   ds->f64_sph_basis = B.basis_version;
   ds->f64_sph_nucl = ctx->nucleus.coord_version;
   ds->f64_sph_cutoff = cutoff;
@@ -822,7 +817,7 @@ qmckl_exit_code run_ao_hessian(qmckl_context context, DeviceState* ds, int64_t P
   Context* ctx = ctx_of(context);
   qmckl_exit_code rc = sync_f64_shells(context, ds);
   if (rc != QMCKL_SUCCESS) return rc;
-  QB_CUDA(launch_ao_hessian(ds->T, ds->rows, P, coord, cutoff_of(ctx), ctx->precision <= 23, out, ds->stream, cusp_r),
+  QB_CUDA(launch_ao_hessian(ds->T, ds->hess, P, coord, cutoff_of(ctx), ctx->precision <= 23, out, ds->stream, cusp_r),
           "qmckl_b200_ao_hessian");
   return QMCKL_SUCCESS;
 }
@@ -1792,11 +1787,11 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   const int64_t ctiles = (chunk + 31) / 32;
   const size_t buf_bytes = std::max<size_t>((size_t)(30 * lda) * (size_t)chunk, sizeof(float) * 160 * (size_t)A * (size_t)ctiles);
   const size_t b_live = (sizeof(int2) * (size_t)S * (size_t)ctiles + 15) / 16 * 16;
-  rc = ensure(context, ds->adj_coord, sizeof(double) * 3 * chunk, fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->adj_buf, buf_bytes, fname);
+  rc = ensure(context, ds->adj_buf, buf_bytes, fname);
+  if (rc == QMCKL_SUCCESS && nchunks > 1) rc = ensure(context, ds->adj_coord, sizeof(double) * 3 * chunk, fname);
   if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_wp, sizeof(uint16_t) * 3 * 5 * chunk * ldw, fname);
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->adj_wt, sizeof(uint16_t) * 3 * 160 * ctiles * ldw, fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->order, order_bytes(chunk), fname);
+  if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->order, order_bytes(chunk), fname);
   if (rc == QMCKL_SUCCESS && points)
     rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 2), fname);
   if (rc == QMCKL_SUCCESS && ds->tc_err.p == nullptr) {
@@ -1806,7 +1801,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_part, sizeof(double) * splits * A * M, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   void* buf = ds->adj_buf.p;
-  double* cc = (double*)ds->adj_coord.p;
+  const double* cc = nchunks > 1 ? (const double*)ds->adj_coord.p : d_coord;   // the chunk's coordinates
   F64Tiles t{};
   t.pts = 32;
   t.adj.live = (int2*)ds->f64_tiles.p;
@@ -1822,10 +1817,12 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   for (int64_t p0 = 0; p0 < P; p0 += chunk) {
     const int64_t n = std::min<int64_t>(chunk, P - p0), rows = 5 * n, tiles = (n + 31) / 32;
     const double* w = d_weight + p0 * 5 * M;
-    QB_CUDA(cudaMemcpy2DAsync(cc, sizeof(double) * n, d_coord + p0, sizeof(double) * P, sizeof(double) * n, 3,
-                              cudaMemcpyDeviceToDevice, s), fname);
+    if (nchunks > 1)
+      QB_CUDA(cudaMemcpy2DAsync(ds->adj_coord.p, sizeof(double) * n, d_coord + p0, sizeof(double) * P,
+                                sizeof(double) * n, 3, cudaMemcpyDeviceToDevice, s),
+              fname);
     int* perm = nullptr;
-    if (tiles > 1) {
+    if (points && tiles > 1) {
       perm = (int*)ds->order.p;
       QB_CUDA(point_order(cc, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(n), perm, s, n), fname);
     }
@@ -1833,7 +1830,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
                              points ? ds->adj_wt.p : nullptr, s),
             fname);
     if (d_grad_coef) {
-      QB_CUDA(launch_ao_vgl_pieces(ds->T, ds->rows, n, cc, perm, cutoff, false, buf, lda, rows * lda, s), fname);
+      QB_CUDA(launch_ao_vgl_pieces(ds->T, n, cc, cutoff, false, buf, lda, rows * lda, s), fname);
       QB_CUDA(tc_gemm_tn_split(buf, lda, rows * lda, A, ds->adj_wp.p, ldw, rows * ldw, (int)M, rows, kps,
                                (double*)ds->adj_part.p, err, s),
               fname);

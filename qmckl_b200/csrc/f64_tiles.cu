@@ -17,12 +17,108 @@
 // distinct bank groups when they are copied to shared memory as they are).
 #include <algorithm>
 
-#include "f64_tile_dev.cuh"
+#include "kernels.cuh"
 
 namespace qb {
 namespace {
 
-constexpr int kPlanThreads = 256;
+constexpr double kShiftT = 1.e-20;
+constexpr int kAoThreads = 256;
+
+__device__ __forceinline__ double ipow_t(double x, int n) {
+  double r = 1.0;
+  for (int i = 0; i < n; ++i) r = r * x;
+  return r;
+}
+
+// Radial VGL of one shell at one point (org/qmckl_ao.org:8798-8828); the
+// arithmetic of ao_kernels.cu shell_radial.
+template <int COMPS>
+__device__ __forceinline__ void radial_t(const double2* __restrict__ prim, int cb, int ce, double x, double y, double z,
+                                         double r2, double cutoff, bool dp_exp, double (&s)[5]) {
+#pragma unroll
+  for (int c = 0; c < 5; ++c) s[c] = 0.0;
+  for (int j = cb; j < ce; ++j) {
+    const double2 ac = prim[j];
+    const double ar2 = ac.x * r2;
+    if (ar2 > cutoff) break;   // primitives are sorted by exponent
+    const double e = dp_exp ? exp(-ar2) : (double)expf(-(float)ar2);
+    s[0] += ac.y * e;
+    if (COMPS == 5) {
+      double f = ac.x * e;
+      f = -f - f;
+      s[1] += ac.y * (f * x);
+      s[2] += ac.y * (f * y);
+      s[3] += ac.y * (f * z);
+      s[4] += ac.y * (f * (3.0 - 2.0 * ar2));
+    }
+  }
+}
+
+// The product rule of one AO and its stores: v = P R with P's derivatives.
+template <int COMPS, int TP>
+__device__ __forceinline__ void put_ao(double* __restrict__ o, bool on, double f, const double (&s)[5], double P0,
+                                       double P1, double P2, double P3, double P4) {
+  o[0] = on ? P0 * s[0] * f : 0.0;
+  if (COMPS == 5) {
+    o[TP] = on ? (P1 * s[0] + P0 * s[1]) * f : 0.0;
+    o[2 * TP] = on ? (P2 * s[0] + P0 * s[2]) * f : 0.0;
+    o[3 * TP] = on ? (P3 * s[0] + P0 * s[3]) * f : 0.0;
+    o[4 * TP] = on ? (P4 * s[0] + P0 * s[4] + 2.0 * (P1 * s[1] + P2 * s[2] + P3 * s[3])) * f : 0.0;
+  }
+}
+
+// All AOs of a shell of angular momentum L <= 3 at the warp's 32 points: the
+// cartesian exponents are compile-time constants.
+template <int COMPS, int TP, int L>
+__device__ __forceinline__ void emit_shell(double* __restrict__ o, int64_t ld, bool on, const double* __restrict__ fac,
+                                           const double (&s)[5], double x, double y, double z) {
+  const double xp[4] = {1.0, x, x * x, x * (x * x)}, yp[4] = {1.0, y, y * y, y * (y * y)},
+               zp[4] = {1.0, z, z * z, z * (z * z)};
+  int i = 0;
+#pragma unroll
+  for (int a = L; a >= 0; --a)
+#pragma unroll
+    for (int b = L - a; b >= 0; --b) {
+      const int c = L - a - b;
+      const double yz = yp[b] * zp[c], xz = xp[a] * zp[c], xy = xp[a] * yp[b];
+      const double P0 = xp[a] * yz + (L >= 1 ? kShiftT : 0.0);
+      const double P1 = a ? (double)a * xp[a > 0 ? a - 1 : 0] * yz : 0.0;
+      const double P2 = b ? (double)b * yp[b > 0 ? b - 1 : 0] * xz : 0.0;
+      const double P3 = c ? (double)c * zp[c > 0 ? c - 1 : 0] * xy : 0.0;
+      double P4 = 0.0;
+      if (a >= 2) P4 += (double)(a * (a - 1)) * xp[a >= 2 ? a - 2 : 0] * yz;
+      if (b >= 2) P4 += (double)(b * (b - 1)) * yp[b >= 2 ? b - 2 : 0] * xz;
+      if (c >= 2) P4 += (double)(c * (c - 1)) * zp[c >= 2 ? c - 2 : 0] * xy;
+      put_ao<COMPS, TP>(o + i * ld, on, fac[i], s, P0, P1, P2, P3, P4);
+      ++i;
+    }
+}
+
+// The same for L >= 4 (org/qmckl_ao.org:6624-6914), its AOs [i0, i1).
+template <int COMPS, int TP>
+__device__ __forceinline__ void emit_shell_any(double* __restrict__ o, int64_t ld, bool on, int L, int i0, int i1,
+                                               const double* __restrict__ fac, const double (&s)[5], double x, double y,
+                                               double z) {
+  int i = 0;
+  for (int a = L; a >= 0; --a)
+    for (int b = L - a; b >= 0 && i < i1; --b, ++i) {
+      if (i < i0) continue;
+      const int c = L - a - b;
+      const double pa = ipow_t(x, a), pb = ipow_t(y, b), pc = ipow_t(z, c);
+      const double pa1 = a >= 1 ? ipow_t(x, a - 1) : 1.0, pb1 = b >= 1 ? ipow_t(y, b - 1) : 1.0,
+                   pc1 = c >= 1 ? ipow_t(z, c - 1) : 1.0;
+      const double pa2 = a >= 2 ? ipow_t(x, a - 2) : 1.0, pb2 = b >= 2 ? ipow_t(y, b - 2) : 1.0,
+                   pc2 = c >= 2 ? ipow_t(z, c - 2) : 1.0;
+      double xy = pa * pb, yz = pb * pc, xz = pa * pc;
+      const double P0 = xy * pc + kShiftT;
+      xy *= (double)c;
+      xz *= (double)b;
+      yz *= (double)a;
+      put_ao<COMPS, TP>(o + i * ld, on, fac[i], s, P0, pa1 * yz, pb1 * xz, pc1 * xy,
+                        (double)(a - 1) * pa2 * yz + (double)(b - 1) * pb2 * xz + (double)(c - 1) * pc2 * xy);
+    }
+}
 
 // AO production of a tile (blockIdx.x) by gridDim.y CTAs.  Each CTA finds the
 // tile's live shells, numbers them by a scan, and its warps then claim (live
@@ -34,8 +130,8 @@ constexpr int kPlanThreads = 256;
 // every point and took 0.73 ms for the 3.3 GB array).  CTA 0 of the tile
 // writes its AO list.
 // Scratch: dynamic shared memory of 2 * shell_num ints.
-template <int COMPS, int TP>
-__global__ void __launch_bounds__(kPlanThreads)
+template <int COMPS, int TP, int PARTS>
+__global__ void __launch_bounds__(kAoThreads, 4)
 ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t cstride, const int* __restrict__ perm,
                 const int64_t tile0, const int shell_num, const F64Shell* __restrict__ sh,
                 const double2* __restrict__ prim, const double* __restrict__ factor, const double cutoff,
@@ -45,26 +141,152 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   constexpr int LD = COMPS * TP + 4;
   static_assert(TP % 32 == 0 && G <= 4, "a tile is 1 to 4 warps of points");
   __shared__ double spts[3 * TP];
-  __shared__ TilePlan<TP> pl;
-  __shared__ int claim;
+  __shared__ unsigned long long wsum[kAoThreads / 32];
+  __shared__ double box[G][6];
+  __shared__ bool isnan_g[G];
+  __shared__ int claim, nopen;
   extern __shared__ int sbuf[];
-  int* live = sbuf;
-  int* lpos = sbuf + shell_num;
-  const int tid = threadIdx.x, lane = tid & 31;
+  int* live = sbuf;               // [count] shell | group mask << 24
+  int* lpos = sbuf + shell_num;   // [count] first list position
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t tile = blockIdx.x;
   const int64_t p0 = (tile0 + tile) * TP;
   const int np = (int)(P - p0 < TP ? P - p0 : TP);
-  for (int t = tid; t < 3 * TP; t += kPlanThreads) {
+  for (int t = tid; t < 3 * TP; t += kAoThreads) {
     const int d = t / TP, i = t - d * TP;
     spts[t] = i < np ? coord[(perm ? (int64_t)perm[p0 + i] : p0 + i) + d * cstride] : 0.0;
   }
-  if (tid == 0) claim = 0;
+  if (tid == 0) claim = nopen = 0;
   __syncthreads();
-  const int2 n = tile_live_shells<TP, kPlanThreads>(pl, spts, np, sh, shell_num, live, lpos);
-  const int nlive = n.x, nao = n.y;
+  if (warp < G) {   // bounding box of each 32 points (NaN coordinates left out)
+    const int i = max(0, min(32 * warp + lane, np - 1));
+    bool bad = false;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      double lo = spts[d * TP + i], hi = lo;
+      bad = bad || isnan(lo);
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      }
+      if (lane == 0) {
+        box[warp][d] = lo;
+        box[warp][3 + d] = hi;
+      }
+    }
+    bad = __any_sync(0xffffffffu, bad);
+    if (lane == 0) isnan_g[warp] = bad;
+  }
+  __syncthreads();
+  // Live shells, one group of 32 points at a time: a shell beyond the group's
+  // bounding box is dead, one that holds the group's first point is live, and
+  // the rest (a fifth of them on the molecules of the tests), packed, are tested
+  // point by point, a thread per shell.
+  for (int s = tid; s < shell_num; s += kAoThreads) live[s] = 0;
+#pragma unroll 1
+  for (int g = 0; g < G; ++g) {
+    if (32 * g >= np) break;
+    for (int s = tid; s < shell_num; s += kAoThreads) {
+      const F64Shell S = sh[s];
+      if (S.r2max < 0.0) continue;   // no primitives
+      // the margin covers the rounding of both distances
+      const double bx = fmax(fmax(box[g][0] - S.x, S.x - box[g][3]), 0.0),
+                   by = fmax(fmax(box[g][1] - S.y, S.y - box[g][4]), 0.0),
+                   bz = fmax(fmax(box[g][2] - S.z, S.z - box[g][5]), 0.0);
+      if (!isnan_g[g] && (bx * bx + by * by + bz * bz) * (1.0 - 1e-9) > S.r2max) continue;
+      const double x = spts[32 * g] - S.x, y = spts[TP + 32 * g] - S.y, z = spts[2 * TP + 32 * g] - S.z;
+      if (x * x + y * y + z * z <= S.r2max)
+        live[s] |= 1 << g;
+      else
+        lpos[atomicAdd(&nopen, 1)] = s;
+    }
+    __syncthreads();
+    const int n = nopen, e = min(np, 32 * g + 32);
+    for (int q = tid; q < n; q += kAoThreads) {
+      const int s = lpos[q];
+      const F64Shell S = sh[s];
+      for (int i = 32 * g; i < e; i += 4) {
+        bool in = false;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const int j = min(i + h, e - 1);
+          const double x = spts[j] - S.x, y = spts[TP + j] - S.y, z = spts[2 * TP + j] - S.z;
+          // a NaN distance counts as inside: the AO is then a NaN, not a zero
+          in = in || !(x * x + y * y + z * z > S.r2max);
+        }
+        if (in) {
+          live[s] |= 1 << g;
+          break;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0) nopen = 0;
+    __syncthreads();
+  }
+  // number them: thread tid owns shells [tid * per, (tid + 1) * per); the scan
+  // counts AOs in the low and shells in the high half
+  const int per = (shell_num + kAoThreads - 1) / kAoThreads;
+  const int s0 = min(shell_num, tid * per), s1 = min(shell_num, s0 + per);
+  unsigned long long local = 0ull;
+  for (int s = s0; s < s1; ++s)
+    if (live[s]) local += (1ull << 32) | (unsigned int)sh[s].na;
+  unsigned long long incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) wsum[warp] = incl;
+  __syncthreads();
+  unsigned long long base = 0ull, total = 0ull;
+  for (int w = 0; w < kAoThreads / 32; ++w) {
+    if (w < warp) base += wsum[w];
+    total += wsum[w];
+  }
+  const int nlive = (int)(total >> 32), nao = (int)(total & 0xffffffffull);
+  base += incl - local;
+  // compact in place: a thread's live shells move to smaller indices, so the
+  // masks are read into registers before anyone writes
+  int mk[4];
+  const bool few = per <= 4;
+  if (few) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) mk[q] = s0 + q < s1 ? live[s0 + q] : 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (mk[q]) {
+        const int at = (int)(base >> 32), k = (int)(base & 0xffffffffull), s = s0 + q;
+        live[at] = s | (mk[q] << 24);
+        lpos[at] = k;
+        base += (1ull << 32) | (unsigned int)sh[s].na;
+      }
+  } else {   // many shells: through the position array, then one more pass
+    for (int s = s0; s < s1; ++s) lpos[s] = live[s];
+    __syncthreads();
+    const unsigned long long b0 = base;
+    for (int s = s0; s < s1; ++s)
+      if (lpos[s]) {
+        live[(int)(base >> 32)] = s | (lpos[s] << 24);
+        base += (1ull << 32);
+      }
+    __syncthreads();
+    unsigned long long b = b0;
+    int na_prev = 0;
+    const int n_mine = (int)(base >> 32) - (int)(b0 >> 32);
+    for (int q = 0; q < n_mine; ++q) {
+      const int at = (int)(b0 >> 32) + q;
+      b += (unsigned int)na_prev;
+      na_prev = sh[live[at] & 0xffffff].na;
+      lpos[at] = (int)(b & 0xffffffffull);
+    }
+  }
+  __syncthreads();
   if (blockIdx.y == 0) {
     int* kl = klist + tile * kmax;
-    for (int q = tid; q < nlive; q += kPlanThreads) {
+    for (int q = tid; q < nlive; q += kAoThreads) {
       const F64Shell S = sh[live[q] & 0xffffff];
       const int k = lpos[q];
       for (int i = 0; i < S.na; ++i) kl[k + i] = S.a0 + i;
@@ -81,15 +303,21 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   }
   if (ac == nullptr) return;   // the lists only
   double* __restrict__ act = ac + (size_t)tile * kmax * LD;
-  const int units = nlive * G;
+  // Shells of l >= 4 are split over PARTS units, which form the radial part
+  // again: with a unit each, their up to 36 AOs are the tile's critical path
+  // (34 us, 18 split, on 100 points of a 5-atom molecule with l = 7).
+  const int units = nlive * G * PARTS;
   for (;;) {
     int u = 0;
     if (lane == 0) u = atomicAdd(&claim, 1);
     u = __shfl_sync(0xffffffffu, u, 0) * (int)gridDim.y + (int)blockIdx.y;
     if (u >= units) break;
+    const int part = u % PARTS;
+    u /= PARTS;
     const int q = G == 1 ? u : u / G, g = G == 1 ? 0 : u % G;
     const int e = live[q];
     const F64Shell S = sh[e & 0xffffff];
+    if (part > 0 && S.l < 4) continue;
     const int i = 32 * g + lane;
     double* o = act + (size_t)lpos[q] * LD + i;
     const double x = spts[i] - S.x, y = spts[TP + i] - S.y, z = spts[2 * TP + i] - S.z;
@@ -101,16 +329,14 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
       on = s[0] != 0.0 && !cusp_masked(cusp_r, S.l, S.nucl, r2, COMPS == 1);
     }
     const double* fac = factor + S.a0;
-    auto put = [&](int k, const double (&v)[COMPS]) {
-#pragma unroll
-      for (int c = 0; c < COMPS; ++c) o[k * LD + c * TP] = v[c];
-    };
     switch (S.l) {
-      case 0: emit_shell<COMPS, 0>(put, on, fac, s, x, y, z); break;
-      case 1: emit_shell<COMPS, 1>(put, on, fac, s, x, y, z); break;
-      case 2: emit_shell<COMPS, 2>(put, on, fac, s, x, y, z); break;
-      case 3: emit_shell<COMPS, 3>(put, on, fac, s, x, y, z); break;
-      default: emit_shell_any<COMPS>(put, on, S.l, S.na, fac, s, x, y, z);
+      case 0: emit_shell<COMPS, TP, 0>(o, LD, on, fac, s, x, y, z); break;
+      case 1: emit_shell<COMPS, TP, 1>(o, LD, on, fac, s, x, y, z); break;
+      case 2: emit_shell<COMPS, TP, 2>(o, LD, on, fac, s, x, y, z); break;
+      case 3: emit_shell<COMPS, TP, 3>(o, LD, on, fac, s, x, y, z); break;
+      default:
+        emit_shell_any<COMPS, TP>(o, LD, on, S.l, S.na * part / PARTS, S.na * (part + 1) / PARTS, fac, s, x, y,
+                                  z);
     }
   }
 }
@@ -553,15 +779,19 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
   if (!(comps == 5 && t.pts == 32) && !(comps == 1 && (t.pts == 32 || t.pts == 128))) return cudaErrorInvalidValue;
   const size_t sm = sizeof(int) * 2 * (size_t)T.shell_num;
   if (sm > 200 * 1024) return cudaErrorInvalidValue;
-  auto kern = comps == 5 ? ao_tiles_kernel<5, 32> : (t.pts == 32 ? ao_tiles_kernel<1, 32> : ao_tiles_kernel<1, 128>);
+  auto kern = T.shell_parts > 1
+                  ? (comps == 5 ? ao_tiles_kernel<5, 32, 4>
+                                : (t.pts == 32 ? ao_tiles_kernel<1, 32, 4> : ao_tiles_kernel<1, 128, 4>))
+                  : (comps == 5 ? ao_tiles_kernel<5, 32, 1>
+                                : (t.pts == 32 ? ao_tiles_kernel<1, 32, 1> : ao_tiles_kernel<1, 128, 1>));
   cudaError_t e =
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1));
   if (e != cudaSuccess) return e;
   // few tiles: several CTAs share one, so that its shells are spread over SMs
   const int parts = t.ac == nullptr ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
-  kern<<<dim3((unsigned)ntiles, (unsigned)parts), kPlanThreads, sm, s>>>(
-      P, coord, cstride, perm, tile0, T.shell_num, sh, T.coef_ac, T.ao_factor, cutoff, dp_exp, cusp_r, T.ao_num, t.ac,
-      t.klist, t.kcount, t.adj);
+  kern<<<dim3((unsigned)ntiles, (unsigned)parts), kAoThreads, sm, s>>>(
+      P, coord, cstride, perm, tile0, T.shell_num, sh, T.coef_ac, T.ao_factor, cutoff, dp_exp, cusp_r, T.ao_num,
+      t.ac, t.klist, t.kcount, t.adj);
   count_launch();
   return cudaGetLastError();
 }

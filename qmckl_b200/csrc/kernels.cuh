@@ -3,7 +3,6 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
-#include <vector>
 
 namespace qb {
 
@@ -21,6 +20,7 @@ constexpr int kBlockSlots = 64;
 // carries its slot, its block-local nucleus and its cartesian powers.
 struct DevTables {
   int32_t nucl_num, shell_num, prim_num, ao_num, nblock, nslot;
+  int32_t shell_parts;            // parts of a shell that separate warps take: 4 with shells of l >= 4, else 1
   const double* nucl_coord;       // [3][nucl]
   const double* nucleus_range;    // [nucl]
   const int32_t* nuc_prim_start;  // [nucl+1] into expo (sorted, de-duplicated per nucleus)
@@ -86,33 +86,24 @@ cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const doubl
 cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const double* coord,
                                 double cutoff, bool dp_exp, double* ao_value, cudaStream_t s,
                                 const double* cusp_r = nullptr);
-// AO arrays through row images (ao_rows.cu).  The tables of its kernels: the
-// shell records, and for each array (0 Hessian, 1 bfloat16 pieces) segments of
-// ao_segment_width(array, ao_num) AOs with the shells [seg.x, seg.y) that have
-// AOs in each; run_shells[n]: the most shells that n segments in a row span.
+// The same FP64 AO VGL stored as 3 bfloat16 pieces (split.cuh) of rows
+// p*5 + c: pieces[q * pstride + row * lda + ao] (lda, pstride multiples of 8).
+cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const double* coord, double cutoff,
+                                 bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s);
+// AO Hessian (ao_hessian.cu): the shell records and segments of `width` =
+// hessian_segment_width(ao_num) AOs, the shells [seg.x, seg.y) with AOs in
+// each; at most max_shells of them.
 struct F64Shell;
 struct AoSegments {
-  const int2* seg;
-  int nseg, width;
-  std::vector<int> run_shells;
-};
-struct AoRowTables {
   const F64Shell* sh;
-  AoSegments seg[2];
+  const int2* seg;
+  int nseg, width, max_shells;
 };
-int ao_segment_width(int array, int64_t ao_num);
+int hessian_segment_width(int64_t ao_num);
 // ao_hessian [3][point_num][4][ao]; `mixed`: FP32 exponentials where a r^2 <= 30.
-cudaError_t launch_ao_hessian(const DevTables& T, const AoRowTables& R, int64_t point_num, const double* coord,
+cudaError_t launch_ao_hessian(const DevTables& T, const AoSegments& g, int64_t point_num, const double* coord,
                               double cutoff, bool mixed, double* ao_hessian, cudaStream_t s,
                               const double* cusp_r = nullptr);
-// The FP64 AO VGL (FP32 exponentials unless dp_exp) as 3 bfloat16 pieces
-// (split.cuh) of rows p*5 + c: pieces[q * pstride + row * lda + ao] (lda,
-// pstride multiples of 8, lda less than 8 past the AOs, 16-byte aligned; the
-// columns past the AOs are zeroed).  perm: the order in which the points are
-// taken (null: as they are; it decides the speed only).
-cudaError_t launch_ao_vgl_pieces(const DevTables& T, const AoRowTables& R, int64_t point_num, const double* coord,
-                                 const int* perm, double cutoff, bool dp_exp, void* pieces, int64_t lda, int64_t pstride,
-                                 cudaStream_t s);
 // Cusp adjustment (cusp.cu, org/qmckl_mo.org:2807-2860, 3099-3185,
 // 2629-2697): adds, for every nucleus closer to a point than its radius, the
 // cubic c0 + c1 r + c2 r^2 + c3 r^3 (prm [nucl][4][mo]) to the point's MO

@@ -1,13 +1,14 @@
-"""AO arrays through row images (ao_rows.cu), GPU, against the oracle.
+"""AO Hessian (ao_hessian.cu) and bfloat16 AO pieces (ao_kernels.cu), GPU.
 
 The AO Hessian goes by segments of at most 256 AOs, whose rows leave in bulk
 copies from the 16-byte phase that they have in the output: odd and even AO
 counts, one segment and several, an output that starts 8 bytes past a 16-byte
-boundary, few points and more items than resident CTAs; the FP64 bar, 1e-12.
-The bfloat16 pieces of the AO VGL feed dL/dC of the mixed adjoint alone: tiles
-of 32 points, segments of 32 AOs, AO counts that are no multiple of 8; against
-the FP64 form, with the bound of the FP32 exponentials and of the three-piece
-products (test_gpu_adjoint.py).
+boundary, few points and more items than resident CTAs; against the oracle at
+the FP64 bar, 1e-12.
+The pieces feed dL/dC of the mixed adjoint alone.  Few points have their
+nucleus blocks spread over warps: few and many points, AO counts that are no
+multiple of 8; against the FP64 form, with the bound of the FP32 exponentials
+and of the three-piece products (test_gpu_adjoint.py).
 """
 import numpy as np
 import pytest
