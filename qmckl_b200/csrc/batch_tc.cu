@@ -6,8 +6,14 @@
 // reads its [3][P_s] coordinates at d_coord + coord_offset[s] and writes its
 // mo_vgl[P_s][5][mo_s] at d_mo_vgl + out_offset[s].
 //
-// Device work queue.  One CTA per SM loops: one thread takes the next item
-// with an atomic increment of the queue head, the CTA runs it, and so on.
+// Device work queue.  One CTA per SM loops: the next item is taken with an
+// atomic increment of the queue head, the CTA runs it, and so on.  Two warps
+// plan a tile item (its points and K blocks) while the one before it runs:
+// planned by the whole CTA between the items, with its chain of dependent
+// loads, it took 1.20 ms on 24 molecules of 8 to 80 nuclei and 0.58 ms on 24
+// of 8, now 1.08 and 0.45.  Where shared memory has no room for a second item
+// (long records next to 160-MO tiles), and after a prep item, all threads plan
+// it in between.
 //   prep item  (system s): the CTA orders the system's points spatially
 //              (counting sort over 16^3 cells of the nuclei's box, in shared
 //              memory) into the permutation buffer, then publishes
@@ -71,15 +77,24 @@ struct alignas(64) BatchDesc {
 struct BatchCtl {                 // shared-memory control block of a CTA
   uint64_t full[kStages], empty[kStages], rec_full[kStages], acc_full;
   uint32_t tmem_slot;
-  int item[4];
-  int ok;
-  int claim;   // chunks of the current item claimed by the producer warps after their first
+};
+// An item of the queue with the plan of its tile; in shared memory followed by
+// int act[kb_max], the tile's K blocks.  Two of them where they fit, so that
+// the next item is claimed and planned while the current one runs.
+struct BatchItem {
   double pts[3 * kPts];
   int64_t pidx[kPts];
-  int rexp[3 * kPts];
-  // followed in shared memory by the tile's K blocks, their flags and the
-  // counts (batch_smem): int act[kb_max], flag[kb_max], n, lo, hi, first
+  int item[3];
+  int ok;
+  int claim;   // chunks claimed by the producer warps after their first
+  int cnt[4];  // K blocks of the tile: count, first of each half, first
+  int pad;
 };
+// What one item and the flags take is bounded by what the systems' records
+// leave (batch_smem).
+constexpr size_t kCtlBytes = 1192;
+static_assert(sizeof(BatchCtl) % 8 == 0 && sizeof(BatchItem) % 8 == 0, "items are 8-byte aligned");
+static_assert(sizeof(BatchCtl) + sizeof(BatchItem) <= kCtlBytes, "one item fits");
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
   int v;
@@ -156,19 +171,60 @@ __device__ void order_system(const BatchDesc& D, const double* coord, int* perm,
   __syncthreads();
 }
 
+// K blocks that are not identically zero over a tile's points, as the masks of
+// their 16-AO k-steps (the outcome of tile_kblock_flags), by the `team`
+// threads hl = 0 .. team - 1: a lane per screening sphere drops those beyond
+// the points' bounding box and tests the others against the points.
+__device__ __forceinline__ void batch_flags(const uint8_t* kskip, int kblocks, const double* pts, int np, int* flags,
+                                            int hl, int team) {
+  for (int k = hl; k < kblocks; k += team) flags[k] = kskip == nullptr ? 0xF : 0;
+  named_bar_sync(2, team);
+  if (kskip == nullptr) return;
+  const int nsph = ((const int2*)kskip)[kblocks - 1].y;
+  const double4* sph = (const double4*)(kskip + kskip_sph_offset(kblocks));
+  const int2* kpos = (const int2*)(kskip + kskip_kpos_offset(kblocks, nsph));
+  const int i = min(hl & 31, np - 1);
+  double lo[3], hi[3];   // NaN coordinates left out
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo[d] = hi[d] = pts[d * kPts + i];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+  }
+  for (int q = hl; q < nsph; q += team) {
+    const double4 c = sph[q];
+    const double bx = fmax(fmax(lo[0] - c.x, c.x - hi[0]), 0.0), by = fmax(fmax(lo[1] - c.y, c.y - hi[1]), 0.0),
+                 bz = fmax(fmax(lo[2] - c.z, c.z - hi[2]), 0.0);
+    // the margin covers the rounding of both distances
+    if ((bx * bx + by * by + bz * bz) * (1.0 - 1e-9) > c.w) continue;
+    bool l = false;
+    for (int j = 0; j < np && !l; ++j) {
+      const double x = pts[j] - c.x, y = pts[kPts + j] - c.y, z = pts[2 * kPts + j] - c.z;
+      l = x * x + y * y + z * z <= c.w;
+    }
+    if (!l) continue;
+    const int2 kp = kpos[q];
+    for (int ks = kp.x >> 4; ks <= (kp.x + kp.y - 1) >> 4; ++ks) atomicOr(&flags[ks >> 2], 1 << (ks & 3));
+  }
+}
+
 template <int PRODW>
-__global__ void __launch_bounds__((PRODW + 2) * 32, 1)
+__global__ void __launch_bounds__((PRODW + 4) * 32, 1)
 batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restrict__ tmaps,
                 const int4* __restrict__ items, const int n_items, int* __restrict__ ctl_words,
                 const double* __restrict__ coord, double* __restrict__ out, int* __restrict__ perm,
-                const int n_tile_max, const int rec_max, const int kb_max, const long long wait_limit,
+                const int n_tile_max, const int rec_max, const int kb_max, const int nbuf, const long long wait_limit,
                 const int publish) {
   constexpr int COMPS = 5;
   constexpr int PIECES = kPieces;
+  static_assert(PIECES == 3, "no row exponents");
   constexpr int CHUNK = BK / PRODW;
   constexpr int NPROD = PRODW * 32;
-  constexpr int NTHREADS = (PRODW + 2) * 32;
-  constexpr int TMA_WARP = PRODW, MMA_WARP = PRODW + 1;
+  constexpr int NTHREADS = (PRODW + 4) * 32;
+  constexpr int TMA_WARP = PRODW, MMA_WARP = PRODW + 1, PLAN_WARP = PRODW + 2;   // two planning warps
   int* err = ctl_words;           // [0] error word, [1] queue head, [2..] ready flags
   int* head = ctl_words + 1;
   int* ready = ctl_words + 2;
@@ -178,6 +234,9 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
   const int STAGE = PIECES * (A_TILE + B_MAX);
   uint8_t* recs = smem + kStages * STAGE;
   BatchCtl& C = *(BatchCtl*)(recs + kStages * rec_max);
+  uint8_t* bufs = (uint8_t*)(&C + 1);
+  const int buf_bytes = (int)sizeof(BatchItem) + (kb_max * 4 + 7) / 8 * 8;
+  int* kflag = (int*)(bufs + nbuf * buf_bytes);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint32_t tmem_cols = 32;
   while ((int)tmem_cols < 3 * n_tile_max) tmem_cols <<= 1;
@@ -203,72 +262,80 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
   tc_fence_after();
   const uint32_t tmem = C.tmem_slot;
 
-  uint32_t kbase = 0;    // K blocks run by this CTA so far: pipeline stage and phase
-  uint32_t ntiles = 0;   // tile items run so far: accumulator phase
-  for (;;) {
-    if (tid == 0) {
+  // Claim the next item into buffer b; of a tile item, once its system's
+  // points are in order, the points and the K blocks.  By the two planning
+  // warps while an item runs, else by all threads.
+  auto plan_item = [&](int b, int team) {
+    BatchItem& F = *(BatchItem*)(bufs + b * buf_bytes);
+    const int hl = tid - (NTHREADS - team);
+    if (hl == 0) {
       int4 it = make_int4(-1, 0, 0, 0);
       if (*(volatile int*)err == 0) {
         const int idx = atomicAdd(head, 1);
         if (idx < n_items) it = items[idx];
       }
-      C.item[0] = it.x;
-      C.item[1] = it.y;
-      C.item[2] = it.z;
+      F.item[0] = it.x;
+      F.item[1] = it.y;
+      F.item[2] = it.z;
+      F.claim = 0;
+      F.ok = it.x < 0 || it.y < 0 || wait_flag(&ready[it.x], wait_limit, err) ? 1 : 0;
     }
+    named_bar_sync(2, team);
+    const int sys = F.item[0], ptile = F.item[1];
+    if (sys < 0 || ptile < 0 || !F.ok) return;
+    const BatchDesc& D = desc[sys];
+    const int64_t P = D.P, p0 = (int64_t)ptile * kPts;
+    const double* crd = coord + D.coord_off;
+    const int* pm = perm + D.perm_off;
+    for (int t = hl; t < 3 * kPts; t += team) {
+      const int d = t / kPts, i = t - d * kPts;
+      const int64_t q = (p0 + i < P) ? (int64_t)__ldcg(pm + p0 + i) : -1;
+      F.pts[t] = q >= 0 ? crd[q + d * P] : 0.0;
+      if (d == 0) F.pidx[i] = q;
+    }
+    // (its first barrier comes after the points, too)
+    batch_flags(D.kskip, D.kblocks, F.pts, (int)(P - p0 < kPts ? P - p0 : kPts), kflag, hl,
+                team);
+    named_bar_sync(2, team);
+    if (warp == PLAN_WARP) tile_kblock_list(kflag, D.kblocks, (int*)(&F + 1), F.cnt, lane, true);
+  };
+
+  uint32_t kbase = 0;    // K blocks run by this CTA so far: pipeline stage and phase
+  uint32_t ntiles = 0;   // tile items run so far: accumulator phase
+  int b = 0;             // the current item's buffer
+  plan_item(0, NTHREADS);
+  for (;;) {
     tc_fence_before();
-    __syncthreads();
+    __syncthreads();   // the item is planned, the one before it done
     tc_fence_after();
-    const int sys = C.item[0], ptile = C.item[1], ntile = C.item[2];
+    BatchItem& F = *(BatchItem*)(bufs + b * buf_bytes);
+    const int sys = F.item[0], ptile = F.item[1], ntile = F.item[2];
     if (sys < 0) break;
     const BatchDesc& D = desc[sys];
-    if (ptile < 0) {
-      // ---------------- prep item: point order of the system (stage memory as scratch)
-      order_system(D, coord, perm, smem, tid, NTHREADS);
-      zero_pad_rows<PIECES, COMPS, kStages>(smem, STAGE, tid, NTHREADS);
-      fence_async_smem();
+    if (ptile < 0 || !F.ok) {
+      if (ptile < 0) {
+        // ---------------- prep item: point order of the system (stage memory as scratch)
+        order_system(D, coord, perm, smem, tid, NTHREADS);
+        zero_pad_rows<PIECES, COMPS, kStages>(smem, STAGE, tid, NTHREADS);
+        fence_async_smem();
+      }
       __syncthreads();
-      if (tid == 0) {
+      if (ptile < 0 && tid == PLAN_WARP * 32) {
         __threadfence();
         if (publish) st_release(&ready[sys], 1);
       }
+      // never planned ahead: a claimed prep item is run at once
+      plan_item(b, NTHREADS);
       continue;
     }
     // ---------------- tile item
-    if (tid == 0) C.ok = wait_flag(&ready[sys], wait_limit, err) ? 1 : 0;
-    __syncthreads();
-    if (!C.ok) continue;
     const int64_t P = D.P;
     const int64_t p0 = (int64_t)ptile * kPts;
-    const double* crd = coord + D.coord_off;
-    const int* pm = perm + D.perm_off;
-    for (int t = tid; t < 3 * kPts; t += NTHREADS) {
-      const int d = t / kPts, i = t - d * kPts;
-      const int64_t q = (p0 + i < P) ? (int64_t)__ldcg(pm + p0 + i) : -1;
-      C.pts[t] = q >= 0 ? crd[q + d * P] : 0.0;
-      if (d == 0) C.pidx[i] = q;
-      C.rexp[t] = PIECES == 2 ? kExpMin : 0;
-    }
-    __syncthreads();
-    if (PIECES == 2) {
-      row_exponents<kPts>(D.rb, C.pts, C.pidx, C.rexp, tid, NTHREADS);
-      __syncthreads();
-    }
     const int kblocks = D.kblocks, n_tile = D.n_tile, rec_bytes = D.rec_bytes;
     const int n0 = ntile * n_tile;
     const int B_TILE = n_tile * BK * 2;
-    // K blocks that are not identically zero over the tile's points (as in
-    // the single-system fused kernel, fused_tc.cu)
-    int* act = (int*)(&C + 1);
-    int* kflag = act + kb_max;
-    int* kcnt = kflag + kb_max;
-    tile_kblock_flags<kPts>(D.kskip, kblocks, C.pts, (int)(P - p0 < kPts ? P - p0 : kPts), kflag, warp, lane,
-                            NTHREADS / 32, true);
-    __syncthreads();
-    if (warp == 0) tile_kblock_list(kflag, kblocks, act, kcnt, lane, true);
-    if (tid == 0) C.claim = 0;
-    __syncthreads();
-    const int nact = kcnt[0];
+    const int* act = (const int*)(&F + 1);
+    const int nact = F.cnt[0];
     if (warp < PRODW) {
       // the item's PRODW chunks per K block, claimed in order from a shared
       // counter (first: chunk `warp` of the first block), as in the
@@ -287,12 +354,12 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
         ok = ok && mbar_wait(&C.rec_full[s], phase, err, 25);
         if (!__all_sync(0xffffffffu, ok)) break;
         if (kstep_live(act[it], c, CHUNK))
-          produce_kblock<PIECES, COMPS, CHUNK>(recs + s * rec_max, C.pts, p0, P, D.cutoff, C.rexp,
+          produce_kblock<PIECES, COMPS, CHUNK>(recs + s * rec_max, F.pts, p0, P, D.cutoff, nullptr,
                                                smem_addr(smem + s * STAGE), c, lane);
         fence_async_smem();
         mbar_arrive(&C.full[s]);
         int nq = 0;
-        if (lane == 0) nq = atomicAdd(&C.claim, 1) + PRODW;
+        if (lane == 0) nq = atomicAdd(&F.claim, 1) + PRODW;
         q = __shfl_sync(0xffffffffu, nq, 0);
       }
     } else if (warp == TMA_WARP) {
@@ -311,6 +378,8 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
           for (int q = 0; q < PIECES; ++q) tma_load_3d(st + q * B_TILE, map, &C.full[s], kb * BK, n0, q);
         }
       }
+    } else if (warp >= PLAN_WARP) {
+      if (nbuf == 2) plan_item(b ^ 1, 64);
     } else {
       if (lane == 0) {
         const uint32_t idesc = mma_idesc<PIECES>(n_tile);
@@ -346,14 +415,14 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
       if (bulk) {
         double* stg = (double*)smem;
         if (ok)
-          epilogue_stage_warp<PIECES, COMPS>(tmem, n_tile, n0, D.n_out, kcnt[2] >= 0, C.rexp, D.scales, stg, ldst,
-                                             warp, lane, warp >> 2, PRODW / 4, kcnt[1] >= 0);
+          epilogue_stage_warp<PIECES, COMPS>(tmem, n_tile, n0, D.n_out, F.cnt[2] >= 0, nullptr, D.scales, stg, ldst,
+                                             warp, lane, warp >> 2, PRODW / 4, F.cnt[1] >= 0);
         fence_async_smem();
         named_bar_sync(1, NPROD);   // all producer warps arrive, whatever their `ok`
         if (ok) {
           const int ncols = min(n_tile, D.n_out - n0);
           for (int r = tid; r < kPts * COMPS; r += NPROD) {
-            const int64_t pq = C.pidx[r / COMPS];
+            const int64_t pq = F.pidx[r / COMPS];
             if (pq >= 0)
               bulk_store(o + (pq * COMPS + r % COMPS) * D.n_out + n0, stg + (size_t)r * ldst, (uint32_t)ncols * 8u);
           }
@@ -361,13 +430,19 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
           bulk_wait_read();
         }
       } else if (ok) {
-        epilogue_warp<PIECES, COMPS>(tmem, n_tile, n0, D.n_out, kcnt[2] >= 0, C.pidx, C.rexp, D.scales, o,
+        epilogue_warp<PIECES, COMPS>(tmem, n_tile, n0, D.n_out, F.cnt[2] >= 0, F.pidx, nullptr, D.scales, o,
                                      (double*)smem + warp * 32 * 16, warp, lane, warp >> 2, PRODW / 4,
-                                     kcnt[1] >= 0);
+                                     F.cnt[1] >= 0);
       }
     }
     kbase += (uint32_t)nact;
     ++ntiles;
+    if (nbuf == 2) {
+      b ^= 1;
+    } else {   // one buffer: the next item is planned when this one is done
+      __syncthreads();
+      plan_item(b, NTHREADS);
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -383,9 +458,9 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
   }
 }
 
-size_t batch_smem(int n_tile_max, int rec_max, int kb_max) {
+size_t batch_smem(int n_tile_max, int rec_max, int kb_max, int nbuf = 1) {
   return 1024 + (size_t)kStages * kPieces * (A_TILE + (size_t)n_tile_max * BK * 2) + (size_t)kStages * rec_max +
-         sizeof(BatchCtl) + (size_t)(2 * kb_max + 4) * 4;
+         kCtlBytes + (size_t)(2 * kb_max + 4) * 4 + (nbuf - 1) * (sizeof(BatchItem) + (size_t)(kb_max * 4 + 7) / 8 * 8);
 }
 
 struct BatchSys {
@@ -502,31 +577,31 @@ cudaError_t build_items(Batch* B) {
   return e;
 }
 
-cudaError_t set_kernel_attrs(Batch* B) {
-  const size_t smem = batch_smem(B->n_tile_max, B->rec_max, B->kb_max);
-  cudaError_t e = cudaFuncSetAttribute(batch_mo_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(batch_mo_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+cudaError_t set_kernel_attrs() {
+  // the most any batch takes: the attribute belongs to the kernel, not to this batch
+  cudaError_t e = cudaFuncSetAttribute(batch_mo_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_mo_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
   return e;
 }
 
 cudaError_t enqueue(Batch* B, const double* coord, double* out) {
-  const size_t smem = batch_smem(B->n_tile_max, B->rec_max, B->kb_max);
+  const int nbuf = batch_smem(B->n_tile_max, B->rec_max, B->kb_max, 2) <= 232448 ? 2 : 1;
+  const size_t smem = batch_smem(B->n_tile_max, B->rec_max, B->kb_max, nbuf);
   cudaError_t e = cudaMemsetAsync(B->ctl.p, 0, sizeof(int) * (2 + B->sys.size()), B->stream);
   if (e != cudaSuccess) return e;
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, B->device);
   const int grid = std::max(1, std::min(sms, B->n_items));
   if (B->prod_warps == 8)
-    batch_mo_kernel<8><<<grid, 10 * 32, smem, B->stream>>>(
+    batch_mo_kernel<8><<<grid, 12 * 32, smem, B->stream>>>(
         (const BatchDesc*)B->desc.p, (const CUtensorMap*)B->tmaps.p, (const int4*)B->items.p, B->n_items,
-        (int*)B->ctl.p, coord, out, (int*)B->perm.p, B->n_tile_max, B->rec_max, B->kb_max, B->wait_limit,
-        B->publish);
+        (int*)B->ctl.p, coord, out, (int*)B->perm.p, B->n_tile_max, B->rec_max, B->kb_max, nbuf,
+        B->wait_limit, B->publish);
   else
-    batch_mo_kernel<16><<<grid, 18 * 32, smem, B->stream>>>(
+    batch_mo_kernel<16><<<grid, 20 * 32, smem, B->stream>>>(
         (const BatchDesc*)B->desc.p, (const CUtensorMap*)B->tmaps.p, (const int4*)B->items.p, B->n_items,
-        (int*)B->ctl.p, coord, out, (int*)B->perm.p, B->n_tile_max, B->rec_max, B->kb_max, B->wait_limit,
-        B->publish);
+        (int*)B->ctl.p, coord, out, (int*)B->perm.p, B->n_tile_max, B->rec_max, B->kb_max, nbuf,
+        B->wait_limit, B->publish);
   return cudaGetLastError();
 }
 
@@ -770,7 +845,7 @@ qmckl_exit_code qmckl_b200_batch_create(const qmckl_context* contexts, const int
       cudaStreamSynchronize(B->stream) != cudaSuccess)
     return bail("descriptor upload failed");
   load_tuning(B);
-  if (build_items(B) != cudaSuccess || set_kernel_attrs(B) != cudaSuccess) return bail("work queue setup failed");
+  if (build_items(B) != cudaSuccess || set_kernel_attrs() != cudaSuccess) return bail("work queue setup failed");
   *batch = (qmckl_b200_batch)(new BatchHandle{kBatchTag, B});
   return QMCKL_SUCCESS;
 }

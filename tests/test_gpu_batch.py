@@ -147,7 +147,7 @@ def test_dependency_wait_cap_reports_failure(batch_case):
     status = pq.b200_batch_synchronize(b, raise_on_error=False)
     assert status == 26
     with pytest.raises(RuntimeError):
-        pq.b200_batch_synchronize(b)
+        assert pq.b200_batch_synchronize(b) == 0
     pq.b200_batch_set_wait_limit(b, 0, publish=True)
     _check_equal_single(batch_case, _run(batch_case))
 
@@ -159,3 +159,48 @@ def test_batch_accuracy_vs_fp64(batch_case):
             continue
         ref = _single(batch_case, s, form=pq.FORM_FP64)
         assert max(comp_error(_slice(batch_case, out, s), ref)) <= 1e-6
+
+
+def _split_primitives(d, k):
+    """The same basis with the primitives of its first k shells given twice, at half the coefficient: longer records."""
+    d = dict(d)
+    num, ind = d["shell_prim_num"], d["shell_prim_index"]
+    pick = [i for s in range(num.size) for i in np.repeat(np.arange(ind[s], ind[s] + num[s]), 2 if s < k else 1)]
+    half = np.array([0.5 if s < k else 1.0 for s in range(num.size) for _ in range(num[s] * (2 if s < k else 1))])
+    new = np.where(np.arange(num.size) < k, 2 * num, num)
+    d["shell_prim_num"], d["shell_prim_index"] = new, np.concatenate([[0], np.cumsum(new)[:-1]])
+    d["exponent"], d["prim_factor"] = d["exponent"][pick], d["prim_factor"][pick]
+    d["coefficient"] = d["coefficient"][pick] * half
+    return d
+
+
+@pytest.mark.parametrize("split,P", [(0, (12001, 4000, 26)), (12, (9000, 25, 1)), (15, (9000, 24, 0)), (18, (9000, 3, 51)),
+                                     (21, (9000, 26, 100))])
+def test_items_planned_ahead(split, P):
+    """Several items per CTA, so that each is planned while the one before runs; with records that leave no room for a
+    second item (160-MO systems with long contractions) it is planned afterwards.  Against the single-system kernel."""
+    import torch
+    systems = [_split_primitives(gen.config(0, walk_num=1), split), gen.config(1, walk_num=1), gen.high_l_config(1)]
+    ctxs = [make_context(s, points=False, form=pq.FORM_MIXED) for s in systems]
+    rng = np.random.default_rng(split)
+    b = pq.b200_batch_create(ctxs, list(P))
+    co, oo, (ct, ot) = pq.b200_batch_layout(b, 3)
+    coord = np.zeros(ct)
+    for s, d in enumerate(systems):
+        xyz = np.asarray(d["nucl_coord"]).reshape(3, -1).T
+        coord[co[s]:co[s] + 3 * P[s]] = (xyz[rng.integers(0, xyz.shape[0], P[s])] + rng.standard_normal((P[s], 3))).T.reshape(-1)
+    d_coord = torch.tensor(coord, dtype=torch.float64, device="cuda")
+    d_out = torch.full((ot,), float("nan"), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    case = dict(systems=systems, ctxs=ctxs, P=P, co=co, oo=oo, coord=coord)
+    try:
+        pq.b200_batch_mo_vgl_device(b, d_coord.data_ptr(), d_out.data_ptr())
+        assert pq.b200_batch_synchronize(b) == 0
+        out = d_out.cpu().numpy()
+        for s in range(3):
+            if P[s]:
+                assert max(comp_error(_slice(case, out, s), _single(case, s))) < 2e-6
+    finally:
+        pq.b200_batch_destroy(b)
+        for c in ctxs:
+            pq.context_destroy(c)
