@@ -129,12 +129,14 @@ __device__ __forceinline__ void emit_shell_any(double* __restrict__ o, int64_t l
 // its lanes on the AOs, as the dense AO kernel works, visits every AO of
 // every point and took 0.73 ms for the 3.3 GB array).  CTA 0 of the tile
 // writes its AO list.
-// Scratch: dynamic shared memory of 2 * shell_num ints.
+// Scratch: dynamic shared memory of 2 * shell_num ints; more shells than fit
+// there come in windows [w0, w0 + shell_num) of all_shells, a launch each, that
+// continue the tile's lists.
 template <int COMPS, int TP, int PARTS>
 __global__ void __launch_bounds__(kAoThreads, 4)
 ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t cstride, const int* __restrict__ perm,
-                const int64_t tile0, const int shell_num, const F64Shell* __restrict__ sh,
-                const double2* __restrict__ prim, const double* __restrict__ factor, const double cutoff,
+                const int64_t tile0, const int w0, const int shell_num, const int all_shells,
+                const F64Shell* __restrict__ sh, const double2* __restrict__ prim, const double* __restrict__ factor, const double cutoff,
                 const bool dp_exp, const double* __restrict__ cusp_r, const int64_t kmax, double* __restrict__ ac,
                 int* __restrict__ klist, int* __restrict__ kcount, const AdjTables adj) {
   constexpr int G = TP / 32;
@@ -157,6 +159,8 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     spts[t] = i < np ? coord[(perm ? (int64_t)perm[p0 + i] : p0 + i) + d * cstride] : 0.0;
   }
   if (tid == 0) claim = nopen = 0;
+  sh += w0;
+  const int k0 = w0 > 0 ? kcount[tile] : 0, q0 = w0 > 0 ? adj.nlive[tile] : 0;   // the lists of the windows before
   __syncthreads();
   if (warp < G) {   // bounding box of each 32 points (NaN coordinates left out)
     const int i = max(0, min(32 * warp + lane, np - 1));
@@ -288,17 +292,17 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     int* kl = klist + tile * kmax;
     for (int q = tid; q < nlive; q += kAoThreads) {
       const F64Shell S = sh[live[q] & 0xffffff];
-      const int k = lpos[q];
+      const int k = k0 + lpos[q];
       for (int i = 0; i < S.na; ++i) kl[k + i] = S.a0 + i;
       if (adj.live != nullptr) {
-        adj.live[tile * shell_num + q] = make_int2(live[q] & 0xffffff, k);
+        adj.live[(int64_t)tile * all_shells + q0 + q] = make_int2(w0 + (live[q] & 0xffffff), k);
         if (adj.inv != nullptr)
           for (int i = 0; i < S.na; ++i) adj.inv[tile * kmax + S.a0 + i] = k + i;
       }
     }
     if (tid == 0) {
-      kcount[tile] = nao;
-      if (adj.live != nullptr) adj.nlive[tile] = nlive;
+      kcount[tile] = k0 + nao;
+      if (adj.live != nullptr) adj.nlive[tile] = q0 + nlive;
     }
   }
   if (ac == nullptr) return;   // the lists only
@@ -319,7 +323,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     const F64Shell S = sh[e & 0xffffff];
     if (part > 0 && S.l < 4) continue;
     const int i = 32 * g + lane;
-    double* o = act + (size_t)lpos[q] * LD + i;
+    double* o = act + (size_t)(k0 + lpos[q]) * LD + i;
     const double x = spts[i] - S.x, y = spts[TP + i] - S.y, z = spts[2 * TP + i] - S.z;
     const double r2 = x * x + y * y + z * z;
     double s[5] = {0., 0., 0., 0., 0.};
@@ -777,8 +781,10 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
                             bool dp_exp, const double* cusp_r, const F64Tiles& t, cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
   if (!(comps == 5 && t.pts == 32) && !(comps == 1 && (t.pts == 32 || t.pts == 128))) return cudaErrorInvalidValue;
-  const size_t sm = sizeof(int) * 2 * (size_t)T.shell_num;
-  if (sm > 200 * 1024) return cudaErrorInvalidValue;
+  // in windows for the adjoint only: the forward refuses so many shells
+  constexpr int kWindow = 200 * 1024 / (2 * (int)sizeof(int));
+  if (T.shell_num > kWindow && t.adj.live == nullptr) return cudaErrorInvalidValue;
+  const size_t sm = sizeof(int) * 2 * (size_t)std::min(T.shell_num, kWindow);
   auto kern = T.shell_parts > 1
                   ? (comps == 5 ? ao_tiles_kernel<5, 32, 4>
                                 : (t.pts == 32 ? ao_tiles_kernel<1, 32, 4> : ao_tiles_kernel<1, 128, 4>))
@@ -788,11 +794,16 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1));
   if (e != cudaSuccess) return e;
   // few tiles: several CTAs share one, so that its shells are spread over SMs
-  const int parts = t.ac == nullptr ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
-  kern<<<dim3((unsigned)ntiles, (unsigned)parts), kAoThreads, sm, s>>>(
-      P, coord, cstride, perm, tile0, T.shell_num, sh, T.coef_ac, T.ao_factor, cutoff, dp_exp, cusp_r, T.ao_num,
-      t.ac, t.klist, t.kcount, t.adj);
-  count_launch();
+  // (not over windows: a window reads the counts that the one before wrote)
+  const int parts = t.ac == nullptr || T.shell_num > kWindow
+                        ? 1
+                        : (int)std::max<int64_t>(1, std::min<int64_t>(8, (8 * 148 + ntiles - 1) / ntiles));
+  for (int w0 = 0; w0 < T.shell_num; w0 += kWindow) {
+    kern<<<dim3((unsigned)ntiles, (unsigned)parts), kAoThreads, sm, s>>>(
+        P, coord, cstride, perm, tile0, w0, std::min(kWindow, T.shell_num - w0), T.shell_num, sh, T.coef_ac, T.ao_factor,
+        cutoff, dp_exp, cusp_r, T.ao_num, t.ac, t.klist, t.kcount, t.adj);
+    count_launch();
+  }
   return cudaGetLastError();
 }
 

@@ -153,3 +153,33 @@ def test_adjoint_coefficients_repeat():
     finally:
         pq.context_destroy(ctx)
     assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
+
+
+def test_adjoint_many_shells():
+    """More shells than a tile's lists hold at a time (25,600): listed in windows."""
+    n, per, P, m = 2600, 10, 40, 3
+    rng = np.random.default_rng(11)
+    S = n * per
+    grid = np.stack(np.meshgrid(*[np.arange(14)] * 3, indexing="ij"), -1).reshape(-1, 3)[:n] * 2.0
+    d = dict(nucl_num=n, charge=np.ones(n), nucl_coord=np.ascontiguousarray(grid.T.astype(float)),
+             nucleus_index=np.arange(0, S, per), nucleus_shell_num=np.full(n, per), shell_ang_mom=np.zeros(S, dtype=np.int32),
+             shell_prim_num=np.ones(S, dtype=np.int64), shell_prim_index=np.arange(S), shell_factor=np.ones(S),
+             exponent=rng.uniform(0.3, 20.0, S), coefficient=np.ones(S), prim_factor=np.ones(S), ao_factor=np.ones(S),
+             ao_num=S, mo_num=m, mo_coef=rng.standard_normal((m, S)))
+    # points around the nuclei on both sides of the window's edge (nucleus 2560)
+    pts = grid[rng.integers(2400, n, P)] + rng.standard_normal((P, 3))
+    w = rng.standard_normal((P, 5, m))
+    ref = O.mo_vgl_adjoint(O.Basis(d), pts, d["nucl_coord"], d["mo_coef"], w)
+    t = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")  # noqa: E731
+    c, dw = t(pts.T), t(w)
+    for form, tol in ((pq.FORM_FP64, 1e-10), (pq.FORM_MIXED, 1e-6)):
+        ctx = make_context(d, points=False, form=form)
+        gc, gn, gr = (torch.full(s, float("nan"), dtype=torch.float64, device="cuda") for s in ((m, S), (n, 3), (3, P)))
+        torch.cuda.synchronize()
+        try:
+            pq.b200_mo_vgl_adjoint_device(ctx, P, c.data_ptr(), dw.data_ptr(), gc.data_ptr(), gn.data_ptr(), gr.data_ptr())
+            pq.b200_synchronize(ctx)
+        finally:
+            pq.context_destroy(ctx)
+        for got, want in zip((gc, gn, gr.T), ref):
+            assert np.abs(got.cpu().numpy() - want).max() <= tol * np.abs(want).max()
