@@ -154,8 +154,8 @@ ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restri
   WarpSmem& sm = smem[warp];
   const int64_t A = T.ao_num;
   const int64_t stride = (int64_t)gridDim.x * kWarps;
-  const int b0 = (int)((int64_t)T.nblock * blockIdx.y / gridDim.y);
-  const int b1 = (int)((int64_t)T.nblock * (blockIdx.y + 1) / gridDim.y);
+  const int per = (T.nblock + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int b0 = (int)blockIdx.y * per, b1 = min(T.nblock, b0 + per);
   for (int64_t p = (int64_t)blockIdx.x * kWarps + warp; p < point_num; p += stride)
   for (int b = b0; b < b1; ++b) {
     const int4 blk = T.block[b];
