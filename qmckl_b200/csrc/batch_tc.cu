@@ -11,7 +11,7 @@
 // plan a tile item (its points and K blocks) while the one before it runs:
 // planned by the whole CTA between the items, with its chain of dependent
 // loads, it took 1.20 ms on 24 molecules of 8 to 80 nuclei and 0.58 ms on 24
-// of 8, now 1.08 and 0.45.  Where shared memory has no room for a second item
+// of 8, now 1.07 and 0.45.  Where shared memory has no room for a second item
 // (long records next to 160-MO tiles), and after a prep item, all threads plan
 // it in between.
 //   prep item  (system s): the CTA orders the system's points spatially
@@ -83,12 +83,11 @@ struct BatchCtl {                 // shared-memory control block of a CTA
 // the next item is claimed and planned while the current one runs.
 struct BatchItem {
   double pts[3 * kPts];
-  int64_t pidx[kPts];
+  int pidx[kPts];   // the points' places in the system (-1: none)
   int item[3];
   int ok;
   int claim;   // chunks claimed by the producer warps after their first
   int cnt[4];  // K blocks of the tile: count, first of each half, first
-  int pad;
 };
 // What one item and the flags take is bounded by what the systems' records
 // leave (batch_smem).
@@ -289,7 +288,7 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
     const int* pm = perm + D.perm_off;
     for (int t = hl; t < 3 * kPts; t += team) {
       const int d = t / kPts, i = t - d * kPts;
-      const int64_t q = (p0 + i < P) ? (int64_t)__ldcg(pm + p0 + i) : -1;
+      const int q = (p0 + i < P) ? __ldcg(pm + p0 + i) : -1;
       F.pts[t] = q >= 0 ? crd[q + d * P] : 0.0;
       if (d == 0) F.pidx[i] = q;
     }
@@ -459,8 +458,10 @@ batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restric
 }
 
 size_t batch_smem(int n_tile_max, int rec_max, int kb_max, int nbuf = 1) {
+  const size_t one = kCtlBytes + (size_t)(2 * kb_max + 4) * 4,
+               two = sizeof(BatchCtl) + 2 * (sizeof(BatchItem) + (size_t)(kb_max * 4 + 7) / 8 * 8) + (size_t)kb_max * 4;
   return 1024 + (size_t)kStages * kPieces * (A_TILE + (size_t)n_tile_max * BK * 2) + (size_t)kStages * rec_max +
-         kCtlBytes + (size_t)(2 * kb_max + 4) * 4 + (nbuf - 1) * (sizeof(BatchItem) + (size_t)(kb_max * 4 + 7) / 8 * 8);
+         (nbuf == 2 ? two : one);
 }
 
 struct BatchSys {

@@ -461,9 +461,9 @@ __device__ __forceinline__ uint32_t mma_idesc(int n_tile) {
 // (tile point i, component c) written to out[(pidx[i] * COMPS + c) * n_out +
 // col] for the MO columns [n0, n0 + n_tile).
 // stage: 32 x 16 doubles of shared scratch for this warp.
-template <int PIECES, int COMPS, int NACC = 3>
+template <int PIECES, int COMPS, int NACC = 3, class Idx>
 __device__ __forceinline__ void epilogue_warp(uint32_t tmem, int n_tile, int n0, int n_out, bool has_second,
-                                              const int64_t* pidx, const int* rexp, const double* scales,
+                                              const Idx* pidx, const int* rexp, const double* scales,
                                               double* out, double* stage, int warp, int lane, int chunk0 = 0,
                                               int chunk_step = 1, bool has_first = true) {
   constexpr int PTS = BM / COMPS;

@@ -174,17 +174,32 @@ def _split_primitives(d, k):
     return d
 
 
-@pytest.mark.parametrize("split,P", [(0, (12001, 4000, 26)), (12, (9000, 25, 1)), (15, (9000, 24, 0)), (18, (9000, 3, 51)),
-                                     (21, (9000, 26, 100))])
-def test_items_planned_ahead(split, P):
-    """Several items per CTA, so that each is planned while the one before runs; with records that leave no room for a
-    second item (160-MO systems with long contractions) it is planned afterwards.  Against the single-system kernel."""
+def _many_aos():
+    """512 nuclei with two f shells each: 10,240 AOs in 160 K blocks of short records."""
+    n, S = 512, 1024
+    grid = np.stack(np.meshgrid(*[np.arange(8)] * 3, indexing="ij"), -1).reshape(-1, 3) * 3.0
+    rng = np.random.default_rng(3)
+    return dict(nucl_num=n, charge=np.ones(n), nucl_coord=np.ascontiguousarray(grid.T), nucleus_index=np.arange(0, S, 2),
+                nucleus_shell_num=np.full(n, 2), shell_ang_mom=np.full(S, 3, dtype=np.int32),
+                shell_prim_num=np.ones(S, dtype=np.int64), shell_prim_index=np.arange(S), shell_factor=np.ones(S),
+                exponent=rng.uniform(0.4, 3.0, S), coefficient=np.ones(S), prim_factor=np.ones(S), ao_factor=np.ones(10 * S),
+                ao_num=10 * S, mo_num=4, mo_coef=rng.standard_normal((4, 10 * S)) / 100.0)
+
+
+@pytest.mark.parametrize("split,many,P", [(0, 0, (12001, 4000, 26)), (15, 0, (9000, 24, 0)), (21, 0, (9000, 26, 100)),
+                                          (12, 1, (9000, 25, 1, 51))])
+def test_items_planned_ahead(split, many, P):
+    """Several items per CTA, so that each is planned while the one before runs; with long records (a contraction given
+    twice) next to 160-MO tiles and many K blocks there is no room for a second item, and it is planned afterwards.
+    Against the single-system kernel."""
     import torch
     systems = [_split_primitives(gen.config(0, walk_num=1), split), gen.config(1, walk_num=1), gen.high_l_config(1)]
+    if many:
+        systems.append(_many_aos())
     ctxs = [make_context(s, points=False, form=pq.FORM_MIXED) for s in systems]
     rng = np.random.default_rng(split)
     b = pq.b200_batch_create(ctxs, list(P))
-    co, oo, (ct, ot) = pq.b200_batch_layout(b, 3)
+    co, oo, (ct, ot) = pq.b200_batch_layout(b, len(systems))
     coord = np.zeros(ct)
     for s, d in enumerate(systems):
         xyz = np.asarray(d["nucl_coord"]).reshape(3, -1).T
@@ -197,7 +212,7 @@ def test_items_planned_ahead(split, P):
         pq.b200_batch_mo_vgl_device(b, d_coord.data_ptr(), d_out.data_ptr())
         assert pq.b200_batch_synchronize(b) == 0
         out = d_out.cpu().numpy()
-        for s in range(3):
+        for s in range(len(systems)):
             if P[s]:
                 assert max(comp_error(_slice(case, out, s), _single(case, s))) < 2e-6
     finally:
