@@ -100,7 +100,8 @@ cudaError_t tc_launch_fused(const TcPlan& plan, int64_t point_num, int comps, co
 cudaError_t tc_set_late_warps(unsigned int ns);
 // Spatial order of points (point_order.cu): perm[P] <- the points in Morton
 // order of 32^3 cells over [box_lo, box_hi], in their own order within a cell.
-// scratch: point_order_bytes(P) bytes, 256-byte aligned.  cstride: distance
+// scratch: point_order_bytes(P) bytes, 256-byte aligned (grows with P: scratch
+// for a count serves every smaller one).  cstride: distance
 // between the x, y and z blocks of coord (default point_num; larger for a
 // slice of a bigger [3][N] array).  The fused kernels take the same stride.
 size_t point_order_bytes(int64_t point_num);

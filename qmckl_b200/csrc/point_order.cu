@@ -255,10 +255,13 @@ int64_t order_ctas(int64_t P) { return (P + order_run(P) - 1) / order_run(P); }
 
 }  // namespace
 
+// The count of CTAs falls where a run grows by 256 points (64 at 65,536 points,
+// 52 at 65,537); the histograms get room for the most that any count up to
+// point_num takes, so that scratch made for a count serves every smaller one.
 size_t point_order_bytes(int64_t point_num) {
   if (point_num <= kOneCta) return 0;
-  return code_bytes(point_num) + sizeof(unsigned int) * kDigits * (size_t)order_ctas(point_num) +
-         sizeof(int) * (size_t)point_num;
+  const int64_t most = std::max<int64_t>(kCtas, (point_num + kMaxRun - 1) / kMaxRun);
+  return code_bytes(point_num) + sizeof(unsigned int) * kDigits * (size_t)most + sizeof(int) * (size_t)point_num;
 }
 
 cudaError_t point_order(const double* coord, int64_t point_num, const double* box_lo, const double* box_hi,
