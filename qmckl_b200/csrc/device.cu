@@ -376,6 +376,7 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
+  std::vector<char> host_f64_sph;   // source of f64_sph's upload
   AoSegments hess{};   // in f64_sph: the shell records and the segments of the AO Hessian
 };
 
@@ -718,7 +719,9 @@ qmckl_exit_code copy_out(qmckl_context context, DeviceState* ds, double* host, c
 DeviceState* state(qmckl_context context) { return ctx_of(context)->extra; }
 
 // The per-shell records of the FP64 tile kernels and of the AO Hessian (basis
-// order), and the latter's segments.
+// order), and the latter's segments; for nuclei that moved since, their
+// positions in the records.  All on the context's stream, behind the kernels
+// that read the records before.
 qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
   const char* fname = "qmckl_b200_mo_fp64";
   Context* ctx = ctx_of(context);
@@ -726,9 +729,13 @@ qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
   const AoDerived& d = B.d;
   const int64_t A = B.ao_num, S = B.shell_num, N = ctx->nucleus.num;
   const double cutoff = cutoff_of(ctx);
-  if (ds->f64_sph.p && ds->f64_sph_basis == B.basis_version && ds->f64_sph_nucl == ctx->nucleus.coord_version &&
-      ds->f64_sph_cutoff == cutoff)
+  if (ds->f64_sph.p && ds->f64_sph_basis == B.basis_version && ds->f64_sph_cutoff == cutoff) {
+    if (ds->f64_sph_nucl != ctx->nucleus.coord_version) {
+      QB_CUDA(launch_place_shells(ds->T, (F64Shell*)ds->f64_sph.p, ds->stream), fname);
+      ds->f64_sph_nucl = ctx->nucleus.coord_version;
+    }
     return QMCKL_SUCCESS;
+  }
   std::vector<F64Shell> sh((size_t)S);
   for (int64_t m = 0; m < N; ++m)
     for (int64_t s = B.nucleus_index[m]; s < B.nucleus_index[m] + B.nucleus_shell_num[m]; ++s) {
@@ -759,12 +766,14 @@ qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
     g.max_shells = std::max(g.max_shells, (int)(s1 - s0));
   }
   g.nseg = (int)segs.size();
-  const size_t sb = sizeof(F64Shell) * (size_t)S;
-  qmckl_exit_code rc = ensure(context, ds->f64_sph, sb + sizeof(int2) * segs.size(), fname);
+  const size_t sb = sizeof(F64Shell) * (size_t)S, bytes = sb + sizeof(int2) * segs.size();
+  qmckl_exit_code rc = ensure(context, ds->f64_sph, bytes, fname);
   if (rc != QMCKL_SUCCESS) return rc;
-  QB_CUDA(cudaMemcpy(ds->f64_sph.p, sh.data(), sb, cudaMemcpyHostToDevice), fname);
-  QB_CUDA(cudaMemcpy((uint8_t*)ds->f64_sph.p + sb, segs.data(), sizeof(int2) * segs.size(), cudaMemcpyHostToDevice),
-          fname);
+  std::vector<char>& H = ds->host_f64_sph;
+  H.resize(bytes);
+  if (S > 0) std::memcpy(H.data(), sh.data(), sb);
+  if (!segs.empty()) std::memcpy(H.data() + sb, segs.data(), bytes - sb);
+  QB_CUDA(cudaMemcpyAsync(ds->f64_sph.p, H.data(), bytes, cudaMemcpyHostToDevice, ds->stream), fname);
   g.sh = (const F64Shell*)ds->f64_sph.p;
   g.seg = (const int2*)((uint8_t*)ds->f64_sph.p + sb);
   ds->hess = g;
@@ -955,19 +964,21 @@ qmckl_exit_code coef_even(qmckl_context context, DeviceState* ds, const double**
   Context* ctx = ctx_of(context);
   const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
   *ldb = M + (M & 1);
+  qmckl_exit_code rc = sync_coef(context, ds);
+  if (rc != QMCKL_SUCCESS) return rc;
   if (!(M & 1)) {
-    qmckl_exit_code rc = sync_coef(context, ds);
     *Bt = (const double*)ds->coef_t.p;
-    return rc;
+    return QMCKL_SUCCESS;
   }
   if (ds->coef_f_version != ctx->mo_basis.coef_version || !ds->coef_f.p) {
-    std::vector<double> cf((size_t)(A * *ldb), 0.0);
-    const std::vector<double>& c = ctx->mo_basis.coefficient;
-    for (int64_t k = 0; k < A; ++k)
-      for (int64_t i = 0; i < M; ++i) cf[(size_t)(k * *ldb + i)] = c[(size_t)(i * A + k)];
-    qmckl_exit_code rc = ensure(context, ds->coef_f, sizeof(double) * cf.size(), fname);
+    // from the device's coefficient_t, on the context's stream, behind the
+    // kernels that read the copy before
+    rc = ensure(context, ds->coef_f, sizeof(double) * (size_t)(A * *ldb), fname);
     if (rc != QMCKL_SUCCESS) return rc;
-    QB_CUDA(cudaMemcpy(ds->coef_f.p, cf.data(), sizeof(double) * cf.size(), cudaMemcpyHostToDevice), fname);
+    QB_CUDA(cudaMemsetAsync(ds->coef_f.p, 0, sizeof(double) * (size_t)(A * *ldb), ds->stream), fname);
+    QB_CUDA(cudaMemcpy2DAsync(ds->coef_f.p, sizeof(double) * *ldb, ds->coef_t.p, sizeof(double) * M, sizeof(double) * M,
+                              A, cudaMemcpyDeviceToDevice, ds->stream),
+            fname);
     ds->coef_f_version = ctx->mo_basis.coef_version;
   }
   *Bt = (const double*)ds->coef_f.p;

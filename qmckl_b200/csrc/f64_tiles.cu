@@ -345,6 +345,16 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   }
 }
 
+__global__ void __launch_bounds__(256)
+place_shells_kernel(const int n, const int nucl_num, const double* __restrict__ nucl_coord, F64Shell* __restrict__ sh) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const int m = sh[i].nucl;
+  sh[i].x = nucl_coord[m];
+  sh[i].y = nucl_coord[m + nucl_num];
+  sh[i].z = nucl_coord[m + 2 * nucl_num];
+}
+
 // ------------------------------------------------------------ contraction
 
 constexpr int BKT = 16;
@@ -774,6 +784,13 @@ F64Tiles f64_tiles_at(void* scratch, int64_t ntiles, int comps, int pts, int64_t
   t.klist = (int*)(t.ac + ld * (size_t)ao_num * (size_t)ntiles);
   t.kcount = t.klist + ao_num * ntiles;
   return t;
+}
+
+cudaError_t launch_place_shells(const DevTables& T, F64Shell* sh, cudaStream_t s) {
+  if (T.shell_num <= 0) return cudaSuccess;
+  place_shells_kernel<<<(unsigned)((T.shell_num + 255) / 256), 256, 0, s>>>(T.shell_num, T.nucl_num, T.nucl_coord, sh);
+  count_launch();
+  return cudaGetLastError();
 }
 
 cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const double* coord, int64_t cstride,

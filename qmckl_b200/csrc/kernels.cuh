@@ -142,6 +142,8 @@ struct F64Shell {
   double x, y, z, r2max, crange;
   int32_t a0, na, cb, ce, l, nucl;
 };
+// The nuclei's positions (T.nucl_coord) into the records of T.shell_num shells.
+cudaError_t launch_place_shells(const DevTables& T, F64Shell* sh, cudaStream_t s);
 // Compact tiles of pts = f64_tile_points points each, f64_tile_bytes per
 // tile: ac[tile][ao_num][comps * pts + 4] (the first kcount[tile] rows hold
 // the tile's live AOs klist[tile][.]).
