@@ -574,7 +574,11 @@ cudaError_t build_items(Batch* B) {
   B->n_items = (int)it.size();
   cudaError_t e = dalloc(B->items, sizeof(int4) * std::max<size_t>(it.size(), 1));
   if (e != cudaSuccess) return e;
-  if (!it.empty()) e = cudaMemcpy(B->items.p, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice);
+  // on the batch's stream, ahead of its launches; waits, since `it` goes
+  if (!it.empty()) {
+    e = cudaMemcpyAsync(B->items.p, it.data(), sizeof(int4) * it.size(), cudaMemcpyHostToDevice, B->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+  }
   return e;
 }
 

@@ -376,7 +376,10 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
-  std::vector<char> host_f64_sph;   // source of f64_sph's upload
+  // sources of uploads on the context's stream
+  std::vector<char> host_f64_sph;
+  std::vector<uint8_t> host_krec, host_kskip;
+  std::vector<float> host_env;
   AoSegments hess{};   // in f64_sph: the shell records and the segments of the AO Hessian
 };
 
@@ -855,7 +858,9 @@ qmckl_exit_code prepare_korder(qmckl_context context, DeviceState* ds, bool* ok)
                      ds->krec_nucl_version == ctx->nucleus.coord_version &&
                      ds->krec_cusp_version == ctx->mo_basis.cusp_version && ds->krec_cutoff == cutoff;
   if (!fresh) {
-    std::vector<uint8_t> h, ks;
+    std::vector<uint8_t>&h = ds->host_krec, &ks = ds->host_kskip;
+    h.clear();
+    ks.clear();
     std::vector<int64_t> perm;
     int rec = 0;
     // the largest record that keeps the VGL kernel within its shared memory
@@ -867,8 +872,9 @@ qmckl_exit_code prepare_korder(qmckl_context context, DeviceState* ds, bool* ok)
     const size_t kbytes = ks.size();
     rc = ensure(context, ds->kskip, kbytes, fname);
     if (rc != QMCKL_SUCCESS) return rc;
-    QB_CUDA(cudaMemcpy(ds->krec.p, h.data(), h.size(), cudaMemcpyHostToDevice), fname);
-    QB_CUDA(cudaMemcpy(ds->kskip.p, ks.data(), kbytes, cudaMemcpyHostToDevice), fname);
+    // on the context's stream, behind the kernels that read the tables before
+    QB_CUDA(cudaMemcpyAsync(ds->krec.p, h.data(), h.size(), cudaMemcpyHostToDevice, ds->stream), fname);
+    QB_CUDA(cudaMemcpyAsync(ds->kskip.p, ks.data(), kbytes, cudaMemcpyHostToDevice, ds->stream), fname);
     ds->rec_bytes = rec;
     ds->krec_basis_version = ctx->ao_basis.basis_version;
     ds->krec_nucl_version = ctx->nucleus.coord_version;
@@ -944,13 +950,15 @@ qmckl_exit_code prepare_mixed(qmckl_context context, DeviceState* ds) {
     ds->tc3_coef_version = ctx->mo_basis.coef_version;
   }
   if (ds->env_basis_version != ctx->ao_basis.basis_version || !ds->env.p) {
-    std::vector<float> env;
+    std::vector<float>& env = ds->host_env;
+    env.clear();
     float r0 = 0.f, il = 0.f;
     build_envelopes(ctx, env, r0, il);
     qmckl_exit_code rc = ensure(context, ds->env, sizeof(float) * std::max<size_t>(env.size(), 1), "qmckl_b200_mo_mixed");
     if (rc != QMCKL_SUCCESS) return rc;
     if (!env.empty())
-      QB_CUDA(cudaMemcpy(ds->env.p, env.data(), sizeof(float) * env.size(), cudaMemcpyHostToDevice), "qmckl_b200_mo_mixed");
+      QB_CUDA(cudaMemcpyAsync(ds->env.p, env.data(), sizeof(float) * env.size(), cudaMemcpyHostToDevice, ds->stream),
+              "qmckl_b200_mo_mixed");
     ds->env_r0 = r0;
     ds->env_inv_log2q = il;
     ds->env_basis_version = ctx->ao_basis.basis_version;

@@ -54,7 +54,8 @@ def _queue(ctx, call, c, w, out):
     ("ao_hessian", pq.FORM_FP64, "nuclei", 20), ("mo_vgl", pq.FORM_FP64, "nuclei", 20),
     ("mo_vgl", pq.FORM_FP64, "coefficients", 21), ("mo_vgl", pq.FORM_FP64, "coefficients", 20),
     ("adjoint", pq.FORM_FP64, "nuclei", 21), ("adjoint", pq.FORM_FP64, "coefficients", 21),
-    ("adjoint", pq.FORM_MIXED, "nuclei", 21), ("adjoint", pq.FORM_MIXED, "coefficients", 21)])
+    ("adjoint", pq.FORM_MIXED, "nuclei", 21), ("adjoint", pq.FORM_MIXED, "coefficients", 21),
+    ("mo_vgl", pq.FORM_MIXED, "nuclei", 20), ("mo_vgl", pq.FORM_MIXED, "coefficients", 21)])
 def test_queued_calls_keep_their_inputs(call, form, change, m):
     d, pts, geometries, coefs, w = _case(m)
     t = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")  # noqa: E731
@@ -86,7 +87,7 @@ def test_queued_calls_keep_their_inputs(call, form, change, m):
         pq.b200_synchronize(ctx)
     finally:
         pq.context_destroy(ctx)
-    if change == "nuclei":
+    if change == "nuclei" and (call, form) != ("mo_vgl", pq.FORM_MIXED):   # its tables are laid out anew
         assert busy   # a nuclear move does not wait for the stream
     for i in range(3):
         for a, b in zip(want[i], got[i]):
