@@ -159,7 +159,7 @@ cudaError_t launch_ao_hessian(const DevTables& T, const AoSegments& g, int64_t p
   const int max_shells = std::max(1, g.max_shells);
   const size_t smem = sizeof(double) * kHessRows * (size_t)(g.width + 2) + sizeof(double) * kHessRad * (size_t)max_shells +
                       sizeof(uint32_t) * 2 * (size_t)g.width + sizeof(int) * (size_t)max_shells;
-  cudaError_t e = cudaFuncSetAttribute(ao_hessian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(ao_hessian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - 1024);
   if (e != cudaSuccess) return e;
   const int64_t per_sm = std::min<int64_t>(12, std::max<int64_t>(1, (int64_t)(227 * 1024) / (int64_t)(smem + 2048)));
   const int64_t grid = std::min<int64_t>(point_num * g.nseg, 148 * per_sm);

@@ -584,8 +584,8 @@ cudaError_t build_items(Batch* B) {
 
 cudaError_t set_kernel_attrs() {
   // the most any batch takes: the attribute belongs to the kernel, not to this batch
-  cudaError_t e = cudaFuncSetAttribute(batch_mo_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_mo_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 232448);
+  cudaError_t e = cudaFuncSetAttribute(batch_mo_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(batch_mo_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   return e;
 }
 

@@ -807,8 +807,7 @@ cudaError_t launch_ao_tiles(const DevTables& T, int64_t P, int comps, const doub
                                 : (t.pts == 32 ? ao_tiles_kernel<1, 32, 4> : ao_tiles_kernel<1, 128, 4>))
                   : (comps == 5 ? ao_tiles_kernel<5, 32, 1>
                                 : (t.pts == 32 ? ao_tiles_kernel<1, 32, 1> : ao_tiles_kernel<1, 128, 1>));
-  cudaError_t e =
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(sm, 1));
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWindow * 2 * (int)sizeof(int));
   if (e != cudaSuccess) return e;
   // few tiles: several CTAs share one, so that its shells are spread over SMs
   // (not over windows: a window reads the counts that the one before wrote)

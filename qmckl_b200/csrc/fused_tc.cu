@@ -535,7 +535,7 @@ cudaError_t launch_fused(const DevTables& T, const CUtensorMap& tb, int64_t P, c
   if constexpr (PIECES == 3 && COMPS == 5)
     if (late_ns != 0u) kern = fused_mo_kernel<PIECES, COMPS, NACC, NST, true>;
   if (NACC == 2 && tplan == nullptr) return cudaErrorInvalidValue;   // the wide form needs a tile plan
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   const int64_t tiles = (P + PTS - 1) / PTS;
   double* tpts = nullptr;

@@ -80,6 +80,12 @@ __device__ __forceinline__ int pack_live_slots(const int32_t* __restrict__ slot_
 // cudaGetLastError() after the launch.
 // cusp_r (optional, [nucl]): the AOs that the cusp adjustment leaves out of
 // the MO sums are written as zero (the arrays then only feed the MO step).
+// A block's most shared memory.  A kernel whose dynamic shared memory differs
+// from call to call is opted in to all of it (less its static part), never to a
+// call's size: the attribute belongs to the kernel, and another thread's
+// smaller call could lower it between a call's opt-in and its launch.
+constexpr int kMaxSmem = 232448;
+
 cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const double* coord,
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s,
                               const double* cusp_r = nullptr);

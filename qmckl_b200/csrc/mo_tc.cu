@@ -807,7 +807,7 @@ cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int64_t M,
   const size_t stage = (size_t)PIECES * (BM * BK * 2 + (size_t)n_tile * BK * 2);
   const size_t smem = 1024 + STAGES * stage + (2 * STAGES + 1) * 8 + 16;
   auto kern = tc_gemm_kernel<PIECES, STAGES>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((M + BM - 1) / BM), (unsigned)n_tiles);
   kern<<<grid, kThreads, smem, s>>>(ta, tb, M, n_out, n_tile, kblocks, comps, scales, out, ldo, err);
@@ -1085,7 +1085,7 @@ cudaError_t tc_gemm_tn_split(const void* x, int64_t ldx, int64_t x_pstride, int6
   if (!make_map(&ty, y, b_num, rows, ldy, 3, y_pstride, BKR)) return cudaErrorInvalidValue;
   const size_t stage = (size_t)3 * ((BM / 64) * MN_BOX + (size_t)(n_tile / 64) * MN_BOX);
   const size_t smem = 1024 + kMnStages * stage + (2 * kMnStages + 1) * 8 + 16;
-  cudaError_t e = cudaFuncSetAttribute(tc_gemm_mn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(tc_gemm_mn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((a_num + BM - 1) / BM), (unsigned)n_tiles, (unsigned)splits);
   tc_gemm_mn_kernel<<<grid, kThreads, smem, s>>>(tx, ty, a_num, b_num, n_tile, kblocks, kps, part, err);
