@@ -90,6 +90,8 @@ __device__ __forceinline__ void adj_ao(const ShellRad& S, const double (&xp)[4],
   q[2] += S.R0 * sz + tz + Pz * u + S.Rd[2] * w + S.v[2] * vy + r1 * y2;
 }
 
+__device__ __forceinline__ double nan_d() { return __longlong_as_double(0x7ff8000000000000ll); }
+
 template <int L, int I>
 __device__ __forceinline__ void adj_shell(const ShellRad& S, const double (&xp)[4], const double (&yp)[4],
                                           const double (&zp)[4], const double* __restrict__ gr, int64_t ld, int tp,
@@ -142,6 +144,14 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
   const int e0 = (int)((int64_t)n * part / parts), e1 = (int)((int64_t)n * (part + 1) / parts);
   const F* gt = gc + (size_t)tile * kmax * LD + lane;
   double pq[3] = {0., 0., 0.}, nq[3] = {0., 0., 0.};
+  if (const unsigned int bad = adj.bad[tile]; bad != 0u && blockIdx.y == 0) {
+    // weights that are not finite meet zero AOs (rare): NaN for their points
+    // and for every nucleus
+    const double nan = nan_d();
+    if (warp == 0 && (bad >> lane & 1u)) pq[0] = pq[1] = pq[2] = nan;
+    if (grad_nucl != nullptr)
+      for (int i = threadIdx.x; i < 3 * T.nucl_num; i += 256) atomicAdd(&grad_nucl[i], nan);
+  }
   int nucl = -1;
   auto flush = [&]() {
     if (nucl >= 0 && grad_nucl != nullptr) {

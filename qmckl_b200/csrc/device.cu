@@ -1812,7 +1812,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->adj_wt, sizeof(uint16_t) * 3 * 160 * ctiles * ldw, fname);
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->order, order_bytes(chunk), fname);
   if (rc == QMCKL_SUCCESS && points)
-    rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 2), fname);
+    rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 3), fname);
   if (rc == QMCKL_SUCCESS && ds->tc_err.p == nullptr) {
     rc = ensure(context, ds->tc_err, sizeof(int), fname);
     if (rc == QMCKL_SUCCESS) QB_CUDA(cudaMemsetAsync(ds->tc_err.p, 0, sizeof(int), s), fname);
@@ -1827,6 +1827,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   t.klist = (int*)((uint8_t*)ds->f64_tiles.p + b_live);
   t.kcount = t.klist + ctiles * A;
   t.adj.nlive = t.kcount + ctiles;
+  t.adj.bad = (unsigned int*)(t.adj.nlive + ctiles);
   const F64Shell* sh = (const F64Shell*)ds->f64_sph.p;
   double lo[3], hi[3];
   nucleus_box(ctx, lo, hi);
@@ -1845,8 +1846,10 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
       perm = (int*)ds->order.p;
       QB_CUDA(point_order(cc, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(n), perm, s, n), fname);
     }
+    if (points)
+      QB_CUDA(launch_ao_tiles(ds->T, n, 5, cc, n, perm, 0, tiles, sh, cutoff, false, nullptr, t, s), fname);
     QB_CUDA(tc_split_weights(w, n, (int)M, perm, (int)ldw, d_grad_coef ? ds->adj_wp.p : nullptr,
-                             points ? ds->adj_wt.p : nullptr, s),
+                             points ? ds->adj_wt.p : nullptr, points ? t.adj.bad : nullptr, s),
             fname);
     if (d_grad_coef) {
       QB_CUDA(launch_ao_vgl_pieces(ds->T, n, cc, cutoff, false, buf, lda, rows * lda, s), fname);
@@ -1858,7 +1861,6 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
               fname);
     }
     if (points) {
-      QB_CUDA(launch_ao_tiles(ds->T, n, 5, cc, n, perm, 0, tiles, sh, cutoff, false, nullptr, t, s), fname);
       QB_CUDA(tc_pullback(ds->adj_wt.p, (int)ldw, tiles, (int)M, ds->adj_ct.p, A, t.klist, t.kcount, (float*)buf, err, s),
               fname);
       QB_CUDA(launch_tile_deriv(ds->T, n, cc, n, perm, 0, tiles, sh, cutoff, t.adj, buf, true, d_grad_nucl,
@@ -1919,6 +1921,7 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
   t.adj.live = (int2*)at;
   at += b_live * (size_t)chunk;
   t.adj.nlive = (int*)at;
+  t.adj.bad = (unsigned int*)(t.adj.nlive + chunk);
   at += b_n * (size_t)chunk;
   int* inv = (int*)at;
   t.adj.inv = d_grad_coef ? inv : nullptr;
@@ -1927,7 +1930,7 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
     const int64_t n = std::min(chunk, tiles - t0);
     if (d_grad_coef) QB_CUDA(cudaMemsetAsync(inv, 0xff, sizeof(int) * (size_t)(n * A), s), fname);
     QB_CUDA(launch_ao_tiles(ds->T, P, 5, d_coord, P, perm, t0, n, sh, cutoff, true, nullptr, t, s), fname);
-    QB_CUDA(launch_weight_tiles(P, t0, n, d_weight, M, perm, ws, ldw, s), fname);
+    QB_CUDA(launch_weight_tiles(P, t0, n, d_weight, M, perm, ws, ldw, t.adj.bad, s), fname);
     if (d_grad_coef) QB_CUDA(launch_adj_coef(n, A, M, t, ws, ldw, part, d_grad_coef, t0 > 0, s), fname);
     if (d_grad_nucl || d_grad_coord) {
       QB_CUDA(launch_adj_pullback(n, A, M, t, ws, ldw, Ct, ldc, s), fname);

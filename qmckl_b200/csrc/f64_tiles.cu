@@ -302,7 +302,10 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     }
     if (tid == 0) {
       kcount[tile] = k0 + nao;
-      if (adj.live != nullptr) adj.nlive[tile] = q0 + nlive;
+      if (adj.live != nullptr) {
+        adj.nlive[tile] = q0 + nlive;
+        adj.bad[tile] = 0u;
+      }
     }
   }
   if (ac == nullptr) return;   // the lists only
@@ -534,10 +537,12 @@ cudaError_t run_tile_gemm(int64_t P, int64_t tile0, int64_t ntiles, int64_t N, c
 constexpr int kAdjPts = 32, kAdjRows = 5 * kAdjPts, kAdjLd = kAdjRows + 4;   // tiles of 32 points
 
 // Loss weights in tile order: ws[tile][c * 32 + p][ldw] = w[perm point][c][.]
-// (zero past the MOs and past the points); a warp per row.
+// (zero past the MOs and past the points), and the tile's points with weights
+// that are not finite; a warp per row.
 __global__ void __launch_bounds__(256)
 weight_tiles_kernel(const int64_t P, const int64_t tile0, const int64_t rows, const double* __restrict__ w,
-                    const int64_t M, const int* __restrict__ perm, double* __restrict__ ws, const int64_t ldw) {
+                    const int64_t M, const int* __restrict__ perm, double* __restrict__ ws, const int64_t ldw,
+                    unsigned int* __restrict__ bad) {
   const int lane = threadIdx.x & 31;
   for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (int64_t)gridDim.x * 8) {
     const int64_t tile = r / kAdjRows;
@@ -546,7 +551,13 @@ weight_tiles_kernel(const int64_t P, const int64_t tile0, const int64_t rows, co
     double* o = ws + r * ldw;
     if (q < P) {
       const double* src = w + ((perm ? (int64_t)perm[q] : q) * 5 + c) * M;
-      for (int64_t n = lane; n < ldw; n += 32) o[n] = n < M ? src[n] : 0.0;
+      bool off = false;
+      for (int64_t n = lane; n < ldw; n += 32) {
+        const double x = n < M ? src[n] : 0.0;
+        off = off || !isfinite(x);
+        o[n] = x;
+      }
+      if (__any_sync(0xffffffffu, off) && lane == 0) atomicOr(&bad[tile], 1u << (pos % kAdjPts));
     } else {
       for (int64_t n = lane; n < ldw; n += 32) o[n] = 0.0;
     }
@@ -681,13 +692,14 @@ adj_gemm_kernel(double* __restrict__ ac, const int* __restrict__ klist, const in
 }
 
 // grad[n][k] (+)= sum over the tiles, in order, of part[tile][inv[tile][k]][n]
-// (inv < 0: AO k is not in the tile's list).  A warp per AO and 64 MOs, with
+// (inv < 0: AO k is not in the tile's list, and only a weight that is not
+// finite, times that zero, adds to the sum).  A warp per AO and 64 MOs, with
 // the list positions of the next 32 tiles in flight beside eight rows; 16 AOs
 // x 64 MOs per CTA, transposed through shared memory.
 __global__ void __launch_bounds__(512)
-sum_tiles_kernel(const double* __restrict__ part, const int* __restrict__ inv, const int64_t ntiles, const int64_t kmax,
-                 const int64_t A, const int64_t M, const int64_t ldw, double* __restrict__ grad,
-                 const bool accumulate) {
+sum_tiles_kernel(const double* __restrict__ part, const int* __restrict__ inv, const unsigned int* __restrict__ bad,
+                 const double* __restrict__ ws, const int64_t ntiles, const int64_t kmax, const int64_t A,
+                 const int64_t M, const int64_t ldw, double* __restrict__ grad, const bool accumulate) {
   __shared__ double tr[64][17];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t k = (int64_t)blockIdx.x * 16 + warp, n = (int64_t)blockIdx.y * 64 + 2 * lane;
@@ -697,6 +709,18 @@ sum_tiles_kernel(const double* __restrict__ part, const int* __restrict__ inv, c
     for (int64_t t0 = 0; t0 < ntiles; t0 += 32) {
       const int at = next;
       next = t0 + 32 + lane < ntiles ? inv[(t0 + 32 + lane) * kmax + k] : -1;
+      const unsigned int pts = at < 0 && t0 + lane < ntiles ? bad[t0 + lane] : 0u;
+      for (unsigned int q = __ballot_sync(0xffffffffu, pts != 0u); q; q &= q - 1) {   // rare
+        const int b = __ffs(q) - 1;
+        for (unsigned int p = __shfl_sync(0xffffffffu, pts, b); p; p &= p - 1)
+          for (int c = 0; c < 5; ++c) {
+            const double* row = ws + ((size_t)(t0 + b) * kAdjRows + c * kAdjPts + __ffs(p) - 1) * ldw;
+            if (n < ldw) {
+              v.x += 0.0 * row[n];
+              v.y += 0.0 * row[n + 1];
+            }
+          }
+      }
       unsigned int m = __ballot_sync(0xffffffffu, at >= 0);
       while (m) {
         double2 x[8];
@@ -845,11 +869,11 @@ cudaError_t launch_tile_gemm(int64_t P, int comps, int64_t tile0, int64_t ntiles
 }
 
 cudaError_t launch_weight_tiles(int64_t P, int64_t tile0, int64_t ntiles, const double* w, int64_t M, const int* perm,
-                                double* ws, int64_t ldw, cudaStream_t s) {
+                                double* ws, int64_t ldw, unsigned int* bad, cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
   const int64_t rows = ntiles * kAdjRows;
   const unsigned grid = (unsigned)std::min<int64_t>((rows + 7) / 8, 148 * 32);
-  weight_tiles_kernel<<<grid, 256, 0, s>>>(P, tile0, rows, w, M, perm, ws, ldw);
+  weight_tiles_kernel<<<grid, 256, 0, s>>>(P, tile0, rows, w, M, perm, ws, ldw, bad);
   count_launch();
   return cudaGetLastError();
 }
@@ -861,7 +885,8 @@ cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64
   cudaError_t e = pick_adj_gemm<true>(ntiles, ao_num, M, t, ws, ldw, nullptr, 0, part, s);
   if (e != cudaSuccess) return e;
   dim3 grid((unsigned)((ao_num + 15) / 16), (unsigned)((M + 63) / 64));
-  sum_tiles_kernel<<<grid, 512, 0, s>>>(part, t.adj.inv, ntiles, ao_num, ao_num, M, ldw, grad, accumulate);
+  sum_tiles_kernel<<<grid, 512, 0, s>>>(part, t.adj.inv, t.adj.bad, ws, ntiles, ao_num, ao_num, M, ldw, grad,
+                                         accumulate);
   count_launch();
   return cudaGetLastError();
 }

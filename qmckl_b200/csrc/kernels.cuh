@@ -155,11 +155,16 @@ cudaError_t launch_place_shells(const DevTables& T, F64Shell* sh, cudaStream_t s
 // the tile's live AOs klist[tile][.]).
 // For the adjoint also: inv[tile][ao_num], the list position of each AO
 // (preset to -1; may be null); live[tile][shell_num], the live shells (shell,
-// first list position), nlive[tile] of them.
+// first list position), nlive[tile] of them; bad[tile], the points of the tile
+// (bits) with a loss weight that is not finite, set by the kernels that lay
+// out the weights after launch_ao_tiles has cleared it.  Such a weight times
+// an AO that is exactly zero is a NaN of dL/dC, dL/dR and dL/dr, also where the
+// AO is in no list.
 struct AdjTables {
   int* inv;
   int2* live;
   int* nlive;
+  unsigned int* bad;
 };
 struct F64Tiles {
   int pts;
@@ -185,9 +190,9 @@ cudaError_t launch_tile_gemm(int64_t P, int comps, int64_t tile0, int64_t ntiles
 
 // FP64 adjoint of the MO VGL over compact VGL tiles (f64_tiles.cu,
 // adjoint.cu) with their AdjTables.
-// Weights in tile order: ws[tile][c * 32 + p][ldw], ldw even.
+// Weights in tile order: ws[tile][c * 32 + p][ldw], ldw even; bad as AdjTables.
 cudaError_t launch_weight_tiles(int64_t P, int64_t tile0, int64_t ntiles, const double* w, int64_t M, const int* perm,
-                                double* ws, int64_t ldw, cudaStream_t s);
+                                double* ws, int64_t ldw, unsigned int* bad, cudaStream_t s);
 // grad[mo][ao] (+)= AO^T W of the tiles; part [ntiles][ao_num][ldw].
 cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws, int64_t ldw,
                             double* part, double* grad, bool accumulate, cudaStream_t s);

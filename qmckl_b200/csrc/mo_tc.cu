@@ -589,11 +589,13 @@ tc_pullback_kernel(const __grid_constant__ CUtensorMap tmW, const uint16_t* __re
 
 // Weight rows w[(p, c)][M] as 3 bfloat16 pieces, in the points' order
 // (rows, for dL/dC) and in tile order (tiled [tile][c * 32 + p], zero past the
-// points; for the pulled-back weights).  Either may be null.  A thread per 8
-// columns of a tile-order row.
+// points; for the pulled-back weights), and the points of each tile whose
+// weights the pieces do not hold (not finite, or beyond their range).  Any of
+// the three may be null.  A thread per 8 columns of a tile-order row.
 __global__ void __launch_bounds__(256)
 split_weights_kernel(const double* __restrict__ w, const int64_t P, const int M, const int* __restrict__ perm,
-                     const int64_t tiles, const int ldw, uint16_t* __restrict__ rows, uint16_t* __restrict__ tiled) {
+                     const int64_t tiles, const int ldw, uint16_t* __restrict__ rows, uint16_t* __restrict__ tiled,
+                     unsigned int* __restrict__ bad) {
   const int cw = ldw / 8;
   const int64_t total = tiles * kPbCols * cw, rstride = P * 5 * ldw, tstride = tiles * kPbCols * ldw;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -605,10 +607,13 @@ split_weights_kernel(const double* __restrict__ w, const int64_t P, const int M,
     uint16_t pc[3][8];
     int64_t row = -1;
     if (q < P) row = (perm ? (int64_t)perm[q] : q) * 5 + c;
+    bool off = false;
 #pragma unroll
     for (int h = 0; h < 8; ++h) {
       uint16_t o[3];
-      split3_bf16(row >= 0 && c8 + h < M ? w[row * M + c8 + h] : 0.0, o);
+      const double x = row >= 0 && c8 + h < M ? w[row * M + c8 + h] : 0.0;
+      split3_bf16(x, o);
+      off = off || (o[0] & 0x7f80u) == 0x7f80u;   // infinite or NaN
 #pragma unroll
       for (int k = 0; k < 3; ++k) pc[k][h] = o[k];
     }
@@ -618,6 +623,7 @@ split_weights_kernel(const double* __restrict__ w, const int64_t P, const int M,
       if (rows != nullptr && row >= 0) *reinterpret_cast<uint4*>(rows + k * rstride + row * ldw + c8) = v;
       if (tiled != nullptr) *reinterpret_cast<uint4*>(tiled + k * tstride + tr * ldw + c8) = v;
     }
+    if (off && bad != nullptr) atomicOr(&bad[tile], 1u << (pos & 31));
   }
 }
 
@@ -1094,13 +1100,13 @@ cudaError_t tc_gemm_tn_split(const void* x, int64_t ldx, int64_t x_pstride, int6
 }
 
 cudaError_t tc_split_weights(const double* w, int64_t P, int M, const int* perm, int ldw, void* rows, void* tiled,
-                             cudaStream_t s) {
+                             unsigned int* bad, cudaStream_t s) {
   if (P <= 0) return cudaSuccess;
   if (ldw < M || ldw % 8 != 0) return cudaErrorInvalidValue;
   const int64_t tiles = (P + 31) / 32;
   const int64_t total = tiles * kPbCols * (ldw / 8);
   const int grid = (int)std::min<int64_t>((total + 255) / 256, (int64_t)sm_count() * 16);
-  split_weights_kernel<<<grid, 256, 0, s>>>(w, P, M, perm, tiles, ldw, (uint16_t*)rows, (uint16_t*)tiled);
+  split_weights_kernel<<<grid, 256, 0, s>>>(w, P, M, perm, tiles, ldw, (uint16_t*)rows, (uint16_t*)tiled, bad);
   count_launch();
   return cudaGetLastError();
 }

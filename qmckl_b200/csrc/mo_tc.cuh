@@ -127,7 +127,8 @@ cudaError_t tc_run_scratch(const DevTables& T, const TcPlan& plan, int64_t point
 //   tc_split_weights : FP64 weights w[(p, c)][M] -> pieces of rows [3][5 P][ldw]
 //                   and of tile-order rows [3][tiles * 160][ldw] (tiles of 32
 //                   points in the order perm, row c * 32 + p, zero past the
-//                   points); either may be null
+//                   points), and bad[tile] |= the points (bits) whose weights are
+//                   not finite as pieces; any of the three may be null
 //   tc_pullback   : gc[tile][m][160] (FP32) = sum over the MOs of
 //                   C[klist[tile][m]][mo] * W[tile][pos][mo], m < kcount[tile],
 //                   from tile-order weight pieces and the pieces ct [3][ao][ldw]
@@ -140,7 +141,7 @@ cudaError_t tc_gemm_tn_split(const void* x, int64_t ldx, int64_t x_pstride, int6
                              int64_t y_pstride, int b_num, int64_t rows, int kps, double* part, int* err,
                              cudaStream_t s);
 cudaError_t tc_split_weights(const double* w, int64_t P, int M, const int* perm, int ldw, void* rows, void* tiled,
-                             cudaStream_t s);
+                             unsigned int* bad, cudaStream_t s);
 cudaError_t tc_pullback(const void* tiled, int ldw, int64_t tiles, int M, const void* ct, int64_t ao_num,
                         const int* klist, const int* kcount, float* gc, int* err, cudaStream_t s);
 
