@@ -31,6 +31,8 @@
 namespace qb {
 namespace {
 
+constexpr int64_t kDerivCtas = 6 * 148;   // the derivative kernel shares tiles out below this many
+
 // One AO of the FP64 adjoint, exponents known at compile time: with the
 // pulled-back weights (G0, g = G1..G3, G4) and P's derivatives,
 //   q = R (G0 dP + HP g + G4 d lap P) + dP (g . dR + G4 lap R)
@@ -112,8 +114,10 @@ __device__ __forceinline__ void adj_shell(const ShellRad& S, const double (&xp)[
 // there are few tiles), lanes are points, the warps take contiguous runs of
 // the tile's live shells.  The pulled-back weights G of the tile are read
 // along the points; q of a point is kept in the lane over the warp's shells
-// and summed over the warps in order (grad_coord is stored by a CTA that owns
-// its points, added to by one that shares them), q of a nucleus is summed
+// and summed over the warps in order and, by sum_shares_kernel, over the
+// tile's CTAs in order, so that grad_coord is the same in every run (on 313
+// tiles in three parts a sum by the tile's last CTA, which waits for its
+// atomics, took 96 us against 84); q of a nucleus is summed
 // over the run of its shells and the lanes and added by one atomic.  0.13 ms on 20,352
 // points of the 2000-AO molecule, bound by the latency of its FP64 chains (a
 // warp per point over all AOs, with the AO derivatives formed first, 1.43 ms).
@@ -244,15 +248,29 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
 #pragma unroll
   for (int d = 0; d < 3; ++d) sq[warp][d][lane] = pq[d];
   __syncthreads();
-  if (warp < 3 && in) {
+  if (warp < 3) {
     double s = 0.0;
 #pragma unroll
     for (int w = 0; w < NW; ++w) s += sq[w][warp][lane];
-    if (gridDim.y == 1)
+    if (gridDim.y > 1)
+      adj.share[((size_t)tile * gridDim.y + blockIdx.y) * 96 + warp * 32 + lane] = s;
+    else if (in)
       grad_coord[pi + warp * gstride] = s;
-    else
-      atomicAdd(&grad_coord[pi + warp * gstride], s);
   }
+}
+
+// grad_coord of tiles shared by `parts` CTAs: their shares summed in order.
+__global__ void __launch_bounds__(192)
+sum_shares_kernel(const int64_t P, const int* __restrict__ perm, const int64_t tile0, const int64_t ntiles,
+                  const int parts, const double* __restrict__ share, double* __restrict__ grad_coord,
+                  const int64_t gstride) {
+  const int64_t i = (int64_t)blockIdx.x * 192 + threadIdx.x, tile = i / 96;
+  const int at = (int)(i - tile * 96);
+  const int64_t qi = (tile0 + tile) * 32 + (at & 31);
+  if (tile >= ntiles || qi >= P) return;
+  double s = 0.0;
+  for (int r = 0; r < parts; ++r) s += share[((size_t)tile * parts + r) * 96 + at];
+  grad_coord[(perm ? (int64_t)perm[qi] : qi) + (at >> 5) * gstride] = s;
 }
 
 // Orbital forces (derivatives with respect to the nuclear coordinates; the
@@ -326,16 +344,31 @@ cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, con
   return cudaGetLastError();
 }
 
+static int deriv_parts(int64_t ntiles) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(8, (kDerivCtas + ntiles - 1) / ntiles));
+}
+
+size_t deriv_share_bytes(int64_t ntiles) {
+  // CTAs that share tiles, for any count up to ntiles: 8 per tile, and below
+  // kDerivCtas + the tiles
+  return sizeof(double) * 96 * (size_t)std::min<int64_t>(8 * ntiles, 2 * kDerivCtas);
+}
+
 cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,
                               int64_t tile0, int64_t ntiles, const F64Shell* sh, double cutoff, const AdjTables& adj,
                               const void* g, bool mixed, double* grad_nucl, double* grad_coord, int64_t gstride,
                               cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
-  const int parts = (int)std::max<int64_t>(1, std::min<int64_t>(8, (6 * 148 + ntiles - 1) / ntiles));
+  const int parts = deriv_parts(ntiles);
   auto k = mixed ? tile_deriv_kernel<true> : tile_deriv_kernel<false>;
   k<<<dim3((unsigned)ntiles, (unsigned)parts), 256, 0, s>>>(T, P, coord, cstride, perm, tile0, sh, cutoff, g, adj, T.ao_num,
                                                             grad_nucl, grad_coord, gstride);
   count_launch();
+  if (grad_coord != nullptr && parts > 1) {
+    sum_shares_kernel<<<(unsigned)((ntiles + 1) / 2), 192, 0, s>>>(P, perm, tile0, ntiles, parts, adj.share, grad_coord,
+                                                                   gstride);
+    count_launch();
+  }
   return cudaGetLastError();
 }
 

@@ -1805,14 +1805,15 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   const int splits = tc_tn_splits(5 * chunk, kps);
   const int64_t ctiles = (chunk + 31) / 32;
   const size_t buf_bytes = std::max<size_t>((size_t)(30 * lda) * (size_t)chunk, sizeof(float) * 160 * (size_t)A * (size_t)ctiles);
-  const size_t b_live = (sizeof(int2) * (size_t)S * (size_t)ctiles + 15) / 16 * 16;
+  const size_t b_live = (sizeof(int2) * (size_t)S * (size_t)ctiles + 15) / 16 * 16, b_share = deriv_share_bytes(ctiles);
   rc = ensure(context, ds->adj_buf, buf_bytes, fname);
   if (rc == QMCKL_SUCCESS && nchunks > 1) rc = ensure(context, ds->adj_coord, sizeof(double) * 3 * chunk, fname);
   if (rc == QMCKL_SUCCESS && d_grad_coef) rc = ensure(context, ds->adj_wp, sizeof(uint16_t) * 3 * 5 * chunk * ldw, fname);
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->adj_wt, sizeof(uint16_t) * 3 * 160 * ctiles * ldw, fname);
   if (rc == QMCKL_SUCCESS && points) rc = ensure(context, ds->order, order_bytes(chunk), fname);
   if (rc == QMCKL_SUCCESS && points)
-    rc = ensure(context, ds->f64_tiles, b_live + sizeof(int) * (size_t)ctiles * (size_t)(A + 3), fname);
+    rc = ensure(context, ds->f64_tiles,
+                b_live + b_share + sizeof(int) * (size_t)ctiles * (size_t)(A + 3), fname);
   if (rc == QMCKL_SUCCESS && ds->tc_err.p == nullptr) {
     rc = ensure(context, ds->tc_err, sizeof(int), fname);
     if (rc == QMCKL_SUCCESS) QB_CUDA(cudaMemsetAsync(ds->tc_err.p, 0, sizeof(int), s), fname);
@@ -1824,7 +1825,8 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   F64Tiles t{};
   t.pts = 32;
   t.adj.live = (int2*)ds->f64_tiles.p;
-  t.klist = (int*)((uint8_t*)ds->f64_tiles.p + b_live);
+  t.adj.share = (double*)((uint8_t*)ds->f64_tiles.p + b_live);
+  t.klist = (int*)((uint8_t*)ds->f64_tiles.p + b_live + b_share);
   t.kcount = t.klist + ctiles * A;
   t.adj.nlive = t.kcount + ctiles;
   t.adj.bad = (unsigned int*)(t.adj.nlive + ctiles);
@@ -1856,7 +1858,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
       QB_CUDA(tc_gemm_tn_split(buf, lda, rows * lda, A, ds->adj_wp.p, ldw, rows * ldw, (int)M, rows, kps,
                                (double*)ds->adj_part.p, err, s),
               fname);
-      QB_CUDA(launch_add_transposed((const double*)ds->adj_part.p, tc_tn_splits(rows, kps), A, M, d_grad_coef, true,
+      QB_CUDA(launch_add_transposed((const double*)ds->adj_part.p, tc_tn_splits(rows, kps), A, M, d_grad_coef, p0 > 0,
                                     s),
               fname);
     }
@@ -1902,7 +1904,7 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
   const int64_t chunks = (tiles + most - 1) / most;
   const int64_t chunk = (tiles + chunks - 1) / chunks;
   rc = ensure(context, ds->order, order_bytes(P), fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, per_tile * (size_t)chunk, fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, per_tile * (size_t)chunk + deriv_share_bytes(chunk), fname);
   if (rc != QMCKL_SUCCESS) return rc;
   int* perm = (int*)ds->order.p;
   double lo[3], hi[3];
@@ -1923,6 +1925,8 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
   t.adj.nlive = (int*)at;
   t.adj.bad = (unsigned int*)(t.adj.nlive + chunk);
   at += b_n * (size_t)chunk;
+  t.adj.share = (double*)at;
+  at += deriv_share_bytes(chunk);
   int* inv = (int*)at;
   t.adj.inv = d_grad_coef ? inv : nullptr;
   const F64Shell* sh = (const F64Shell*)ds->f64_sph.p;
@@ -1961,9 +1965,9 @@ qmckl_exit_code qmckl_b200_mo_vgl_adjoint_device(qmckl_context context, const in
   const int64_t P = point_num, A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num, N = ctx->nucleus.num;
   const bool mixed = use_mixed(ctx) || ctx->precision <= 23;
   cudaStream_t s = ds->stream;
-  if (d_grad_coef) QB_CUDA(cudaMemsetAsync(d_grad_coef, 0, sizeof(double) * M * A, s), fname);
+  // dL/dR is added up; dL/dC and dL/dr are stored where there are points
   if (d_grad_nucl) QB_CUDA(cudaMemsetAsync(d_grad_nucl, 0, sizeof(double) * 3 * N, s), fname);
-  if (d_grad_coord) QB_CUDA(cudaMemsetAsync(d_grad_coord, 0, sizeof(double) * 3 * P, s), fname);
+  if (d_grad_coef && P == 0) QB_CUDA(cudaMemsetAsync(d_grad_coef, 0, sizeof(double) * M * A, s), fname);
   if (P == 0 || (!d_grad_coef && !d_grad_nucl && !d_grad_coord)) return QMCKL_SUCCESS;
   if (mixed) return adjoint_mixed(context, ds, P, d_coord, d_weight, d_grad_coef, d_grad_nucl, d_grad_coord);
   return adjoint_f64(context, ds, P, d_coord, d_weight, d_grad_coef, d_grad_nucl, d_grad_coord);

@@ -159,13 +159,16 @@ cudaError_t launch_place_shells(const DevTables& T, F64Shell* sh, cudaStream_t s
 // (bits) with a loss weight that is not finite, set by the kernels that lay
 // out the weights after launch_ao_tiles has cleared it.  Such a weight times
 // an AO that is exactly zero is a NaN of dL/dC, dL/dR and dL/dr, also where the
-// AO is in no list.
+// AO is in no list.  share: deriv_share_bytes, the shares of dL/dr of the CTAs
+// that share a tile.
 struct AdjTables {
   int* inv;
   int2* live;
   int* nlive;
   unsigned int* bad;
+  double* share;
 };
+size_t deriv_share_bytes(int64_t ntiles);
 struct F64Tiles {
   int pts;
   double* ac;
@@ -200,7 +203,7 @@ cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64
 // with ldc even, zero past the MOs).
 cudaError_t launch_adj_pullback(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws,
                                 int64_t ldw, const double* Ct, int64_t ldc, cudaStream_t s);
-// grad_nucl [nucl][3] -= and grad_coord [3][gstride] (zeroed before) +=, either
+// grad_nucl [nucl][3] -= and grad_coord [3][gstride] =, either
 // may be null, from the pulled-back weights g of the tiles: FP64
 // [tile][ao_num][164], or (mixed) FP32 [tile][ao_num][160] with FP32
 // exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic.
