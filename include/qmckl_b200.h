@@ -207,6 +207,13 @@ qmckl_exit_code qmckl_b200_get_fused_plan(const int64_t ao_num, const int64_t mo
  * starts.  The results must not change. */
 qmckl_exit_code qmckl_b200_inject_late_warps(const int64_t ns);
 
+/* Test hook: bound the scratch of this context's chunked evaluations (FP64 MO
+ * VGL and value, the adjoint of both forms) to about `bytes` instead of their
+ * 2 to 4 GiB, so that few points already take several chunks (the smallest
+ * chunk is one tile of points; 0 = their own bound).  The results must not
+ * change beyond the order of their sums. */
+qmckl_exit_code qmckl_b200_set_scratch_limit(qmckl_context context, const int64_t bytes);
+
 /* Number of kernels this library launched since the process started. */
 int64_t qmckl_b200_kernel_launch_count(void);
 

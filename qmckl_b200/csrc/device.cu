@@ -376,6 +376,7 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
+  int64_t scratch_limit = 0;   // test hook: bound of the chunked evaluations' scratch (0: theirs)
   // sources of uploads on the context's stream
   std::vector<char> host_f64_sph;
   std::vector<uint8_t> host_krec, host_kskip;
@@ -790,6 +791,8 @@ qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
 size_t perm_bytes(int64_t P) { return (sizeof(int) * (size_t)P + 255) / 256 * 256; }
 size_t order_bytes(int64_t P) { return perm_bytes(P) + (point_order_bytes(P) + 255) / 256 * 256; }
 
+int64_t scratch_budget(const DeviceState* ds, int64_t bytes) { return ds->scratch_limit > 0 ? ds->scratch_limit : bytes; }
+
 // Box of the nuclei, widened by 4 bohr: the grid of the spatial point order.
 void nucleus_box(const Context* ctx, double* lo, double* hi) {
   const int64_t N = ctx->nucleus.num;
@@ -1011,7 +1014,7 @@ qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, in
   if (rc != QMCKL_SUCCESS) return rc;
   const int pts = f64_tile_points(comps, P);
   const int64_t tiles = (P + pts - 1) / pts;
-  const int64_t budget = (int64_t)4 << 30;
+  const int64_t budget = scratch_budget(ds, (int64_t)4 << 30);
   const int64_t most = std::max<int64_t>(1, budget / (int64_t)f64_tile_bytes(comps, pts, A));
   const int64_t chunks = (tiles + most - 1) / most;
   const int64_t chunk = (tiles + chunks - 1) / chunks;
@@ -1634,6 +1637,16 @@ qmckl_exit_code qmckl_b200_get_fused_plan(const int64_t ao_num, const int64_t mo
   return QMCKL_SUCCESS;
 }
 
+qmckl_exit_code qmckl_b200_set_scratch_limit(qmckl_context context, const int64_t bytes) {
+  if (qmckl_context_check(context) == QMCKL_NULL_CONTEXT) return QMCKL_INVALID_CONTEXT;
+  if (bytes < 0)
+    return qmckl_failwith(context, QMCKL_INVALID_ARG_2, "qmckl_b200_set_scratch_limit", "bytes must not be negative");
+  qmckl_exit_code rc = dev_attach(context);
+  if (rc != QMCKL_SUCCESS) return rc;
+  state(context)->scratch_limit = bytes;
+  return QMCKL_SUCCESS;
+}
+
 qmckl_exit_code qmckl_b200_inject_late_warps(const int64_t ns) {
   if (ns < 0 || ns > 10000000) return QMCKL_INVALID_ARG_1;
   return tc_set_late_warps((unsigned int)ns) == cudaSuccess ? QMCKL_SUCCESS : QMCKL_FAILURE;
@@ -1797,7 +1810,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
     ds->adj_ct_version = ctx->mo_basis.coef_version;
   }
   const bool points = d_grad_nucl || d_grad_coord;
-  const int64_t budget = (int64_t)2 << 30;
+  const int64_t budget = scratch_budget(ds, (int64_t)2 << 30);
   const int64_t row_bytes = std::max<int64_t>(20 * A, 30 * lda);   // G (FP32) or the AO pieces, per point
   const int64_t max_chunk = std::min<int64_t>(P, std::max<int64_t>(64, budget / row_bytes));
   const int64_t nchunks = (P + max_chunk - 1) / max_chunk;
@@ -1899,7 +1912,7 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
                b_inv = (sizeof(int) * (size_t)A + 15) / 16 * 16, b_n = 16, b_w = sizeof(double) * 5 * (size_t)pts * (size_t)ldw,
                b_part = d_grad_coef ? sizeof(double) * (size_t)A * (size_t)ldw : 0;
   const size_t per_tile = b_ao + b_live + b_inv + b_n + b_w + b_part;
-  const int64_t budget = (int64_t)4 << 30;
+  const int64_t budget = scratch_budget(ds, (int64_t)4 << 30);
   const int64_t most = std::max<int64_t>(1, budget / (int64_t)per_tile);
   const int64_t chunks = (tiles + most - 1) / most;
   const int64_t chunk = (tiles + chunks - 1) / chunks;

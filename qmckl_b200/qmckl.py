@@ -509,6 +509,10 @@ def b200_get_fused_plan(ao_num, mo_num, pieces=3):
     return tuple(x.value for x in v)
 
 
+def b200_set_scratch_limit(ctx, nbytes):
+    _call("qmckl_b200_set_scratch_limit", ctx, C.c_int64(nbytes))
+
+
 def b200_inject_late_warps(ns):
     f = lib().qmckl_b200_inject_late_warps
     f.restype = C.c_int32
