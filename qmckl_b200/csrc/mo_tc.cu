@@ -604,7 +604,7 @@ split_weights_kernel(const double* __restrict__ w, const int64_t P, const int M,
     const int64_t tile = tr / kPbCols;
     const int pos = (int)(tr - tile * kPbCols), c = pos >> 5;
     const int64_t q = tile * 32 + (pos & 31);
-    uint16_t pc[3][8];
+    __align__(16) uint16_t pc[3][8];   // stored 16 bytes at a time
     int64_t row = -1;
     if (q < P) row = (perm ? (int64_t)perm[q] : q) * 5 + c;
     bool off = false;
