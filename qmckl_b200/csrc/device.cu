@@ -376,6 +376,7 @@ struct DeviceState {
   double f64_sph_cutoff = -1.0;
   uint64_t coef_f_version = ~0ull;
   DevBuf f64_sph, coef_f, f64_tiles;
+  int64_t tile_room = 0;       // what f64_tiles got where the device had no more (0: never short)
   int64_t scratch_limit = 0;   // test hook: bound of the chunked evaluations' scratch (0: theirs)
   // sources of uploads on the context's stream
   std::vector<char> host_f64_sph;
@@ -793,6 +794,28 @@ size_t order_bytes(int64_t P) { return perm_bytes(P) + (point_order_bytes(P) + 2
 
 int64_t scratch_budget(const DeviceState* ds, int64_t bytes) { return ds->scratch_limit > 0 ? ds->scratch_limit : bytes; }
 
+// The FP64 tiles' scratch for `chunk` of them, `tile` bytes each, and `more`.
+// Where the device has no room for it: half as many tiles (one at least), for
+// this context's later calls as well.
+qmckl_exit_code ensure_tiles(qmckl_context context, DeviceState* ds, size_t tile, size_t more, int64_t& chunk,
+                             const char* where) {
+  DevBuf& b = ds->f64_tiles;
+  if (ds->tile_room > 0) chunk = std::min(chunk, std::max<int64_t>(1, ds->tile_room / (int64_t)tile));
+  while (chunk > 1 && (b.p == nullptr || b.cap < tile * (size_t)chunk + more)) {
+    if (alloc_should_fail()) return qmckl_failwith(context, QMCKL_ALLOCATION_FAILED, where, "device allocation");
+    release(b);
+    if (cudaMalloc(&b.p, tile * (size_t)chunk + more) == cudaSuccess) {
+      b.cap = tile * (size_t)chunk + more;
+      return QMCKL_SUCCESS;
+    }
+    cudaGetLastError();
+    b.p = nullptr;
+    chunk = (chunk + 1) / 2;
+    ds->tile_room = (int64_t)tile * chunk;
+  }
+  return ensure(context, b, tile * (size_t)chunk + more, where);
+}
+
 // Box of the nuclei, widened by 4 bohr: the grid of the spatial point order.
 void nucleus_box(const Context* ctx, double* lo, double* hi) {
   const int64_t N = ctx->nucleus.num;
@@ -1000,7 +1023,8 @@ qmckl_exit_code coef_even(qmckl_context context, DeviceState* ds, const double**
 // spatial tiles, per tile only the AOs of the shells that reach one of its
 // points, produced compactly and summed in the basis order (f64_tiles.cu).
 // The AO array is not formed.  cr: cusp radii or null.  Tiles go in chunks
-// that bound the scratch to about 4 GiB (one tile at least).
+// that bound the scratch to about 4 GiB, less where the device has no room (one
+// tile at least).
 qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, int comps, const double* coord,
                            const double* cr, double* out) {
   const char* fname = "qmckl_b200_mo_fp64";
@@ -1017,9 +1041,9 @@ qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, in
   const int64_t budget = scratch_budget(ds, (int64_t)4 << 30);
   const int64_t most = std::max<int64_t>(1, budget / (int64_t)f64_tile_bytes(comps, pts, A));
   const int64_t chunks = (tiles + most - 1) / most;
-  const int64_t chunk = (tiles + chunks - 1) / chunks;
+  int64_t chunk = (tiles + chunks - 1) / chunks;
   rc = ensure(context, ds->order, order_bytes(P), fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, f64_tile_bytes(comps, pts, A) * (size_t)chunk, fname);
+  if (rc == QMCKL_SUCCESS) rc = ensure_tiles(context, ds, f64_tile_bytes(comps, pts, A), 0, chunk, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   int* perm = (int*)ds->order.p;
   double lo[3], hi[3];
@@ -1915,9 +1939,10 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
   const int64_t budget = scratch_budget(ds, (int64_t)4 << 30);
   const int64_t most = std::max<int64_t>(1, budget / (int64_t)per_tile);
   const int64_t chunks = (tiles + most - 1) / most;
-  const int64_t chunk = (tiles + chunks - 1) / chunks;
+  int64_t chunk = (tiles + chunks - 1) / chunks;
   rc = ensure(context, ds->order, order_bytes(P), fname);
-  if (rc == QMCKL_SUCCESS) rc = ensure(context, ds->f64_tiles, per_tile * (size_t)chunk + deriv_share_bytes(chunk), fname);
+  if (rc == QMCKL_SUCCESS)
+    rc = ensure_tiles(context, ds, per_tile, deriv_share_bytes(chunk), chunk, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   int* perm = (int*)ds->order.p;
   double lo[3], hi[3];
