@@ -8,13 +8,17 @@
 // every sum over tiles, is the same in every run.
 //
 // The sort is bound by launches and load latencies, not by its bytes.  Up to
-// kOneCta points one CTA does all of it in one launch; above, each pass is a
-// histogram and a scatter, whose offsets every scatter CTA sums for itself.
-// 1,920 points: 8 us in one launch, against 17 us of a memset, cell counting,
-// a one-CTA scan of the 32 K cells and a scatter, four launches (the whole
-// mixed evaluation 44.8 -> 31.8 us).  162,816 points: 36 us alone, against 27,
-// of which nothing shows in the evaluation (2,351 and 2,352 us): the price of
-// the fixed order.
+// kOneCta points one CTA does all of it in one launch; above it takes three: the
+// digit counts of the first pass, its scatter, which also counts the second
+// pass's digits, and the second scatter; every scatter CTA sums the counts of
+// all for itself, so that their number is bounded (with 4096 points each, 8
+// million points cost 0.65 ms more).  Kernel times: 1,920 points 8 us in one
+// launch, 40,704 points 22 us in three (27 us with a count launch per pass).
+// As cell counting, a one-CTA scan of the 32 K cells and an unordered scatter
+// (four launches with the memset) the mixed evaluation of 1,920 points took
+// 44.8 us against 31.8, the mixed value of 10,000 points of a 90-AO molecule
+// 53.5 against 54.4 (57.8 with a count launch per pass), that of 40,704 points
+// 91.3 against 90.4 (94.5).
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -27,6 +31,7 @@ constexpr int kDigits = 256;
 constexpr int kOneCta = 4096;
 constexpr int kCtas = 64;         // CTAs of a pass, when that gives runs of kMinRun to kMaxRun points
 constexpr int kMinRun = 1024, kMaxRun = 4096;
+constexpr int64_t kMaxCtas = 592;   // 4 per SM
 
 __device__ __forceinline__ unsigned int spread5(unsigned int x) {   // 5 bits -> every third bit
   x &= 31u;
@@ -85,9 +90,10 @@ __device__ __forceinline__ void warp_ranks(int b, int e, Count* wh, int lane, Di
 // of smaller digits, those of digit d in front of this CTA and those of the
 // CTA's warps before w.  256 Q threads: thread (q, d) takes NW / Q warps.
 // With several CTAs, thread d < 256 brings its digit's total over all of them
-// and its count before this one; with one (ONE) both follow from wh.
+// and its count before these items; with one (ONE) both follow from wh.
+// Returns the items of digit d in the thread's warps.
 template <int NW, int Q, bool ONE, class Count>
-__device__ __forceinline__ void warp_offsets(Count (*wh)[kDigits], unsigned int (*part)[kDigits], unsigned int* dsum,
+__device__ __forceinline__ unsigned int warp_offsets(Count (*wh)[kDigits], unsigned int (*part)[kDigits], unsigned int* dsum,
                                              unsigned int all, unsigned int in_front, int tid) {
   constexpr int W = NW / Q;
   const int lane = tid & 31, warp = tid >> 5, d = tid & (kDigits - 1), q = tid / kDigits;
@@ -133,6 +139,7 @@ __device__ __forceinline__ void warp_offsets(Count (*wh)[kDigits], unsigned int 
     run += c[w];
   }
   __syncthreads();
+  return mine;
 }
 
 __global__ void __launch_bounds__(1024)
@@ -179,89 +186,99 @@ order_one_kernel(const double* __restrict__ coord, const int P, const int64_t cs
   }
 }
 
-// Digit counts of each CTA's run of points, hist[cta][256]; the first pass
-// also writes the cell codes.
-template <int PASS>
+// Cell codes, and the counts of their low digits in each CTA's run of points,
+// hist[cta][256]; the counts of the second pass, taken while the first one
+// scatters, are cleared.
 __global__ void __launch_bounds__(256)
 order_hist_kernel(const double* __restrict__ coord, const int64_t P, const int64_t cstride, const double3 origin,
                   const double inv_cell, const int64_t run, unsigned short* __restrict__ code,
-                  const int* __restrict__ src, unsigned int* __restrict__ hist) {
+                  unsigned int* __restrict__ hist, unsigned int* __restrict__ hist2) {
   __shared__ unsigned int h[kDigits];
   const int tid = threadIdx.x;
   h[tid] = 0u;
+  hist2[(size_t)blockIdx.x * kDigits + tid] = 0u;
   __syncthreads();
   const int64_t b = blockIdx.x * run, e = min(P, b + run);
   for (int64_t i = b + tid; i < e; i += 256) {
-    unsigned int c;
-    if (PASS == 0) {
-      c = cell_code(coord, cstride, i, origin, inv_cell);
-      code[i] = (unsigned short)c;
-      c &= 255u;
-    } else {
-      c = (unsigned int)code[src[i]] >> 8;
-    }
-    atomicAdd(&h[c], 1u);
+    const unsigned int c = cell_code(coord, cstride, i, origin, inv_cell);
+    code[i] = (unsigned short)c;
+    atomicAdd(&h[c & 255u], 1u);
   }
   __syncthreads();
   hist[(size_t)blockIdx.x * kDigits + tid] = h[tid];
 }
 
+// One pass over the CTA's run, kMaxRun points at a time: their places by the
+// pass's digit.  The first pass also counts the high digits of the runs that
+// its points go to.
 template <int PASS>
 __global__ void __launch_bounds__(256)
 order_scatter_kernel(const int64_t P, const int64_t run, const unsigned short* __restrict__ code,
-                     const int* __restrict__ src, const unsigned int* __restrict__ hist, int* __restrict__ dst) {
+                     const int* __restrict__ src, const unsigned int* __restrict__ hist, int* __restrict__ dst,
+                     unsigned int* __restrict__ hist2) {
   constexpr int NW = 8, R = kMaxRun / (32 * NW);
   __shared__ unsigned int wh[NW][kDigits];
   __shared__ unsigned int part[1][kDigits], dsum[8];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t b0 = blockIdx.x * run;
-  const int n = (int)min(run, P - b0), seg = (int)run / NW;
-  const int b = min(n, warp * seg), e = min(n, b + seg);
-  unsigned char dig[R];
-  unsigned short rank[R];
-#pragma unroll
-  for (int w = 0; w < NW; ++w) wh[w][tid] = 0u;
-  __syncthreads();
-  warp_ranks<R>(b, e, wh[warp], lane,
-                [&](int i) { return PASS == 0 ? code[b0 + i] & 255 : code[src[b0 + i]] >> 8; }, dig, rank);
+  const int64_t end = min(P, (blockIdx.x + 1) * run);
   unsigned int all = 0u, in_front = 0u;
-  for (int c0 = 0; c0 < (int)gridDim.x; c0 += 32) {
-    unsigned int v[32];
+  for (int64_t b0 = blockIdx.x * run; b0 < end; b0 += kMaxRun) {
+    const int step = (int)min((int64_t)kMaxRun, run), n = (int)min((int64_t)step, end - b0), seg = step / NW;
+    const int b = min(n, warp * seg), e = min(n, b + seg);
+    unsigned char dig[R];
+    unsigned short rank[R];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = c0 + j < (int)gridDim.x ? hist[(size_t)(c0 + j) * kDigits + tid] : 0u;
+    for (int w = 0; w < NW; ++w) wh[w][tid] = 0u;
+    __syncthreads();
+    warp_ranks<R>(b, e, wh[warp], lane,
+                  [&](int i) { return PASS == 0 ? code[b0 + i] & 255 : code[src[b0 + i]] >> 8; }, dig, rank);
+    if (b0 == blockIdx.x * run) {
+      for (int c0 = 0; c0 < (int)gridDim.x; c0 += 32) {
+        unsigned int v[32];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      all += v[j];
-      if (c0 + j < (int)blockIdx.x) in_front += v[j];
+        for (int j = 0; j < 32; ++j) v[j] = c0 + j < (int)gridDim.x ? hist[(size_t)(c0 + j) * kDigits + tid] : 0u;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          all += v[j];
+          if (c0 + j < (int)blockIdx.x) in_front += v[j];
+        }
+      }
     }
-  }
-  __syncthreads();
-  warp_offsets<NW, 1, false>(wh, part, dsum, all, in_front, tid);
+    __syncthreads();
+    in_front += warp_offsets<NW, 1, false>(wh, part, dsum, all, in_front, tid);
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int i = b + 32 * r + lane;
-    if (i < e) dst[wh[warp][dig[r]] + rank[r]] = PASS == 0 ? (int)(b0 + i) : src[b0 + i];
+    for (int r = 0; r < R; ++r) {
+      const int i = b + 32 * r + lane;
+      if (i >= e) continue;
+      const unsigned int at = wh[warp][dig[r]] + rank[r];
+      dst[at] = PASS == 0 ? (int)(b0 + i) : src[b0 + i];
+      if (PASS == 0) atomicAdd(&hist2[(size_t)(at / (unsigned int)run) * kDigits + (code[b0 + i] >> 8)], 1u);
+    }
+    __syncthreads();   // wh is cleared for the next points
   }
 }
 
 size_t code_bytes(int64_t P) { return (sizeof(unsigned short) * (size_t)P + 255) / 256 * 256; }
 
-// points per CTA of the multi-CTA passes: whole warp rounds (8 warps x 32 points)
+// points per CTA of the multi-CTA passes: whole warp rounds (8 warps x 32
+// points) of up to kMaxRun, then whole kMaxRuns that leave at most kMaxCtas
+// CTAs, each of which reads the counts of all
 int64_t order_run(int64_t P) {
   const int64_t want = (P + kCtas - 1) / kCtas;
+  if (P > kMaxCtas * kMaxRun) return ((P + kMaxCtas - 1) / kMaxCtas + kMaxRun - 1) / kMaxRun * kMaxRun;
   return (std::min<int64_t>(kMaxRun, std::max<int64_t>(kMinRun, want)) + 255) / 256 * 256;
 }
 int64_t order_ctas(int64_t P) { return (P + order_run(P) - 1) / order_run(P); }
 
 }  // namespace
 
-// The count of CTAs falls where a run grows by 256 points (64 at 65,536 points,
-// 52 at 65,537); the histograms get room for the most that any count up to
+// The count of CTAs falls where a run grows (64 at 65,536 points, 52 at
+// 65,537); the two histograms get room for the most that any count up to
 // point_num takes, so that scratch made for a count serves every smaller one.
 size_t point_order_bytes(int64_t point_num) {
   if (point_num <= kOneCta) return 0;
-  const int64_t most = std::max<int64_t>(kCtas, (point_num + kMaxRun - 1) / kMaxRun);
-  return code_bytes(point_num) + sizeof(unsigned int) * kDigits * (size_t)most + sizeof(int) * (size_t)point_num;
+  const int64_t most = std::min(kMaxCtas, std::max<int64_t>(kCtas, (point_num + kMaxRun - 1) / kMaxRun));
+  return code_bytes(point_num) + 2 * sizeof(unsigned int) * kDigits * (size_t)most + sizeof(int) * (size_t)point_num;
 }
 
 cudaError_t point_order(const double* coord, int64_t point_num, const double* box_lo, const double* box_hi,
@@ -282,12 +299,12 @@ cudaError_t point_order(const double* coord, int64_t point_num, const double* bo
   unsigned int* hist = (unsigned int*)((uint8_t*)scratch + code_bytes(point_num));
   const int64_t run = order_run(point_num);
   const unsigned ctas = (unsigned)order_ctas(point_num);
-  int* mid = (int*)(hist + (size_t)ctas * kDigits);
-  order_hist_kernel<0><<<ctas, 256, 0, s>>>(coord, point_num, cstride, origin, inv, run, code, nullptr, hist);
-  order_scatter_kernel<0><<<ctas, 256, 0, s>>>(point_num, run, code, nullptr, hist, mid);
-  order_hist_kernel<1><<<ctas, 256, 0, s>>>(coord, point_num, cstride, origin, inv, run, code, mid, hist);
-  order_scatter_kernel<1><<<ctas, 256, 0, s>>>(point_num, run, code, mid, hist, perm);
-  count_launch(4);
+  unsigned int* hist2 = hist + (size_t)ctas * kDigits;
+  int* mid = (int*)(hist2 + (size_t)ctas * kDigits);
+  order_hist_kernel<<<ctas, 256, 0, s>>>(coord, point_num, cstride, origin, inv, run, code, hist, hist2);
+  order_scatter_kernel<0><<<ctas, 256, 0, s>>>(point_num, run, code, nullptr, hist, mid, hist2);
+  order_scatter_kernel<1><<<ctas, 256, 0, s>>>(point_num, run, code, mid, hist2, perm, nullptr);
+  count_launch(3);
   return cudaGetLastError();
 }
 

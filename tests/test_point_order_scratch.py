@@ -3,7 +3,7 @@
 The batched loop and the chunked adjoint size the scratch for their largest
 point count and then sort smaller counts in it, so its size must not fall as
 the count grows, and it must hold what the sort lays out in it: 2-byte cell
-codes, 1 KB of digit counts per block of the multi-block sort, 4-byte indices.
+codes, 2 KB of digit counts per block of the multi-block sort, 4-byte indices.
 """
 import ctypes
 
@@ -19,22 +19,24 @@ def _bytes():
 
 
 def _blocks(n):
-    """Blocks of a pass: runs of 1024 to 4096 points, whole 256s, aiming at 64 blocks."""
+    """Blocks of a pass: runs of 1024 to 4096 points, whole 256s, aiming at 64 blocks; whole 4096s for 592 blocks."""
     run = -(-min(4096, max(1024, -(-n // 64))) // 256) * 256
+    if n > 592 * 4096:
+        run = -(-(-(-n // 592)) // 4096) * 4096
     return -(-n // run)
 
 
 def test_scratch_serves_every_smaller_count():
     f = _bytes()
     edges = np.arange(256, 400_000, 256)
-    counts = sorted(set(int(e + o) for e in edges for o in (-1, 0, 1)) | {66_000, 65_000, 1_000_000, 6_170_000})
+    counts = sorted(set(int(e + o) for e in edges for o in (-1, 0, 1)) | {66_000, 65_000, 1_000_000, 2_424_832, 2_424_833, 6_170_000})
     size = [f(n) for n in counts]
     assert all(a <= b for a, b in zip(size, size[1:]))
 
 
 def test_scratch_holds_the_layout():
     f = _bytes()
-    for n in [4097, 16_385, 65_535, 65_536, 65_537, 131_073, 262_144, 262_145, 1_000_001, 6_170_000]:
+    for n in [4097, 16_385, 65_535, 65_536, 65_537, 131_073, 262_144, 262_145, 1_000_001, 2_424_832, 2_424_833, 6_170_000]:
         codes = -(-2 * n // 256) * 256
-        assert f(n) >= codes + 1024 * _blocks(n) + 4 * n
+        assert f(n) >= codes + 2048 * _blocks(n) + 4 * n
     assert f(4096) == 0
