@@ -393,10 +393,12 @@ fused_mo_kernel(const DevTables T, const __grid_constant__ CUtensorMap tmB, cons
 // kernel's own prologue finds them.  One CTA per tile, bound by the tests'
 // instructions: a thread per screening sphere drops the spheres beyond the
 // tile's bounding box and takes those that hold its first point; the others,
-// packed, are tested against all points.  (Lanes over a block's spheres, each
-// looping over the points, cost every warp its longest loop: 117 and 301 us on
-// 162,816 and 179,200 points of the 2000- and 5000-AO molecules, now 52 and
-// 77.)
+// packed, are tested against all points, few of them by several threads each
+// (a value tile's 128 points one after the other, by a thread per sphere, are
+// the kernel's time on small bases: 14.4 against 8.0 us on 90 AOs).  (Lanes over
+// a block's spheres, each looping over the points, cost every warp its longest
+// loop: 117 and 301 us on 162,816 and 179,200 points of the 2000- and 5000-AO
+// molecules, now 52 and 77.)
 template <int PTS>
 __global__ void __launch_bounds__(256)
 tile_plan_kernel(const int64_t P, const double* __restrict__ coord, const int64_t cstride, const int* __restrict__ perm,
@@ -461,12 +463,13 @@ tile_plan_kernel(const int64_t P, const double* __restrict__ coord, const int64_
           open[atomicAdd(&nopen, 1)] = q;
       }
       __syncthreads();
-      const int n = nopen;
-      for (int i = tid; i < n; i += 256) {
-        const int q = open[i];
+      // few spheres: up to 8 threads each, every one with its share of the points
+      const int n = nopen, sh = n <= 32 ? 3 : n <= 64 ? 2 : n <= 128 ? 1 : 0;
+      for (int i = tid; i < n << sh; i += 256) {
+        const int q = open[i >> sh];
         const double4 c = sph[q];
         bool in = false;
-        for (int j = 1; j < np && !in; j += 4) {
+        for (int j = 1 + 4 * (i & ((1 << sh) - 1)); j < np && !in; j += 4 << sh) {
 #pragma unroll
           for (int h = 0; h < 4; ++h) {
             const int k = min(j + h, np - 1);
