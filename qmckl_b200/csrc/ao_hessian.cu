@@ -15,7 +15,8 @@
 // 5,087 points x 1000 AOs (0.49 GB): 0.124 ms, 3.9 TB/s.  A warp per point
 // over all its AOs with stores from registers took 0.198 ms, tiles of 32
 // points with lanes on the points 0.18 ms (the few live shells of a segment
-// keep too few warps busy with 12 rows per AO).
+// keep too few warps busy with 12 rows per AO).  Small molecules at many points
+// take the warp per point (hessian_by_warps).
 #include <algorithm>
 
 #include "ao_derivs.cuh"
@@ -28,7 +29,13 @@ namespace {
 constexpr int kHessRows = 12, kThreadsH = 128;
 constexpr int kHessRad = 7;   // R, R1, R2, R3, displacement
 
-__global__ void __launch_bounds__(kThreadsH)
+// CTAs per SM: as many as the registers allow (80 a thread).  More, where small
+// images left room for them, ran as a second, nearly empty wave of CTAs that
+// each had as many items as the first (20,000 points x 400 AOs 0.30 ms with 7,
+// 0.22 with 6).
+constexpr int kHessCtas = 6;
+
+__global__ void __launch_bounds__(kThreadsH, kHessCtas)
 ao_hessian_kernel(const int64_t P, const double* __restrict__ coord, const F64Shell* __restrict__ sh,
                   const double2* __restrict__ prim, const int32_t* __restrict__ ao_code,
                   const double* __restrict__ factor, const int2* __restrict__ segs, const int nseg, const int width,
@@ -146,22 +153,130 @@ ao_hessian_kernel(const int64_t P, const double* __restrict__ coord, const F64Sh
   if (tid < kHessRows) tcx::bulk_wait_read();
 }
 
+// The same with a warp per point over all its AOs, lanes on the AOs, and stores
+// from registers: through the point's nucleus blocks, the lanes stage a block's
+// displacements and radial parts in shared memory, then sweep its AOs.
+constexpr int kWarpsH = 8;
+struct HessSmem {
+  double rad[kBlockSlots][4];   // R, R1, R2, R3 of the block's shells
+  double nuc[kBlockNuc][4];     // displacement, r^2 (negative when screened out)
+  uint8_t act[kBlockSlots];     // the shells whose nucleus is in range
+};
+
+__global__ void __launch_bounds__(kWarpsH * 32)
+ao_hessian_warp_kernel(const DevTables T, const int64_t P, const double* __restrict__ coord, const double cutoff,
+                       const bool fp32_exp, const double* __restrict__ cusp_r, double* __restrict__ out) {
+  __shared__ HessSmem smem[kWarpsH];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  HessSmem& sm = smem[warp];
+  const int64_t A = T.ao_num;
+  for (int64_t p = (int64_t)blockIdx.x * kWarpsH + warp; p < P; p += (int64_t)gridDim.x * kWarpsH) {
+    for (int b = 0; b < T.nblock; ++b) {
+      const int4 blk = T.block[b];
+      const int2 slots = T.block_slots[b];
+      if (lane < blk.y - blk.x) {
+        const int n = blk.x + lane, N = T.nucl_num;
+        const double x = coord[p] - T.nucl_coord[n], y = coord[p + P] - T.nucl_coord[n + N],
+                     z = coord[p + 2 * P] - T.nucl_coord[n + 2 * N];
+        const double r2 = x * x + y * y + z * z;
+        sm.nuc[lane][0] = x;
+        sm.nuc[lane][1] = y;
+        sm.nuc[lane][2] = z;
+        sm.nuc[lane][3] = !(r2 > cutoff * T.nucleus_range[n]) ? r2 : -1.0;
+      }
+      __syncwarp();
+      const int nlive = pack_live_slots(T.slot_nuc, blk.x, slots, sm.nuc, sm.act, lane);
+      for (int i = lane; i < nlive; i += 32) {
+        const int ls = sm.act[i], s = slots.x + ls;
+        const double r2 = sm.nuc[T.slot_nuc[s] - blk.x][3];
+        const int2 cr = T.slot_coef[s];
+        double a[4] = {0., 0., 0., 0.};
+        for (int j = cr.x; j < cr.y; ++j) {
+          const double2 ac = T.coef_ac[j];
+          const double ar2 = ac.x * r2;
+          if (ar2 > cutoff) break;   // primitives are sorted by exponent
+          const double e = (fp32_exp && ar2 <= 30.0) ? (double)expf(-(float)ar2) : exp(-ar2);
+          const double ce = ac.y * e;
+          a[0] += ce;
+          a[1] -= ac.x * ce;
+          a[2] += ac.x * ac.x * ce;
+          a[3] -= ac.x * ac.x * ac.x * ce;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sm.rad[ls][c] = a[c];
+      }
+      __syncwarp();
+      for (int k = blk.z + lane; k < blk.w; k += 32) {
+        const int code = T.ao_code[k];
+        const double* nc = sm.nuc[(code >> 24) & 31];
+        const double* R = sm.rad[(code >> 16) & 255];
+        const double r2 = nc[3];
+        double g[3], H[3][3] = {{0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}}, Tl[3] = {0., 0., 0.};
+        if (!(r2 < 0.0) && R[0] != 0.0 &&   // a NaN distance gives NaNs
+            !cusp_masked(cusp_r, (code >> 12) & 15, blk.x + ((code >> 24) & 31), r2, false)) {
+          const double v[3] = {nc[0], nc[1], nc[2]}, R3[3] = {R[0], R[1], R[2]};
+          ao_derivs<double>(code, T.ao_factor[k], v, R3, 4.0 * r2 * R[2] + 6.0 * R[1], 20.0 * R[2] + 8.0 * r2 * R[3], g,
+                            H, Tl);
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          double* o = out + (((int64_t)d * P + p) * 4) * A + k;
+          o[0] = H[d][0];
+          o[A] = H[d][1];
+          o[2 * A] = H[d][2];
+          o[3 * A] = Tl[d];
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
 }  // namespace
 
-int hessian_segment_width(int64_t ao_num) {
-  const int64_t n = std::max<int64_t>(1, (ao_num + 255) / 256);   // at most 256 AOs: 12-row images of 25 KB
+// Segments of at most 256 AOs (images of 25 KB, six CTAs per SM; 320 on 600 or
+// 800 AOs of s, p and d shells is the same or slower).  With shells of high
+// angular momentum an item's radial parts are few, and its fixed cost counts:
+// 320 (10,000 points x 914 AOs 0.30 -> 0.25 ms).  Molecules of up to 448 AOs with
+// no more shells than threads in one (10,000 points x 380 AOs 0.115 -> 0.098 ms;
+// 400 AOs of 180 shells are slower in one).
+int hessian_segment_width(int64_t ao_num, int64_t shell_num) {
+  if (ao_num <= 448 && shell_num <= kThreadsH) return (int)std::max<int64_t>(32, (ao_num + 31) / 32 * 32);
+  const int64_t limit = ao_num >= 5 * shell_num ? 320 : 256;
+  const int64_t n = std::max<int64_t>(1, (ao_num + limit - 1) / limit);
   return (int)std::max<int64_t>(32, ((ao_num + n - 1) / n + 31) / 32 * 32);
+}
+
+// Where a warp per point is the faster one: an image costs 4 to 7 ns per segment
+// and point however few AOs it holds, a warp about 0.03 ns per AO once there are
+// points for all warps.  Up to 208 AOs from 10 points per AO on (40,000 points x
+// 55 AOs 84 against 171 us, x 200 AOs 199 against 213 to 271; 1,000 points x 200
+// AOs 15 against 13).  With shells of high angular momentum, most of whose work
+// is the AOs', up to 640 AOs from 5,000 points on (10,000 x 519 AOs 158 against
+// 176 us) and any from 20,000 on (40,000 x 638 AOs 0.61 against 0.67 ms, x 914
+// AOs 0.88 to 1.11 against 0.74 to 0.98).
+static bool hessian_by_warps(const DevTables& T, int64_t points) {
+  if (T.ao_num <= 208) return points >= std::max<int64_t>(1000, 10 * (int64_t)T.ao_num);
+  if (T.ao_num < 5 * T.shell_num) return false;
+  return points >= (T.ao_num <= 272 ? 10 * (int64_t)T.ao_num : T.ao_num <= 640 ? 5000 : 20000);
 }
 
 cudaError_t launch_ao_hessian(const DevTables& T, const AoSegments& g, int64_t point_num, const double* coord,
                               double cutoff, bool mixed, double* ao_hessian, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0 || T.ao_num <= 0) return cudaSuccess;
+  if (hessian_by_warps(T, point_num)) {
+    const int64_t grid = std::min<int64_t>((point_num + kWarpsH - 1) / kWarpsH, 148 * 8);
+    ao_hessian_warp_kernel<<<(unsigned)grid, kWarpsH * 32, 0, s>>>(T, point_num, coord, cutoff, mixed, cusp_r,
+                                                                   ao_hessian);
+    count_launch();
+    return cudaGetLastError();
+  }
   const int max_shells = std::max(1, g.max_shells);
   const size_t smem = sizeof(double) * kHessRows * (size_t)(g.width + 2) + sizeof(double) * kHessRad * (size_t)max_shells +
                       sizeof(uint32_t) * 2 * (size_t)g.width + sizeof(int) * (size_t)max_shells;
   cudaError_t e = cudaFuncSetAttribute(ao_hessian_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem - 1024);
   if (e != cudaSuccess) return e;
-  const int64_t per_sm = std::min<int64_t>(12, std::max<int64_t>(1, (int64_t)(227 * 1024) / (int64_t)(smem + 2048)));
+  const int64_t per_sm = std::min<int64_t>(kHessCtas, std::max<int64_t>(1, (int64_t)(227 * 1024) / (int64_t)(smem + 2048)));
   const int64_t grid = std::min<int64_t>(point_num * g.nseg, 148 * per_sm);
   ao_hessian_kernel<<<(unsigned)grid, kThreadsH, smem, s>>>(point_num, coord, g.sh, T.coef_ac, T.ao_code, T.ao_factor,
                                                             g.seg, g.nseg, g.width, max_shells, T.ao_num, cutoff, mixed,

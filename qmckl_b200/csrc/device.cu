@@ -760,7 +760,7 @@ qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
       e.nucl = (int32_t)m;
     }
   AoSegments g{};
-  g.width = hessian_segment_width(A);
+  g.width = hessian_segment_width(A, S);
   std::vector<int2> segs;
   int64_t s0 = 0;
   for (int64_t a0 = 0; a0 < A; a0 += g.width) {

@@ -59,7 +59,7 @@ __device__ __forceinline__ bool cusp_masked(const double* cusp_r, int l, int nuc
 }
 
 // Whole warp: the positions (relative to slots.x) of a nucleus block's shells
-// whose nucleus is in range of the point (nuc[.][3] >= 0), packed in slot
+// whose nucleus is in range of the point (nuc[.][3] not negative), packed in slot
 // order into act; returns their count.  The radial staging then runs over
 // the live shells only, in as few 32-lane passes as they need.
 __device__ __forceinline__ int pack_live_slots(const int32_t* __restrict__ slot_nuc, int blk_first, int2 slots,
@@ -67,7 +67,7 @@ __device__ __forceinline__ int pack_live_slots(const int32_t* __restrict__ slot_
   int n = 0;
   for (int s0 = slots.x; s0 < slots.y; s0 += 32) {
     const int s = s0 + lane;
-    const bool live = s < slots.y && nuc[slot_nuc[s] - blk_first][3] >= 0.0;
+    const bool live = s < slots.y && !(nuc[slot_nuc[s] - blk_first][3] < 0.0);
     const unsigned int m = __ballot_sync(0xffffffffu, live);
     if (live) act[n + __popc(m & ((1u << lane) - 1u))] = (uint8_t)(s - slots.x);
     n += __popc(m);
@@ -76,16 +76,16 @@ __device__ __forceinline__ int pack_live_slots(const int32_t* __restrict__ slot_
   return n;
 }
 
-// AO kernels (ao_kernels.cu).  coord is [3][point_num].  All return
-// cudaGetLastError() after the launch.
-// cusp_r (optional, [nucl]): the AOs that the cusp adjustment leaves out of
-// the MO sums are written as zero (the arrays then only feed the MO step).
 // A block's most shared memory.  A kernel whose dynamic shared memory differs
 // from call to call is opted in to all of it (less its static part), never to a
 // call's size: the attribute belongs to the kernel, and another thread's
 // smaller call could lower it between a call's opt-in and its launch.
 constexpr int kMaxSmem = 232448;
 
+// AO kernels (ao_kernels.cu).  coord is [3][point_num].  All return
+// cudaGetLastError() after the launch.
+// cusp_r (optional, [nucl]): the AOs that the cusp adjustment leaves out of
+// the MO sums are written as zero (the arrays then only feed the MO step).
 cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const double* coord,
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s,
                               const double* cusp_r = nullptr);
@@ -97,7 +97,7 @@ cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const dou
 cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const double* coord, double cutoff,
                                  bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s);
 // AO Hessian (ao_hessian.cu): the shell records and segments of `width` =
-// hessian_segment_width(ao_num) AOs, the shells [seg.x, seg.y) with AOs in
+// hessian_segment_width AOs, the shells [seg.x, seg.y) with AOs in
 // each; at most max_shells of them.
 struct F64Shell;
 struct AoSegments {
@@ -105,7 +105,7 @@ struct AoSegments {
   const int2* seg;
   int nseg, width, max_shells;
 };
-int hessian_segment_width(int64_t ao_num);
+int hessian_segment_width(int64_t ao_num, int64_t shell_num);
 // ao_hessian [3][point_num][4][ao]; `mixed`: FP32 exponentials where a r^2 <= 30.
 cudaError_t launch_ao_hessian(const DevTables& T, const AoSegments& g, int64_t point_num, const double* coord,
                               double cutoff, bool mixed, double* ao_hessian, cudaStream_t s,
