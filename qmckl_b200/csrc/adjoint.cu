@@ -31,7 +31,8 @@
 namespace qb {
 namespace {
 
-constexpr int64_t kDerivCtas = 6 * 148;   // the derivative kernel shares tiles out below this many
+// the derivative kernel shares tiles out below this many, among up to kDerivParts CTAs each
+constexpr int64_t kDerivCtas = 6 * 148, kDerivParts = 24;
 
 // One AO of the FP64 adjoint, exponents known at compile time: with the
 // pulled-back weights (G0, g = G1..G3, G4) and P's derivatives,
@@ -125,7 +126,9 @@ __device__ __forceinline__ void adj_shell(const ShellRad& S, const double (&xp)[
 // exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic
 // (displacements, r^2, radial sums and the cancelling radial combinations in
 // FP64; q summed in FP64); 0.18 ms, against 0.93 with a warp per point over all
-// AOs.  Two or three CTAs per tile below 900 tiles: 0.24 and 0.14 ms with one.
+// AOs.  Below 888 tiles (kDerivCtas) 2 to 24 CTAs share a tile: two at 636
+// tiles, where it took 0.24 ms mixed and 0.14 FP64 with one.  adj.live null: all
+// shells for every tile, G's rows the AOs.
 template <bool MIXED>
 __global__ void __launch_bounds__(256, MIXED ? 3 : 2)
 tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__ coord, const int64_t cstride,
@@ -143,7 +146,7 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
   const int64_t pi = in ? (perm ? (int64_t)perm[qi] : qi) : 0;
   const double px = in ? coord[pi] : 0.0, py = in ? coord[pi + cstride] : 0.0, pz = in ? coord[pi + 2 * cstride] : 0.0;
   // with shells of l >= 4, T.shell_parts entries per shell share its AOs
-  const int n = adj.nlive[tile] * T.shell_parts;
+  const int n = (adj.live != nullptr ? adj.nlive[tile] : T.shell_num) * T.shell_parts;
   const int part = (int)blockIdx.y * NW + warp, parts = (int)gridDim.y * NW;
   const int e0 = (int)((int64_t)n * part / parts), e1 = (int)((int64_t)n * (part + 1) / parts);
   const F* gt = gc + (size_t)tile * kmax * LD + lane;
@@ -170,8 +173,10 @@ tile_deriv_kernel(const DevTables T, const int64_t P, const double* __restrict__
     nq[0] = nq[1] = nq[2] = 0.0;
   };
   for (int e = e0; e < e1; ++e) {
-    const int2 le = adj.live[tile * T.shell_num + e / T.shell_parts];
+    int2 le = make_int2(e / T.shell_parts, 0);
+    if (adj.live != nullptr) le = adj.live[tile * T.shell_num + le.x];
     const F64Shell S = sh[le.x];
+    if (adj.live == nullptr) le.y = S.a0;
     const int sp = e % T.shell_parts;
     if (sp > 0 && S.l < 4) continue;
     if (S.nucl != nucl) {
@@ -344,14 +349,18 @@ cudaError_t launch_forces(int which, int64_t P, int64_t A, int64_t M, int N, con
   return cudaGetLastError();
 }
 
-static int deriv_parts(int64_t ntiles) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>(8, (kDerivCtas + ntiles - 1) / ntiles));
+// CTAs per tile: enough to fill the chip, up to 8, or up to 24 where there are
+// shells (or parts of shells) for all their warps (60 points x 380 AOs, l up to
+// 7: the mixed adjoint 93 us with 8, 79 with 24; x 1000 AOs 84 and 74).
+static int deriv_parts(int64_t ntiles, int64_t entries) {
+  const int64_t most = std::max<int64_t>(8, std::min<int64_t>(kDerivParts, entries / 8));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(most, (kDerivCtas + ntiles - 1) / ntiles));
 }
 
 size_t deriv_share_bytes(int64_t ntiles) {
-  // CTAs that share tiles, for any count up to ntiles: 8 per tile, and below
-  // kDerivCtas + the tiles
-  return sizeof(double) * 96 * (size_t)std::min<int64_t>(8 * ntiles, 2 * kDerivCtas);
+  // CTAs that share tiles, for any count up to ntiles: kDerivParts per tile, and
+  // below kDerivCtas + the tiles
+  return sizeof(double) * 96 * (size_t)std::min<int64_t>(kDerivParts * ntiles, 2 * kDerivCtas);
 }
 
 cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,
@@ -359,7 +368,7 @@ cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord
                               const void* g, bool mixed, double* grad_nucl, double* grad_coord, int64_t gstride,
                               cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
-  const int parts = deriv_parts(ntiles);
+  const int parts = deriv_parts(ntiles, (int64_t)T.shell_num * T.shell_parts);
   auto k = mixed ? tile_deriv_kernel<true> : tile_deriv_kernel<false>;
   k<<<dim3((unsigned)ntiles, (unsigned)parts), 256, 0, s>>>(T, P, coord, cstride, perm, tile0, sh, cutoff, g, adj, T.ao_num,
                                                             grad_nucl, grad_coord, gstride);

@@ -1806,6 +1806,14 @@ namespace {
 // entry with 2048 rows, 7.0e-7 with 4096 and 1.7e-6 with 16384.
 constexpr int kAdjointSliceRows = 2048;
 
+// Whether the mixed adjoint takes all AOs for every tile instead of the lists
+// of those that reach it: up to 2 million (point, AO) pairs the order and the
+// lists, two to four dependent launches, cost more than the AOs they leave out
+// (100 AOs, 1,000 points: 86 against 102 us, 20,000 points: 210 against 232;
+// 240 AOs: 10,000 points 211 and 213, 20,000 points 333 against 318; 1000 AOs:
+// 2,000 points 174 and 176, 4,000 points 267 against 247).
+bool adjoint_all_aos(int64_t points, int64_t aos) { return points * aos <= 2000000; }
+
 // Mixed-form adjoint: the two contractions on the tensor cores.  Per chunk of
 // points: the weights W[(p,c)][mo] as 3 bfloat16 pieces, in the points' order
 // and in the order of spatial tiles of 32 points; the AOs in FP64 arithmetic
@@ -1880,13 +1888,17 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
       QB_CUDA(cudaMemcpy2DAsync(ds->adj_coord.p, sizeof(double) * n, d_coord + p0, sizeof(double) * P,
                                 sizeof(double) * n, 3, cudaMemcpyDeviceToDevice, s),
               fname);
+    const bool all = points && adjoint_all_aos(n, A);
     int* perm = nullptr;
-    if (points && tiles > 1) {
+    if (points && tiles > 1 && !all) {
       perm = (int*)ds->order.p;
       QB_CUDA(point_order(cc, n, lo, hi, (uint8_t*)ds->order.p + perm_bytes(n), perm, s, n), fname);
     }
-    if (points)
+    if (all) {
+      QB_CUDA(cudaMemsetAsync(t.adj.bad, 0, sizeof(unsigned int) * (size_t)tiles, s), fname);
+    } else if (points) {
       QB_CUDA(launch_ao_tiles(ds->T, n, 5, cc, n, perm, 0, tiles, sh, cutoff, false, nullptr, t, s), fname);
+    }
     QB_CUDA(tc_split_weights(w, n, (int)M, perm, (int)ldw, d_grad_coef ? ds->adj_wp.p : nullptr,
                              points ? ds->adj_wt.p : nullptr, points ? t.adj.bad : nullptr, s),
             fname);
@@ -1900,9 +1912,12 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
               fname);
     }
     if (points) {
-      QB_CUDA(tc_pullback(ds->adj_wt.p, (int)ldw, tiles, (int)M, ds->adj_ct.p, A, t.klist, t.kcount, (float*)buf, err, s),
+      AdjTables adj = t.adj;
+      if (all) adj.live = nullptr;
+      QB_CUDA(tc_pullback(ds->adj_wt.p, (int)ldw, tiles, (int)M, ds->adj_ct.p, A, all ? nullptr : t.klist, t.kcount,
+                          (float*)buf, err, s),
               fname);
-      QB_CUDA(launch_tile_deriv(ds->T, n, cc, n, perm, 0, tiles, sh, cutoff, t.adj, buf, true, d_grad_nucl,
+      QB_CUDA(launch_tile_deriv(ds->T, n, cc, n, perm, 0, tiles, sh, cutoff, adj, buf, true, d_grad_nucl,
                                 d_grad_coord ? d_grad_coord + p0 : nullptr, P, s),
               fname);
     }

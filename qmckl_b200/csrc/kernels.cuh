@@ -204,7 +204,8 @@ cudaError_t launch_adj_coef(int64_t ntiles, int64_t ao_num, int64_t M, const F64
 cudaError_t launch_adj_pullback(int64_t ntiles, int64_t ao_num, int64_t M, const F64Tiles& t, const double* ws,
                                 int64_t ldw, const double* Ct, int64_t ldc, cudaStream_t s);
 // grad_nucl [nucl][3] -= and grad_coord [3][gstride] =, either
-// may be null, from the pulled-back weights g of the tiles: FP64
+// may be null, from the pulled-back weights g of the tiles' listed AOs (all AOs
+// where adj.live is null): FP64
 // [tile][ao_num][164], or (mixed) FP32 [tile][ao_num][160] with FP32
 // exponentials where a r^2 <= 30 and FP32 per-AO derivative arithmetic.
 cudaError_t launch_tile_deriv(const DevTables& T, int64_t P, const double* coord, int64_t cstride, const int* perm,

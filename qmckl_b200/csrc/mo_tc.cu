@@ -435,7 +435,7 @@ tc_pullback_kernel(const __grid_constant__ CUtensorMap tmW, const uint16_t* __re
   uint32_t* tmem_slot = (uint32_t*)(drained + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int64_t tile = blockIdx.y;
-  const int nk = kcount[tile];
+  const int nk = klist != nullptr ? kcount[tile] : (int)kmax;
   const int kblocks = (K + BK - 1) / BK;
   constexpr uint32_t kCols = 512;   // two accumulators of 160 columns
   if (tid == 0) {
@@ -517,7 +517,7 @@ tc_pullback_kernel(const __grid_constant__ CUtensorMap tmW, const uint16_t* __re
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int m = m0 + (tid >> 3) + 16 * i;
-        row_ao[i] = m < nk ? klist[tile * kmax + m] : -1;
+        row_ao[i] = m >= nk ? -1 : klist != nullptr ? klist[tile * kmax + m] : m;
       }
       for (int kb = 0; kb < kblocks; ++kb, ++g) {
         const int s = g % kPbStages;
@@ -1129,7 +1129,7 @@ cudaError_t tc_pullback(const void* tiled, int ldw, int64_t tiles, int M, const 
                             tiles * kPbCols * ldw, kPbCols))
       return cudaErrorInvalidValue;
     tc_pullback_kernel<<<dim3((unsigned)gx, (unsigned)n), kThreads, smem, s>>>(
-        tw, (const uint16_t*)ct, ldw, ao_num * ldw, M, klist + t0 * ao_num, kcount + t0, ao_num,
+        tw, (const uint16_t*)ct, ldw, ao_num * ldw, M, klist != nullptr ? klist + t0 * ao_num : nullptr, kcount + t0, ao_num,
         gc + (size_t)t0 * ao_num * kPbCols, err);
     count_launch();
   }

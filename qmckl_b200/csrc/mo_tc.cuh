@@ -132,7 +132,8 @@ cudaError_t tc_run_scratch(const DevTables& T, const TcPlan& plan, int64_t point
 //   tc_pullback   : gc[tile][m][160] (FP32) = sum over the MOs of
 //                   C[klist[tile][m]][mo] * W[tile][pos][mo], m < kcount[tile],
 //                   from tile-order weight pieces and the pieces ct [3][ao][ldw]
-//                   of coefficient_t (klist, gc rows: ao_num per tile)
+//                   of coefficient_t (klist, gc rows: ao_num per tile); klist
+//                   null: all AOs
 // err: a device error word set by a timed-out barrier wait.
 cudaError_t tc_split_rows(const double* x, int64_t rows, int cols, int64_t ldx, void* pieces, int ldp,
                           int64_t pstride, cudaStream_t s);
