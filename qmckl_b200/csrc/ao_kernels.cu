@@ -138,13 +138,13 @@ __device__ __forceinline__ void stage_block(const DevTables& T, WarpSmem& sm, co
   __syncwarp();
 }
 
-// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1), a warp per (point, `per`
-// nucleus blocks).  SPLIT: each value
+// FP64 AO VGL (COMPS = 5) or AO value (COMPS = 1), a warp per (point,
+// gridDim.y'th of the nucleus blocks).  SPLIT: each value
 // stored as 3 bfloat16 pieces (split.cuh) at pieces[q * pstride + row * lda
 // + ao], rows p * COMPS + c, instead of FP64 in `out`.
 template <int COMPS, bool SPLIT = false>
 __global__ void __launch_bounds__(kWarps * 32)
-ao_f64_kernel(const DevTables T, const int per, const int64_t point_num, const double* __restrict__ coord,
+ao_f64_kernel(const DevTables T, const int64_t point_num, const double* __restrict__ coord,
               const double cutoff, const bool dp_exp, double* __restrict__ out,
               uint16_t* __restrict__ pieces = nullptr, const int64_t lda = 0, const int64_t pstride = 0,
               const double* __restrict__ cusp_r = nullptr) {
@@ -154,8 +154,10 @@ ao_f64_kernel(const DevTables T, const int per, const int64_t point_num, const d
   WarpSmem& sm = smem[warp];
   const int64_t A = T.ao_num;
   const int64_t stride = (int64_t)gridDim.x * kWarps;
+  const int per = (T.nblock + (int)gridDim.y - 1) / (int)gridDim.y;
+  const int b0 = (int)blockIdx.y * per, b1 = min(T.nblock, b0 + per);
   for (int64_t p = (int64_t)blockIdx.x * kWarps + warp; p < point_num; p += stride)
-  for (int b = (int)blockIdx.y * per, b1 = min(T.nblock, b + per); b < b1; ++b) {
+  for (int b = b0; b < b1; ++b) {
     const int4 blk = T.block[b];
     const int2 slots = T.block_slots[b];
     const double px = coord[p], py = coord[p + point_num], pz = coord[p + 2 * point_num];
@@ -311,10 +313,9 @@ __global__ void shell_vgl_kernel(const DevTables T, const int64_t point_num,
 // warps, on the config-1 molecule).  Points too few to fill the chip (8 CTAs
 // per SM) have their blocks spread all the same: 100 points x 5000 AOs, the
 // pieces, 15 us against 169 us.
-dim3 ao_grid(const DevTables& T, int64_t points, int* per) {
+dim3 ao_grid(const DevTables& T, int64_t points) {
   const int64_t want = (points + kWarps - 1) / kWarps, cap = 148 * 8;
   const int64_t split = std::min<int64_t>(std::max(1, T.nblock), std::max<int64_t>(1, cap / want));
-  *per = (int)((T.nblock + split - 1) / split);
   return dim3((unsigned)std::min(want, cap), (unsigned)split);
 }
 
@@ -323,9 +324,7 @@ dim3 ao_grid(const DevTables& T, int64_t points, int* per) {
 cudaError_t launch_ao_vgl_f64(const DevTables& T, int64_t point_num, const double* coord,
                               double cutoff, bool dp_exp, double* ao_vgl, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
-  int per = 1;
-  const dim3 grid = ao_grid(T, point_num, &per);
-  ao_f64_kernel<5><<<grid, kWarps * 32, 0, s>>>(T, per, point_num, coord, cutoff, dp_exp, ao_vgl, nullptr, 0, 0, cusp_r);
+  ao_f64_kernel<5><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_vgl, nullptr, 0, 0, cusp_r);
   count_launch();
   return cudaGetLastError();
 }
@@ -334,9 +333,7 @@ cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const do
                                  bool dp_exp, void* pieces, int64_t lda, int64_t pstride, cudaStream_t s) {
   if (point_num <= 0) return cudaSuccess;
   if (lda < T.ao_num || lda % 8 != 0 || pstride % 8 != 0) return cudaErrorInvalidValue;
-  int per = 1;
-  const dim3 grid = ao_grid(T, point_num, &per);
-  ao_f64_kernel<5, true><<<grid, kWarps * 32, 0, s>>>(T, per, point_num, coord, cutoff, dp_exp, nullptr,
+  ao_f64_kernel<5, true><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, nullptr,
                                                       (uint16_t*)pieces, lda, pstride);
   count_launch();
   return cudaGetLastError();
@@ -345,9 +342,7 @@ cudaError_t launch_ao_vgl_pieces(const DevTables& T, int64_t point_num, const do
 cudaError_t launch_ao_value_f64(const DevTables& T, int64_t point_num, const double* coord,
                                 double cutoff, bool dp_exp, double* ao_value, cudaStream_t s, const double* cusp_r) {
   if (point_num <= 0) return cudaSuccess;
-  int per = 1;
-  const dim3 grid = ao_grid(T, point_num, &per);
-  ao_f64_kernel<1><<<grid, kWarps * 32, 0, s>>>(T, per, point_num, coord, cutoff, dp_exp, ao_value, nullptr, 0, 0,
+  ao_f64_kernel<1><<<ao_grid(T, point_num), kWarps * 32, 0, s>>>(T, point_num, coord, cutoff, dp_exp, ao_value, nullptr, 0, 0,
                                                 cusp_r);
   count_launch();
   return cudaGetLastError();
