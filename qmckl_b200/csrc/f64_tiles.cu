@@ -148,7 +148,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   __shared__ bool isnan_g[G];
   __shared__ int claim, nopen;
   extern __shared__ int sbuf[];
-  int* live = sbuf;               // [count] shell | group mask << 24
+  int* live = sbuf;               // [shell_num] whether the shell is live, then [count] the live shells
   int* lpos = sbuf + shell_num;   // [count] first list position
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t tile = blockIdx.x;
@@ -201,7 +201,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
       if (!isnan_g[g] && (bx * bx + by * by + bz * bz) * (1.0 - 1e-9) > S.r2max) continue;
       const double x = spts[32 * g] - S.x, y = spts[TP + 32 * g] - S.y, z = spts[2 * TP + 32 * g] - S.z;
       if (x * x + y * y + z * z <= S.r2max)
-        live[s] |= 1 << g;
+        live[s] = 1;
       else
         lpos[atomicAdd(&nopen, 1)] = s;
     }
@@ -220,7 +220,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
           in = in || !(x * x + y * y + z * z > S.r2max);
         }
         if (in) {
-          live[s] |= 1 << g;
+          live[s] = 1;
           break;
         }
       }
@@ -252,7 +252,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   const int nlive = (int)(total >> 32), nao = (int)(total & 0xffffffffull);
   base += incl - local;
   // compact in place: a thread's live shells move to smaller indices, so the
-  // masks are read into registers before anyone writes
+  // flags are read into registers before anyone writes
   int mk[4];
   const bool few = per <= 4;
   if (few) {
@@ -263,7 +263,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     for (int q = 0; q < 4; ++q)
       if (mk[q]) {
         const int at = (int)(base >> 32), k = (int)(base & 0xffffffffull), s = s0 + q;
-        live[at] = s | (mk[q] << 24);
+        live[at] = s;
         lpos[at] = k;
         base += (1ull << 32) | (unsigned int)sh[s].na;
       }
@@ -273,7 +273,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     const unsigned long long b0 = base;
     for (int s = s0; s < s1; ++s)
       if (lpos[s]) {
-        live[(int)(base >> 32)] = s | (lpos[s] << 24);
+        live[(int)(base >> 32)] = s;
         base += (1ull << 32);
       }
     __syncthreads();
@@ -283,7 +283,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     for (int q = 0; q < n_mine; ++q) {
       const int at = (int)(b0 >> 32) + q;
       b += (unsigned int)na_prev;
-      na_prev = sh[live[at] & 0xffffff].na;
+      na_prev = sh[live[at]].na;
       lpos[at] = (int)(b & 0xffffffffull);
     }
   }
@@ -291,11 +291,11 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
   if (blockIdx.y == 0) {
     int* kl = klist + tile * kmax;
     for (int q = tid; q < nlive; q += kAoThreads) {
-      const F64Shell S = sh[live[q] & 0xffffff];
+      const F64Shell S = sh[live[q]];
       const int k = k0 + lpos[q];
       for (int i = 0; i < S.na; ++i) kl[k + i] = S.a0 + i;
       if (adj.live != nullptr) {
-        adj.live[(int64_t)tile * all_shells + q0 + q] = make_int2(w0 + (live[q] & 0xffffff), k);
+        adj.live[(int64_t)tile * all_shells + q0 + q] = make_int2(w0 + live[q], k);
         if (adj.inv != nullptr)
           for (int i = 0; i < S.na; ++i) adj.inv[tile * kmax + S.a0 + i] = k + i;
       }
@@ -322,8 +322,7 @@ ao_tiles_kernel(const int64_t P, const double* __restrict__ coord, const int64_t
     const int part = u % PARTS;
     u /= PARTS;
     const int q = G == 1 ? u : u / G, g = G == 1 ? 0 : u % G;
-    const int e = live[q];
-    const F64Shell S = sh[e & 0xffffff];
+    const F64Shell S = sh[live[q]];
     if (part > 0 && S.l < 4) continue;
     const int i = 32 * g + lane;
     double* o = act + (size_t)(k0 + lpos[q]) * LD + i;
