@@ -727,8 +727,7 @@ DeviceState* state(qmckl_context context) { return ctx_of(context)->extra; }
 // order), and the latter's segments; for nuclei that moved since, their
 // positions in the records.  All on the context's stream, behind the kernels
 // that read the records before.
-qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds) {
-  const char* fname = "qmckl_b200_mo_fp64";
+qmckl_exit_code sync_f64_shells(qmckl_context context, DeviceState* ds, const char* fname) {
   Context* ctx = ctx_of(context);
   const AoBasisRec& B = ctx->ao_basis;
   const AoDerived& d = B.d;
@@ -852,11 +851,12 @@ qmckl_exit_code run_ao_value(qmckl_context context, DeviceState* ds, int64_t P, 
 
 qmckl_exit_code run_ao_hessian(qmckl_context context, DeviceState* ds, int64_t P, const double* coord, double* out,
                                const double* cusp_r = nullptr) {
+  const char* fname = "qmckl_b200_ao_hessian";
   Context* ctx = ctx_of(context);
-  qmckl_exit_code rc = sync_f64_shells(context, ds);
+  qmckl_exit_code rc = sync_f64_shells(context, ds, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   QB_CUDA(launch_ao_hessian(ds->T, ds->hess, P, coord, cutoff_of(ctx), ctx->precision <= 23, out, ds->stream, cusp_r),
-          "qmckl_b200_ao_hessian");
+          fname);
   return QMCKL_SUCCESS;
 }
 
@@ -993,8 +993,7 @@ qmckl_exit_code prepare_mixed(qmckl_context context, DeviceState* ds) {
 }
 
 // coefficient_t with an even row length (a padded copy for an odd MO count).
-qmckl_exit_code coef_even(qmckl_context context, DeviceState* ds, const double** Bt, int64_t* ldb) {
-  const char* fname = "qmckl_b200_mo_fp64";
+qmckl_exit_code coef_even(qmckl_context context, DeviceState* ds, const double** Bt, int64_t* ldb, const char* fname) {
   Context* ctx = ctx_of(context);
   const int64_t A = ctx->ao_basis.ao_num, M = ctx->mo_basis.mo_num;
   *ldb = M + (M & 1);
@@ -1033,8 +1032,8 @@ qmckl_exit_code run_mo_f64(qmckl_context context, DeviceState* ds, int64_t P, in
   if (P <= 0) return QMCKL_SUCCESS;
   const double* Bt = nullptr;
   int64_t ldb = 0;
-  qmckl_exit_code rc = sync_f64_shells(context, ds);
-  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Bt, &ldb);
+  qmckl_exit_code rc = sync_f64_shells(context, ds, fname);
+  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Bt, &ldb, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   const int pts = f64_tile_points(comps, P);
   const int64_t tiles = (P + pts - 1) / pts;
@@ -1833,7 +1832,7 @@ qmckl_exit_code adjoint_mixed(qmckl_context context, DeviceState* ds, int64_t P,
   const int64_t ldw = (M + 7) / 8 * 8, lda = (A + 7) / 8 * 8;
   const int kps = kAdjointSliceRows / 32;
   qmckl_exit_code rc = sync_coef(context, ds);
-  if (rc == QMCKL_SUCCESS) rc = sync_f64_shells(context, ds);
+  if (rc == QMCKL_SUCCESS) rc = sync_f64_shells(context, ds, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   if (ds->adj_ct_version != ctx->mo_basis.coef_version || !ds->adj_ct.p) {
     rc = ensure(context, ds->adj_ct, sizeof(uint16_t) * 3 * A * ldw, fname);
@@ -1939,8 +1938,8 @@ qmckl_exit_code adjoint_f64(qmckl_context context, DeviceState* ds, int64_t P, c
   cudaStream_t s = ds->stream;
   const double* Ct = nullptr;
   int64_t ldc = 0;
-  qmckl_exit_code rc = sync_f64_shells(context, ds);
-  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Ct, &ldc);
+  qmckl_exit_code rc = sync_f64_shells(context, ds, fname);
+  if (rc == QMCKL_SUCCESS) rc = coef_even(context, ds, &Ct, &ldc, fname);
   if (rc != QMCKL_SUCCESS) return rc;
   const int64_t ldw = M + (M & 1);
   const int pts = f64_tile_points(5, P);
