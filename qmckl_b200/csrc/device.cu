@@ -349,8 +349,9 @@ struct DeviceState {
   DevBuf order;      // point order: perm[P], the sort's scratch, the fused kernel's tile plan
   int rec_bytes = 0;
   uint64_t krec_basis_version = ~0ull, krec_nucl_version = ~0ull;
-  // derivatives: AO Hessian and the MO VGL adjoint (FP64 coefficient [mo][ao],
-  // per-chunk coordinates, AO / pulled-back weight buffer, split-K partials)
+  // derivatives: AO Hessian and the mixed form's adjoint (coordinates of a
+  // chunk, AO pieces / pulled-back weights, split-K partials; the FP64 form
+  // works in f64_tiles)
   DevBuf ao_hessian;
   DevBuf adj_coord, adj_buf, adj_part;
   // mixed-form adjoint: bfloat16 pieces of the weights and of coefficient_t
@@ -1787,12 +1788,13 @@ qmckl_exit_code qmckl_b200_ao_hessian_device(qmckl_context context, const int64_
 // Adjoint of MO VGL.  With L = sum_{p,c,i} W[p][c][i] mo_vgl[p][c][i]:
 //   grad_coef[i][k]  = sum_{p,c} W[p][c][i] ao_vgl[p][c][k]
 //   grad_nucl[a][d]  = dL/dR_a,  grad_coord[d][p] = dL/dr_p
-// Points are processed in chunks that bound the scratch to about 2 GiB.  Per
-// chunk: the AO matrix is recomputed (nothing of the forward pass is kept),
-// grad_coef accumulates AO^T W (split-K FP64 GEMM, partials summed in a fixed
-// order), the AO buffer is then overwritten with G = W C ([point][5][ao]) and
-// the derivative kernel contracts G with the AO Hessian and Laplacian
-// gradient into grad_nucl / grad_coord.
+// Points are processed in chunks that bound the scratch to about 2 GiB in the
+// mixed form and 4 GiB in the FP64 form (less where the device has no room).
+// Per chunk: the AOs are recomputed (nothing of the forward pass is kept),
+// grad_coef accumulates AO^T W in a fixed order, G = W C is formed for the AOs
+// that reach each tile of points, and the derivative kernel contracts it with
+// the AO Hessian and Laplacian gradient into grad_nucl (by atomics) and
+// grad_coord (in a fixed order).
 }  // extern "C"
 
 namespace qb {

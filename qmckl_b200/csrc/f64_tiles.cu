@@ -391,7 +391,9 @@ __device__ __forceinline__ void dmma_t(double& d0, double& d1, double a, double 
 // staged in shared memory (read from global memory at each step it cost a
 // load latency per step: 1.14 against 0.91 ms).  0.91 ms = 37 TFLOP/s of the
 // executed products on 40,704 points, 2000 AOs, 160 MOs (1.10 ms = 30 TFLOP/s
-// with 8-byte gathers of a dense AO array in 128-row tiles).
+// with 8-byte gathers of a dense AO array in 128-row tiles).  That form is at
+// the 128 registers that two CTAs of 256 threads allow, and spills 28 bytes
+// outside the k loop's products.
 template <int COMPS, int TP, int MB, int WM, int WN, int NT, int STG>
 __global__ void __launch_bounds__(32 * WM * WN, WM == 1 ? 5 : 2)
 tile_gemm_kernel(const int64_t P, const int64_t tile0, const int64_t ntiles, const int64_t N,

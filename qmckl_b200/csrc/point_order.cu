@@ -5,7 +5,8 @@
 // grid over the box of the nuclei (coordinates clamped), points of one cell in
 // their own order: a stable least-significant-digit radix sort of the 15-bit
 // cell codes in two passes (8 and 7 bits), so that the order, and with it
-// every sum over tiles, is the same in every run.
+// the tiles and their sums taken in tile order (dL/dC), are the same in every
+// run.
 //
 // The sort is bound by launches and load latencies, not by its bytes.  Up to
 // kOneCta points one CTA does all of it in one launch; above it takes three: the
