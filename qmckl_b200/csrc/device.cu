@@ -804,12 +804,14 @@ qmckl_exit_code ensure_tiles(qmckl_context context, DeviceState* ds, size_t tile
   while (chunk > 1 && (b.p == nullptr || b.cap < tile * (size_t)chunk + more)) {
     if (alloc_should_fail()) return qmckl_failwith(context, QMCKL_ALLOCATION_FAILED, where, "device allocation");
     release(b);
-    if (cudaMalloc(&b.p, tile * (size_t)chunk + more) == cudaSuccess) {
+    const cudaError_t e = cudaMalloc(&b.p, tile * (size_t)chunk + more);
+    if (e == cudaSuccess) {
       b.cap = tile * (size_t)chunk + more;
       return QMCKL_SUCCESS;
     }
     cudaGetLastError();
     b.p = nullptr;
+    if (e != cudaErrorMemoryAllocation) break;   // no want of room (a stream under capture): ensure reports it
     chunk = (chunk + 1) / 2;
     ds->tile_room = (int64_t)tile * chunk;
   }
