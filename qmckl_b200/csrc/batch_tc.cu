@@ -222,7 +222,7 @@ using Team = std::integral_constant<int, N>;   // threads that plan an item
 
 // 16 producer warps: 640 threads leave 96 registers, with 32 bytes spilled; the
 // code around the planning is sensitive to its size (the same tests written as
-// one function for both teams cost 7 to 11% on large batches).
+// one loop or one function for both teams cost 2 to 11% on large batches).
 template <int PRODW>
 __global__ void __launch_bounds__((PRODW + 4) * 32, 1)
 batch_mo_kernel(const BatchDesc* __restrict__ desc, const CUtensorMap* __restrict__ tmaps,
