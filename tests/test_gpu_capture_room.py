@@ -2,6 +2,8 @@
 (device memory cannot be allocated there), and the context then evaluates as
 before: the failed allocation is not taken for a full device, which would leave
 it with small chunks (GPU)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -39,15 +41,18 @@ def test_a_capture_does_not_shrink_the_chunks():
         pq.b200_set_stream(ctx, stream.cuda_stream)
         pq.b200_mo_value_device(ctx, P, c.data_ptr(), values.data_ptr())   # tables, order, a fifth of the scratch
         pq.b200_synchronize(ctx)
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(stream):
-            graph.capture_begin(capture_error_mode="thread_local")
+        # by the runtime itself: torch's allocator would take the capture that fails for one that goes on
+        rt = ctypes.CDLL("libcudart.so.12")
+        s, graph = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p()
+        assert rt.cudaStreamBeginCapture(s, 1) == 0   # thread-local
+        try:
             with pytest.raises(RuntimeError):
                 pq.b200_mo_vgl_device(ctx, P, c.data_ptr(), out.data_ptr())
-            try:
-                graph.capture_end()
-            except RuntimeError:   # the capture was invalidated
-                pass
+        finally:
+            rt.cudaStreamEndCapture(s, ctypes.byref(graph))   # the capture was invalidated
+            if graph.value:
+                rt.cudaGraphDestroy(graph)
+            rt.cudaGetLastError()
         torch.cuda.synchronize()
         out.fill_(float("nan"))
         assert launches(ctx) == want
